@@ -112,7 +112,7 @@ namespace {
 using namespace sphpass;
 
 // Slot-ordered packs for one adjoint step (a.rho points at rho' of the step):
-//   X4 {x, y, z, m}   V4 {vx, vy, vz, rho'}   Q4 {P, P'(rho'), P/B, 0}   A4 {abar, 0}   PF float4 x
+//   X4 {x, y, z, m}   V4 {vx, vy, vz, rho'}   Q4 {P, P'(rho'), P/B, 0}   A4 {abar, 0}   pf FP32 x
 template <int DIM>
 __global__ void adjoint_prep_kernel(SphArgs a) {
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -146,7 +146,7 @@ __global__ void adjoint_prep_kernel(SphArgs a) {
   ((double4_32a*)a.s[1])[k] = make_double4_32a(v[0], v[1], v[2], rho);
   ((double4_32a*)a.s[2])[k] = make_double4_32a(P, Pd, PB, 0.0);
   ((double4_32a*)a.s[3])[k] = make_double4_32a(ab[0], ab[1], ab[2], 0.0);
-  ((float4*)a.s[4])[k] = make_float4((float)x[0], (float)x[1], (float)x[2], 0.f);
+  pf_store<DIM>(a.pf, k, (float)x[0], (float)x[1], (float)x[2]);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -154,7 +154,7 @@ __global__ void adjoint_prep_kernel(SphArgs a) {
 // as FP32 (hi, lo) pairs, so the differences x_i - x_j and v_i - v_j keep FP32 relative
 // accuracy despite the cancellation; every other factor and the pair derivatives are FP32; the
 // adjoint state and the parameter sums stay double.
-//   s0 {x.hi, y.hi, z.hi, m} (also the prefilter positions)   s1 {x.lo, y.lo, z.lo, 0}
+//   s0 {x.hi, y.hi, z.hi, m} (x.hi, y.hi, z.hi also in pf)   s1 {x.lo, y.lo, z.lo, 0}
 //   s2 {vx.hi, vy.hi, vz.hi, rho'}   s3 {vx.lo, vy.lo, vz.lo, 0}   s4 {P, P', P/B, 0}
 //   s5 {abar, 0}   s6 float dbar
 // Per-particle sums (adjoint increments and parameter terms) use Kahan compensation.
@@ -209,6 +209,7 @@ __global__ void adjoint_prep_f_kernel(SphArgs a) {
   const double Pd = K.d.B * ((double)(K.gamma - 2) * pw + 2.0) * inv_r2 / rho;
   const double PB = (pw - 1.0) * inv_r2;
   ((float4*)a.s[0])[k] = make_float4(hx[0], hx[1], hx[2], (float)m);
+  pf_store<DIM>(a.pf, k, hx[0], hx[1], hx[2]);
   ((float4*)a.s[1])[k] = make_float4(lxs[0], lxs[1], lxs[2], 0.f);
   ((float4*)a.s[2])[k] = make_float4(hv[0], hv[1], hv[2], (float)rho);
   ((float4*)a.s[3])[k] = make_float4(lvs[0], lvs[1], lvs[2], 0.f);
@@ -425,7 +426,7 @@ int launch_adjoint_prep(cudaStream_t st, const SphArgs& a, bool fp32) {
   return PG_OK;
 }
 
-typedef void (*AdjKernel)(SphArgs, int);
+typedef void (*AdjKernel)(SphArgs);
 
 // The two-sided passes of the mixed-precision adjoint (the FP64 adjoint evaluates each pair once:
 // pg_adjoint_sym.cu).
@@ -440,10 +441,6 @@ AdjKernel adjoint_kernel(int dim, int stage, bool fp32) {
   return dim == 2 ? adjoint_kernel_dim<2>(stage) : adjoint_kernel_dim<3>(stage);
 }
 
-// Prefilter positions (float4 x, y, z) of the list kernel and of overflow walks: the FP64 packs
-// keep them in s4; the mixed-precision packs use the FP32 hi parts in s0.
-int adjoint_pf_index(bool fp32) { return fp32 ? 0 : 4; }
-
 int launch_adjoint_pass(cudaStream_t st, const SphArgs& a, int stage, int grid, bool fp32) {
   if (!fp32) {
     set_error("the FP64 adjoint runs the pair-once kernels");
@@ -452,7 +449,7 @@ int launch_adjoint_pass(cudaStream_t st, const SphArgs& a, int stage, int grid, 
   if (a.n == 0) return PG_OK;
   const uint32_t ntiles = (a.n + kSphThreads - 1) / kSphThreads;
   if (grid <= 0 || (uint32_t)grid > ntiles) grid = (int)ntiles;
-  adjoint_kernel(a.dim, stage, fp32)<<<grid, kSphThreads, 0, st>>>(a, adjoint_pf_index(fp32));
+  adjoint_kernel(a.dim, stage, fp32)<<<grid, kSphThreads, 0, st>>>(a);
   PG_CUDA_TRY(cudaGetLastError());
   return PG_OK;
 }
@@ -625,12 +622,12 @@ int pg_backward(pg_system* s, const double* dL_dx, double* dL_dalpha, double* dL
   PG_TRY(A->lr.ensure(8 * nn));
   PG_TRY(A->ga.ensure(8 * nn));
   PG_TRY(A->gb.ensure(8 * nn));
-  PG_TRY(A->X4.ensure(32 * (nn + pg::kPackPad)));
-  PG_TRY(A->V4.ensure(32 * (nn + pg::kPackPad)));
-  PG_TRY(A->Q4.ensure(32 * (nn + pg::kPackPad)));
-  PG_TRY(A->A4.ensure(32 * (nn + pg::kPackPad)));
-  PG_TRY(A->PF.ensure(16 * (nn + pg::kPackPad)));
-  PG_TRY(A->DB.ensure(8 * (nn + pg::kPackPad)));
+  PG_TRY(A->X4.ensure(32 * nn));
+  PG_TRY(A->V4.ensure(32 * nn));
+  PG_TRY(A->Q4.ensure(32 * nn));
+  PG_TRY(A->A4.ensure(32 * nn));
+  PG_TRY(A->PF.ensure(4 * pg::chunked_floats(nn, s->dim)));
+  PG_TRY(A->DB.ensure(8 * nn));
   if (fp32 && (A->pass_grid_fp32 != (int)fp32 || A->pass_grid[pg::SPH_MOM] == 0)) {
     int dev = 0, sms = 0;
     PG_CUDA_TRY(cudaGetDevice(&dev));
@@ -663,7 +660,7 @@ int pg_backward(pg_system* s, const double* dL_dx, double* dL_dalpha, double* dL
     a.s[1] = A->V4.p;
     a.s[2] = A->Q4.p;
     a.s[3] = A->A4.p;
-    a.s[4] = A->PF.p;
+    a.s[4] = nullptr;
     a.s[5] = A->DB.p;
     a.s[6] = A->PS.p;
     a.s[7] = nullptr;
@@ -678,6 +675,7 @@ int pg_backward(pg_system* s, const double* dL_dx, double* dL_dalpha, double* dL
   a.nlen = A->nlen.as<uint32_t>();
   a.nresume = A->nresume.as<uint32_t>();
   if (fp32) a.fcache = nullptr;
+  a.pf = A->PF.as<float>();
 
   // Segment seg recomputed into buffer set b on the handle's stream: the steps from the
   // segment's checkpoint, keeping each step's state, rho' and neighbour structure.  It waits
@@ -721,11 +719,11 @@ int pg_backward(pg_system* s, const double* dL_dx, double* dL_dalpha, double* dL
       a.cell_start = A->seg_start[b].as<uint32_t>() + (size_t)t * ncp1;
       PG_TRY(pg::launch_adjoint_prep(st, a, fp32));
       if (fp32) {
-        PG_TRY(pg::launch_sph_list_pf(st, a, pg::adjoint_pf_index(fp32), 0, pg::kSphThreads));
+        PG_TRY(pg::launch_sph_list_pf(st, a, 0, pg::kSphThreads));
         PG_TRY(pg::launch_adjoint_pass(st, a, pg::SPH_MOM, A->pass_grid[pg::SPH_MOM], fp32));
         PG_TRY(pg::launch_adjoint_pass(st, a, pg::SPH_CONT, A->pass_grid[pg::SPH_CONT], fp32));
       } else {
-        PG_TRY(pg::launch_sph_list_exact(st, a, pg::adjoint_pf_index(fp32), 0, pg::kSphThreads));
+        PG_TRY(pg::launch_sph_list_exact(st, a, 0, pg::kSphThreads));
         for (int part = 0; part < 5; ++part) PG_TRY(pg::launch_adjoint_sym(st, a, part));
       }
     }

@@ -93,7 +93,7 @@ __device__ __forceinline__ uint32_t first_above(const uint32_t* __restrict__ my,
 }
 
 // The slot-ordered packs of the adjoint step (adjoint_prep_kernel):
-//   s0 X {x, y, z, m}  s1 V {v, rho'}  s2 Q {P, P', P/B}  s3 A {abar}  s4 float4 x  s5 dbar
+//   s0 X {x, y, z, m}  s1 V {v, rho'}  s2 Q {P, P', P/B}  s3 A {abar}  s5 dbar  pf FP32 x
 //   s6 per-slot partial sums (kSlotSums planes of n doubles)
 struct Packs {
   const double4_32a *X, *V, *Q, *A;
@@ -224,12 +224,12 @@ __device__ __forceinline__ void add_own(Sums& s, const MomTerms<DIM>& m, double 
 template <int DIM, class OnPair>
 __device__ __forceinline__ void resume_walk(const SphArgs& a, const SphK& K, const Packs& P, uint32_t k,
                                             const double4_32a& xk, OnPair&& on_pair) {
-  const float4* __restrict__ PF = (const float4*)a.s[4];
+  const float* __restrict__ PF = a.pf;
   const SphK* Kp;
   const Target T = target_of(a, k, &Kp, a.reach);
   const GridK& g = K.g;
   const int R = a.reach, RZ = DIM == 3 ? R : 0, side = 2 * R + 1, nrows = side * (2 * RZ + 1);
-  const float4 pi = PF[k];
+  const float4 pi = pf_at<DIM>(PF, k);
   const float thr = prefilter_threshold<false>(K, pi);
   const int row0 = (int)a.nresume[2 * (size_t)k];
   const uint32_t t0 = a.nresume[2 * (size_t)k + 1];
@@ -239,7 +239,7 @@ __device__ __forceinline__ void resume_walk(const SphArgs& a, const SphK& K, con
     const uint32_t rb = g.cell_base + ((uint32_t)z * g.ny + (uint32_t)y) * g.nx;
     const uint32_t e = a.cell_start[rb + T.x1 + 1];
     for (uint32_t t = row == row0 ? t0 : a.cell_start[rb + T.x0]; t < e; ++t)
-      if (prefilter_hit<DIM, false>(pi, PF[t], thr) && is_neighbor<DIM>(K.d, xk, P.X[t])) on_pair(t);
+      if (prefilter_hit<DIM, false>(pi, pf_at<DIM>(PF, t), thr) && is_neighbor<DIM>(K.d, xk, P.X[t])) on_pair(t);
   }
 }
 

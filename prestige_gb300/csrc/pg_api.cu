@@ -20,6 +20,7 @@
 #include <vector>
 
 #include "pg_arith.cuh"
+#include "pg_candidates.cuh"
 #include "pg_internal.cuh"
 #include "pg_kernels.cuh"
 #include "pg_system.cuh"
@@ -144,7 +145,8 @@ int ensure_sorted_buffers(pg_system* s) {
   sph_sorted_layout(s->arith, sz);
   const size_t n = s->n ? s->n : 1;
   for (int i = 0; i < 6; ++i)
-    if (sz[i]) PG_TRY(s->sorted[i].ensure(sz[i] * (n + kPackPad)));
+    if (sz[i]) PG_TRY(s->sorted[i].ensure(sz[i] * n));
+  PG_TRY(s->pf.ensure(4 * chunked_floats(n, s->dim)));
   PG_TRY(s->nlist.ensure(4 * ((n + kListTile - 1) / kListTile) * kListTile * (size_t)s->list_cap));
   // per list entry: {m_j F, u} (double-word, 16 B, written by the continuity pass and read by the
   // momentum pass of the same step) or the pair values of the IEEE step (pg_sph_sym.cu)
@@ -169,6 +171,7 @@ SphArgs sph_args(pg_system* s, int integrate, bool rates) {
   a.sorted_id = s->nw.sorted_id;
   a.cell_start = s->nw.cell_start.as<uint32_t>();
   for (int i = 0; i < 6; ++i) a.s[i] = s->sorted[i].p;
+  a.pf = s->pf.as<float>();
   a.s[6] = a.s[7] = nullptr;
   a.pos = s->pos.p;
   a.vel = s->vel.p;
@@ -559,7 +562,7 @@ int choose_overlap(pg_system* s, int sms) {
   if (s->model == PG_MODEL_SPH && s->arith == ARITH_F64_EXACT && s->n >= 1000000) {
     // IEEE step: the lists of the last three quarters of the slots (ALU work) beside the pair
     // values (FP64 work) of the slots of the first quarter whose partners all lie in it
-    const int locc = sph_list_occupancy(s->arith, s->dim, -1, s->block);
+    const int locc = sph_list_occupancy(s->arith, s->dim, s->grids[0].reach, -1, s->block);
     if (locc < 1) return PG_OK;
     PG_TRY(ensure_aux_stream(s));
     s->ov_pass_grid = 0;
@@ -568,7 +571,7 @@ int choose_overlap(pg_system* s, int sms) {
     return PG_OK;
   }
   if (s->model != PG_MODEL_SPH || s->arith != ARITH_F64_DF || s->n < 1000000) return PG_OK;
-  const int rp = sph_list_regs(s->arith, s->dim, SPH_CONT, s->lanes), rl = sph_list_regs(s->arith, s->dim, -1);
+  const int rp = sph_list_regs(s->arith, s->dim, s->grids[0].reach, SPH_CONT, s->lanes), rl = sph_list_regs(s->arith, s->dim, s->grids[0].reach, -1);
   if (rp <= 0 || rl <= 0) return PG_OK;
   const int per_block_p = ((rp + 7) / 8) * 8 * s->block, per_block_l = ((rl + 7) / 8) * 8 * s->block;
   const int regs = 65536, threads = 2048;
@@ -590,10 +593,10 @@ int choose_pass_grid(pg_system* s) {
   PG_CUDA_TRY(cudaGetDevice(&dev));
   PG_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   for (int st = 0; st < 3; ++st) {
-    const int occ = sph_list_occupancy(s->arith, s->dim, st, st == SPH_MOM ? mom_block(s) : s->block, s->lanes);
+    const int occ = sph_list_occupancy(s->arith, s->dim, s->grids[0].reach, st, st == SPH_MOM ? mom_block(s) : s->block, s->lanes);
     s->pass_grid[st] = occ > 0 ? occ * sms : 0;  // persistent: one resident wave
   }
-  const int locc = sph_list_occupancy(s->arith, s->dim, -1, s->block);
+  const int locc = sph_list_occupancy(s->arith, s->dim, s->grids[0].reach, -1, s->block);
   s->list_grid = locc > 0 ? locc * sms : 0;
   return choose_overlap(s, sms);
 }
@@ -1492,6 +1495,7 @@ int pg_memory_bytes(pg_system* s, size_t* bytes) {
                               &s->contacts, &s->err};
   for (const pg::DevBuf* d : bufs) b += d->bytes;
   for (int i = 0; i < 6; ++i) b += s->sorted[i].bytes;
+  b += s->pf.bytes;
   b += s->nlist.bytes + s->nlen.bytes + s->nresume.bytes + s->fcache.bytes;
   for (auto& kv : s->user) b += kv.second->bytes;
   b += s->adjoint_bytes();

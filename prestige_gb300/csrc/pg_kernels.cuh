@@ -18,9 +18,6 @@ enum Arith {
 constexpr int kSphThreads = 128;     // default block size of the SPH kernels
 constexpr int kSphMaxThreads = 256;  // largest block size of the list-based kernels
 constexpr uint32_t kListTile = 32;  // slots per tile of the neighbour-list array
-constexpr size_t kPackPad = 16;      // records allocated past the end of every sorted pack: the
-                                     // list kernel's batched loads run up to kListBatch - 1 past
-                                     // the last slot
 
 // Stages of the SPH pair pass.
 enum SphStage {
@@ -68,6 +65,7 @@ struct SphArgs {
   const uint32_t* sorted_id;
   const uint32_t* cell_start;
   void* s[8];                // sorted packed arrays (layout per arithmetic mode)
+  float* pf;                 // sorted FP32 positions of the candidate walks, in chunks (pg_candidates.cuh)
   void* pos;                 // canonical state, id order
   void* vel;
   void* rho;
@@ -102,10 +100,10 @@ int launch_sph_list(cudaStream_t st, const SphArgs& a, int arith, int grid, int 
 int launch_sph_list_pass(cudaStream_t st, const SphArgs& a, int arith, int stage, int grid, int block,
                          int lanes = 1);
 int sph_pass_lanes(int arith, int stage, int lanes);
-int sph_list_regs(int arith, int dim, int stage, int lanes = 1);  // registers per thread of a list kernel (stage < 0) or pass
-int sph_list_occupancy(int arith, int dim, int stage, int block, int lanes = 1);  // stage < 0: the list kernel
-// The list kernel with an explicit FP32 prefilter-position pack a.s[pf_index] (conservative test).
-int launch_sph_list_pf(cudaStream_t st, const SphArgs& a, int pf_index, int grid, int block);
+int sph_list_regs(int arith, int dim, int reach, int stage, int lanes = 1);  // registers per thread of a list kernel (stage < 0) or pass
+int sph_list_occupancy(int arith, int dim, int reach, int stage, int block, int lanes = 1);  // stage < 0: the list kernel
+// The list kernel with the conservative FP32 test on the positions a.pf.
+int launch_sph_list_pf(cudaStream_t st, const SphArgs& a, int grid, int block);
 // The IEEE f64 step with each neighbour pair evaluated once (pg_sph_sym.cu), over complete lists:
 // part 0 and 1 the continuity pass (pair values, then the sums, rho' and the {rho', P'} pack),
 // part 2 and 3 the momentum pass (pair values, then the sums and the update).  a.fcache holds
@@ -121,7 +119,6 @@ size_t sph_sym_entry_bytes();
 int launch_adjoint_prep(cudaStream_t st, const SphArgs& a, bool fp32);
 int launch_adjoint_pass(cudaStream_t st, const SphArgs& a, int stage, int grid, bool fp32);
 int adjoint_pass_occupancy(int dim, int stage, bool fp32);
-int adjoint_pf_index(bool fp32);
 // The FP64 adjoint passes with each pair evaluated once (pg_adjoint_sym.cu), over exact lists
 // (launch_sph_list_exact): part 0 the mirror indices, 1, 2 the momentum adjoint, 3, 4 the
 // continuity adjoint.
@@ -130,8 +127,8 @@ int launch_adjoint_sym(cudaStream_t st, const SphArgs& a, int part);
 size_t adjoint_sym_entry_bytes();
 size_t adjoint_sym_slot_bytes();
 // The list kernel with the f64 test of the exact neighbours on the double4 positions a.s[0] and
-// the FP32 prefilter positions a.s[pf_index].
-int launch_sph_list_exact(cudaStream_t st, const SphArgs& a, int pf_index, int grid, int block);
+// the FP32 positions a.pf.
+int launch_sph_list_exact(cudaStream_t st, const SphArgs& a, int grid, int block);
 // Bytes per particle of the sorted packed arrays s[0..5] for an arithmetic mode.
 void sph_sorted_layout(int arith, size_t sizes[6]);
 

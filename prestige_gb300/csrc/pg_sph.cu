@@ -49,7 +49,7 @@ template <> __device__ __forceinline__ float2 make2<float>(float a, float b) { r
 
 // ---------------------------------------------------------------------------------------
 // Sorted gather: slot k <- particle sorted_id[k]; precomputes P = p / rho^2.
-//   IEEE modes:   s0 {x, y, z, m}   s1 {vx, vy, vz, 0}   s2 {rho, P}   (f64: s3 float4 x)
+//   IEEE modes:   s0 {x, y, z, m}   s1 {vx, vy, vz, 0}   s2 {rho, P}   (pf: FP32 x, y, z)
 // ---------------------------------------------------------------------------------------
 template <class Ops, int DIM>
 __global__ void sph_gather_real(SphArgs a) {
@@ -75,14 +75,14 @@ __global__ void sph_gather_real(SphArgs a) {
   ((R4*)a.s[0])[k] = A;
   ((R4*)a.s[1])[k] = B;
   ((typename V2<R>::T*)a.s[2])[k] = make2<R>(rho, tait_pterm<Ops>(consts<R>(K), K.gamma, rho));
-  if (sizeof(R) == 8) ((float4*)a.s[3])[k] = make_float4((float)x[0], (float)x[1], (float)x[2], 0.f);
+  pf_store<DIM>(a.pf, k, (float)x[0], (float)x[1], (float)x[2]);
 }
 
 // Packs of the f64 fast (double-word) mode:
-//   s0 {x,y,z,m}.hi (the list kernel's FP32 positions)
+//   pf x.hi, y.hi, z.hi (the list kernel's FP32 positions)
 //   s1 DfRecord {x,y,z,m}.hi, {x,y,z,m}.lo, {vx,vy,vz,0}.hi, {vx,vy,vz,0}.lo (the pair passes)
 //   s4 {rho.hi, rho.lo, P.hi, P.lo}   s5 double {x,y,z} for the exact neighbour test near 2h.
-// Positions in s0 and s1 are shifted (see sph_gather_df).
+// Positions in pf and s1 are shifted (see sph_gather_df).
 
 // p / rho^2 of the Tait law in double-word arithmetic on the FP32 pipe (relative error about
 // 1e-12: (rho/rho0)^gamma - 1 loses the digits its cancellation takes).
@@ -168,7 +168,7 @@ __global__ void sph_gather_df(SphArgs a) {
   df_split_fast(v[1], &bh.y, &bl.y);
   df_split_fast(v[2], &bh.z, &bl.z);
   bh.w = bl.w = 0.f;
-  ((float4*)a.s[0])[k] = ah;
+  pf_store<DIM>(a.pf, k, ah.x, ah.y, ah.z);
   DfRecord rec;
   rec.ah = ah;
   rec.al = al;
@@ -518,12 +518,11 @@ struct DfPairs {
 // ---------------------------------------------------------------------------------------
 // Launch plumbing: one table of kernel instantiations per (arith, dim, stage).
 // ---------------------------------------------------------------------------------------
-typedef void (*PassKernel)(SphArgs, int);
+typedef void (*PassKernel)(SphArgs);
 
 // Kernel table for the list-based passes and the list kernel (stage < 0).
 template <int DIM, int STAGE, int LANES>
-PassKernel list_pass_lanes(int arith, int* pf_index) {
-  *pf_index = 0;
+PassKernel list_pass_lanes(int arith) {
   switch (arith) {
     case ARITH_F64_DF: return sph_list_pass_kernel<DfPairs<DIM, STAGE>, DIM, false, LANES>;
     case ARITH_F32_FAST: return sph_list_pass_kernel<RealPairs<OpsFF, DIM, false, STAGE>, DIM, true, LANES>;
@@ -532,59 +531,61 @@ PassKernel list_pass_lanes(int arith, int* pf_index) {
 }
 
 template <int DIM, int STAGE>
-PassKernel list_pass_for(int arith, int* pf_index, int lanes) {
-  if (lanes == 2) return list_pass_lanes<DIM, STAGE, 2>(arith, pf_index);
-  if (lanes == 4) return list_pass_lanes<DIM, STAGE, 4>(arith, pf_index);
+PassKernel list_pass_for(int arith, int lanes) {
+  if (lanes == 2) return list_pass_lanes<DIM, STAGE, 2>(arith);
+  if (lanes == 4) return list_pass_lanes<DIM, STAGE, 4>(arith);
   switch (arith) {
     case ARITH_F64_EXACT:
-      *pf_index = 3;
       return sph_list_pass_kernel<RealPairs<OpsD, DIM, true, STAGE>, DIM, false>;
     case ARITH_F64_DF:
-      *pf_index = 0;
       return sph_list_pass_kernel<DfPairs<DIM, STAGE>, DIM, false>;
     case ARITH_F32_EXACT:
-      *pf_index = 0;
       return sph_list_pass_kernel<RealPairs<OpsF, DIM, false, STAGE>, DIM, true>;
     case ARITH_F32_FAST:
-      *pf_index = 0;
       return sph_list_pass_kernel<RealPairs<OpsFF, DIM, false, STAGE>, DIM, true>;
     default:
       return nullptr;
   }
 }
 
+// The list kernel with the batch that suits the rows' length (see sph_list_kernel).
+template <int DIM, bool EXACT_PF, int XD>
+PassKernel walk_kernel(int reach) {
+  if constexpr (DIM == 3) {
+    if (reach == 1) return sph_list_kernel<DIM, EXACT_PF, XD, 16>;
+  }
+  return sph_list_kernel<DIM, EXACT_PF, XD, 8>;
+}
+
 template <int DIM>
-PassKernel list_kernel_dim(int arith, int stage, int lanes, int* pf_index) {
+PassKernel list_kernel_dim(int arith, int stage, int lanes, int reach) {
   switch (stage) {
-    case SPH_RATES: return list_pass_for<DIM, SPH_RATES>(arith, pf_index, 1);
-    case SPH_CONT: return list_pass_for<DIM, SPH_CONT>(arith, pf_index, lanes);
-    case SPH_MOM: return list_pass_for<DIM, SPH_MOM>(arith, pf_index, lanes);
+    case SPH_RATES: return list_pass_for<DIM, SPH_RATES>(arith, 1);
+    case SPH_CONT: return list_pass_for<DIM, SPH_CONT>(arith, lanes);
+    case SPH_MOM: return list_pass_for<DIM, SPH_MOM>(arith, lanes);
     default: break;
   }
   switch (arith) {  // the list kernel
     case ARITH_F64_EXACT:  // exact lists (FP32 prefilter, the f64 test in the band): the passes skip the test
-      *pf_index = 3;
-      return sph_list_kernel<DIM, false, 0>;
+      return walk_kernel<DIM, false, 0>(reach);
     case ARITH_F64_DF:  // exact lists: the double-word passes skip the neighbour test
-      *pf_index = 0;
-      return sph_list_kernel<DIM, false, 5>;
+      return walk_kernel<DIM, false, 5>(reach);
     case ARITH_F32_EXACT:
     case ARITH_F32_FAST:
-      *pf_index = 0;
-      return sph_list_kernel<DIM, true, -1>;
+      return walk_kernel<DIM, true, -1>(reach);
     default:
       return nullptr;
   }
 }
 
-PassKernel list_kernel(int arith, int dim, int stage, int lanes, int* pf_index) {
+PassKernel list_kernel(int arith, int dim, int stage, int lanes, int reach) {
   lanes = sph_pass_lanes(arith, stage, lanes);
-  return dim == 2 ? list_kernel_dim<2>(arith, stage, lanes, pf_index)
-                  : list_kernel_dim<3>(arith, stage, lanes, pf_index);
+  return dim == 2 ? list_kernel_dim<2>(arith, stage, lanes, reach)
+                  : list_kernel_dim<3>(arith, stage, lanes, reach);
 }
 
 // lanes: threads per slot of the kernel (1 for the list kernel); a block covers block / lanes slots.
-int launch_table(cudaStream_t st, const SphArgs& a, PassKernel kern, int pf, int grid, int block, int lanes) {
+int launch_table(cudaStream_t st, const SphArgs& a, PassKernel kern, int grid, int block, int lanes) {
   if (!kern) {
     set_error("unknown arithmetic mode or stage");
     return PG_EINVAL;
@@ -601,7 +602,7 @@ int launch_table(cudaStream_t st, const SphArgs& a, PassKernel kern, int pf, int
   const uint32_t spb = (uint32_t)(block / lanes);
   const uint32_t ntiles = (a.k_end + spb - 1) / spb - a.k_begin / spb;
   if (grid <= 0 || (uint32_t)grid > ntiles) grid = (int)ntiles;
-  kern<<<grid, block, 0, st>>>(a, pf);
+  kern<<<grid, block, 0, st>>>(a);
   PG_CUDA_TRY(cudaGetLastError());
   return PG_OK;
 }
@@ -611,12 +612,12 @@ int launch_table(cudaStream_t st, const SphArgs& a, PassKernel kern, int pf, int
 void sph_sorted_layout(int arith, size_t sz[6]) {
   for (int i = 0; i < 6; ++i) sz[i] = 0;
   switch (arith) {
-    case ARITH_F64_EXACT:  // double4 {x,m}, double4 {v,0}, double2 {rho,P}, float4 prefilter positions
-      sz[0] = 32; sz[1] = 32; sz[2] = 16; sz[3] = 16;
+    case ARITH_F64_EXACT:  // double4 {x,m}, double4 {v,0}, double2 {rho,P}
+      sz[0] = 32; sz[1] = 32; sz[2] = 16;
       break;
-    case ARITH_F64_DF:  // float4 A.hi (list kernel), DfRecord {A.hi, A.lo, V.hi, V.lo} (pair passes),
-                        // float4 {rho, P} (hi, lo), double4 exact positions
-      sz[0] = 16; sz[1] = 64; sz[4] = 16; sz[5] = 32;
+    case ARITH_F64_DF:  // DfRecord {A.hi, A.lo, V.hi, V.lo} (pair passes), float4 {rho, P} (hi, lo),
+                        // double4 exact positions
+      sz[1] = 64; sz[4] = 16; sz[5] = 32;
       break;
     default:  // float4 {x,m}, float4 {v,0}, float2 {rho,P}
       sz[0] = 16; sz[1] = 16; sz[2] = 8;
@@ -675,39 +676,36 @@ int launch_sph_repack_rho(cudaStream_t st, const SphArgs& a, int arith) {
 }
 
 int launch_sph_list(cudaStream_t st, const SphArgs& a, int arith, int grid, int block) {
-  int pf = 0;
-  PassKernel kern = list_kernel(arith, a.dim, -1, 1, &pf);
-  return launch_table(st, a, kern, pf, grid, block, 1);
+  PassKernel kern = list_kernel(arith, a.dim, -1, 1, a.reach);
+  return launch_table(st, a, kern, grid, block, 1);
 }
 
-int launch_sph_list_pf(cudaStream_t st, const SphArgs& a, int pf_index, int grid, int block) {
-  PassKernel kern = a.dim == 2 ? sph_list_kernel<2, false, -1> : sph_list_kernel<3, false, -1>;
-  return launch_table(st, a, kern, pf_index, grid, block, 1);
+int launch_sph_list_pf(cudaStream_t st, const SphArgs& a, int grid, int block) {
+  PassKernel kern = a.dim == 2 ? walk_kernel<2, false, -1>(a.reach) : walk_kernel<3, false, -1>(a.reach);
+  return launch_table(st, a, kern, grid, block, 1);
 }
 
-int launch_sph_list_exact(cudaStream_t st, const SphArgs& a, int pf_index, int grid, int block) {
-  PassKernel kern = a.dim == 2 ? sph_list_kernel<2, false, 0> : sph_list_kernel<3, false, 0>;
-  return launch_table(st, a, kern, pf_index, grid, block, 1);
+int launch_sph_list_exact(cudaStream_t st, const SphArgs& a, int grid, int block) {
+  PassKernel kern = a.dim == 2 ? walk_kernel<2, false, 0>(a.reach) : walk_kernel<3, false, 0>(a.reach);
+  return launch_table(st, a, kern, grid, block, 1);
 }
 
 int launch_sph_list_pass(cudaStream_t st, const SphArgs& a, int arith, int stage, int grid, int block, int lanes) {
-  int pf = 0;
   lanes = sph_pass_lanes(arith, stage, lanes);
-  PassKernel kern = list_kernel(arith, a.dim, stage, lanes, &pf);
-  return launch_table(st, a, kern, pf, grid, block, lanes);
+  PassKernel kern = list_kernel(arith, a.dim, stage, lanes, a.reach);
+  return launch_table(st, a, kern, grid, block, lanes);
 }
 
-int sph_list_regs(int arith, int dim, int stage, int lanes) {
-  int pf = 0;
-  PassKernel kern = list_kernel(arith, dim, stage, lanes, &pf);
+int sph_list_regs(int arith, int dim, int reach, int stage, int lanes) {
+  PassKernel kern = list_kernel(arith, dim, stage, lanes, reach);
   cudaFuncAttributes attr;
   if (!kern || cudaFuncGetAttributes(&attr, kern) != cudaSuccess) return 0;
   return attr.numRegs;
 }
 
-int sph_list_occupancy(int arith, int dim, int stage, int block, int lanes) {
-  int pf = 0, blocks = 0;
-  PassKernel kern = list_kernel(arith, dim, stage, lanes, &pf);
+int sph_list_occupancy(int arith, int dim, int reach, int stage, int block, int lanes) {
+  int blocks = 0;
+  PassKernel kern = list_kernel(arith, dim, stage, lanes, reach);
   if (!kern) return 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kern, block, 0) != cudaSuccess) return 0;
   return blocks;

@@ -12,6 +12,7 @@
 #include <stdint.h>
 
 #include "pg_arith.cuh"
+#include "pg_candidates.cuh"
 #include "pg_internal.cuh"
 #include "pg_kernels.cuh"
 
@@ -130,153 +131,160 @@ __device__ __noinline__ bool exact_neighbor_call(const double4_32a* X, uint32_t 
   return exact_neighbor<DIM>(X, k, t, four_h2);
 }
 
-// FP32 r^2 of a candidate, in the operation order of the prefilter (EXACT_PF: IEEE single, no
-// contraction; otherwise with fused multiply-add).
-template <int DIM, bool EXACT_PF>
-__device__ __forceinline__ float candidate_r2(const float4& pi, const float4& pj) {
-  if (EXACT_PF) {
-    const float d0 = __fsub_rn(pi.x, pj.x), d1 = __fsub_rn(pi.y, pj.y);
-    float r2 = __fadd_rn(__fmul_rn(d0, d0), __fmul_rn(d1, d1));
-    if (DIM == 3) {
-      const float d2 = __fsub_rn(pi.z, pj.z);
-      r2 = __fadd_rn(r2, __fmul_rn(d2, d2));
-    }
-    return r2;
-  }
-  const float d0 = pi.x - pj.x, d1 = pi.y - pj.y;
-  float r2 = fmaf(d1, d1, d0 * d0);
-  if (DIM == 3) {
-    const float d2 = pi.z - pj.z;
-    r2 = fmaf(d2, d2, r2);
-  }
-  return r2;
-}
-
-// List membership of a candidate for target k (t != k is tested by the caller).  XD < 0: the FP32
-// prefilter (hit; a superset of the neighbours, the pair passes repeat the exact test).
-// XD >= 0: exactly the oracle's f64 test.  hit: a neighbour for certain; below: under the
-// conservative threshold.  Candidates below but not hit (a narrow band around (2h)^2, and
-// coincident FP32 positions) are left to exact_neighbor on the f64 positions a.s[XD].
+// List membership of candidate t of target k where the packed test did not decide (out of line).
+// XD < 0: the FP32 test (EXACT_PF: the oracle's IEEE test, coincident positions excluded; otherwise the
+// conservative prefilter, whose hits the pair passes test again).  XD >= 0: exactly the oracle's f64
+// test, decided by FP32 outside its band and by the f64 positions a.s[XD] inside.
 template <int DIM, bool EXACT_PF, int XD>
-__device__ __forceinline__ void classify(const float4& pi, const float4& pj, float thr, float thr_lo, bool& hit,
-                                         bool& below) {
-  const float r2 = candidate_r2<DIM, EXACT_PF>(pi, pj);
-  if (XD < 0) {
-    hit = r2 < thr && (!EXACT_PF || r2 > 0.f);
-    below = false;
-  } else {
-    hit = r2 < thr_lo && r2 > 0.f;
-    below = r2 < thr;
-  }
+__device__ __noinline__ bool listed_slow(const float* PF, const double4_32a* X, uint32_t k, uint32_t t, float thr,
+                                         float thr_lo, double four_h2) {
+  if (t == k) return false;
+  const float4 pi = pf_at<DIM>(PF, k), pj = pf_at<DIM>(PF, t);
+  if (XD < 0) return prefilter_hit<DIM, EXACT_PF>(pi, pj, thr);
+  const float d0 = pi.x - pj.x, d1 = pi.y - pj.y, d2 = pi.z - pj.z;
+  const float r2 = DIM == 3 ? fmaf(d2, d2, fmaf(d1, d1, d0 * d0)) : fmaf(d1, d1, d0 * d0);
+  if (r2 < thr_lo && r2 > 0.f) return true;
+  return r2 < thr && exact_neighbor<DIM>(X, k, t, four_h2);
 }
 
 // ---------------------------------------------------------------------------------------
 // Neighbour lists.  sph_list_kernel walks the candidates of every slot once per step and writes
-// the listed slots (classify: with XD < 0 the FP32 test (exact for f32 systems), with XD >= 0
-// exactly the f64 neighbours;
-// never the slot itself) in walk order (rows z, then y ascending; slots ascending along a row)
-// to nlist in warp tiles (list_base: entry q of the 32 slots of a tile is one 128-byte line, so a
-// warp's reads of one entry index coalesce and its writes fill whole sectors while they are in
-// L2); nlen[k] = number of listed slots (may exceed cap).  When the list fills, nresume[2k],
-// [2k+1] = (row, slot) of the first listed candidate that did not fit, so the pair passes can
-// continue the walk from there.
+// the listed slots (with XD < 0 the FP32 test (exact for f32 systems), with XD >= 0 exactly the
+// f64 neighbours; never the slot itself) in walk order (rows z, then y ascending; slots ascending
+// along a row) to nlist in warp tiles (list_base: entry q of the 32 slots of a tile is one
+// 128-byte line, so a warp's reads of one entry index coalesce and its writes fill whole sectors
+// while they are in L2); nlen[k] = number of listed slots (may exceed cap).  When the list fills,
+// nresume[2k], [2k+1] = (row, slot) of the first listed candidate that did not fit, so the pair
+// passes can continue the walk from there.
 //
-// Each lane walks its own rows, kListBatch candidates at a time: loads without a clamp (the
-// packs are padded by kPackPad records), the FP32 classification folded into bit masks, the rare
-// f64 band tests once per batch, then the pushes of the batch's hits in order.  The next row's
-// slot range is loaded while the current row is walked.  Lanes whose targets share a cell walk
-// the same candidates in step, so their loads coalesce (pruning each lane's rows to the cells
-// its own target can reach was measured: it breaks that, and the walk got slower).
+// Each lane walks its own rows, B candidates at a time (screen_batch: packed FP32 tests of
+// consecutive slots), then stores the batch's hits in order; the lanes of a warp keep to the same
+// row number, so the row bookkeeping runs once per row and warp.  What bounds it is instruction
+// issue (and, through it, the latency of the loads), so the test is kept short: one sign bit per
+// candidate decides, and one minimum per batch says whether every decision was certain.  The
+// candidates near (2h)^2 or coincident with the target
+// are decided one at a time (listed_slow).  The next batch is loaded before the hits of the
+// current one are stored, the next row's slot range while the current row is walked.  Lanes whose
+// targets share a cell walk the same candidates in step, so their loads coalesce (pruning each
+// lane's rows to the cells its own target can reach was measured: it breaks that, and the walk got
+// slower).
+//
+// B: long rows (3D with a reach of one cell, about 50 slots a row) take 16 candidates a batch, short
+// ones (3D with a reach of two, about 11; 2D, about 17) take 8.  ms per build with 8 / 16: 3D
+// 700k particles f32, reach 1 0.366 / 0.317; 262k f64, reach 2 0.113 / 0.126; 2D 6.1M 0.284 / 0.296
+// (the lists of the first 70 % of the slots).
+// Against the walk over {x, y, z, w} records, 16 to a batch, with two compares per candidate and
+// each lane at its own row: 262k 0.153 -> 0.113 ms, f32 700k 0.412 -> 0.317, 4M (first 70 %) 1.39 -> 1.19.
 // ---------------------------------------------------------------------------------------
-constexpr int kListBatch = 16;
-static_assert(kPackPad >= (size_t)kListBatch - 1, "sorted packs must be padded for a whole batch past the end");
 
 // Offset of slot k's entry 0 in the tiled list array (entry q at + q * kListTile).
 __device__ __forceinline__ size_t list_base(uint32_t k, uint32_t cap) {
   return (size_t)(k / kListTile) * cap * kListTile + (k % kListTile);
 }
 
-__device__ __forceinline__ void list_push(const SphArgs& a, uint32_t* my, uint32_t& cnt, uint32_t k, int row,
-                                          uint32_t t) {
-  if (cnt < a.cap) {
-    my[(size_t)cnt * kListTile] = t;
-  } else if (cnt == a.cap) {
-    a.nresume[2 * (size_t)k] = (uint32_t)row;
-    a.nresume[2 * (size_t)k + 1] = t;
-  }
-  ++cnt;
-}
-
-template <int DIM, bool EXACT_PF, int XD>
-__global__ void __launch_bounds__(kSphMaxThreads) sph_list_kernel(SphArgs a, int pf_index) {
+template <int DIM, bool EXACT_PF, int XD, int B>
+__global__ void __launch_bounds__(kSphMaxThreads) sph_list_kernel(SphArgs a) {
   const int tid = threadIdx.x;
-  const float4* __restrict__ PF = (const float4*)a.s[pf_index];
+  const float* __restrict__ PF = a.pf;
   const double4_32a* __restrict__ X = (const double4_32a*)a.s[XD < 0 ? 0 : XD];
   const uint32_t* __restrict__ start = a.cell_start;
   const int R = a.reach;
   const int RZ = DIM == 3 ? R : 0;
-  const int side = 2 * R + 1;
-  const int nrows = side * (2 * RZ + 1);
+  const int nrows = (2 * R + 1) * (2 * RZ + 1);
   const uint32_t bs = blockDim.x;
   const uint32_t tile1 = (a.k_end + bs - 1) / bs;
+  constexpr unsigned kAll = (1u << B) - 1;
 
   for (uint32_t tile = a.k_begin / bs + blockIdx.x; tile < tile1; tile += gridDim.x) {
     const SphK* Kp;
     const Target T = target_of(a, tile * bs + tid, &Kp, R);
     const SphK& K = *Kp;
     const GridK& g = K.g;
-    const float4 pi = PF[T.k];
+    const float4 pi = pf_at<DIM>(PF, T.k);
     const float thr = prefilter_threshold<EXACT_PF>(K, pi);
-    const float thr_lo = XD < 0 ? 0.f : certain_threshold(K, pi);
+    const float thr_lo = XD < 0 ? thr : certain_threshold(K, pi);
+    Screen S;
+    screen_target(S, pi);
+    if (EXACT_PF) screen_exact(S, thr);
+    else screen_band(S, thr_lo, thr);
     uint32_t* __restrict__ my = a.nlist + list_base(T.k, a.cap);  // entry q at my[q * kListTile]
     uint32_t cnt = 0;
-    // slot range of a row (empty outside the grid); the next row's range is loaded while the
-    // current row is walked
-    auto row_range = [&](int r, uint32_t& a, uint32_t& b) {
-      const int z = T.cz + r / side - RZ, y = T.cy + r % side - R;
-      a = b = 0;
-      if (T.live && z >= 0 && z < g.nz && y >= 0 && y < g.ny) {
-        const uint32_t rb = g.cell_base + ((uint32_t)z * g.ny + (uint32_t)y) * g.nx;
-        a = start[rb + T.x0];
-        b = start[rb + T.x1 + 1];
+    // The (2R + 1)^(DIM - 1) rows, z then y ascending, in step for the whole warp (the row number is
+    // uniform; a row outside the grid is empty).  tn, en: the slot range of row `row + 1`.
+    uint32_t tn = 0, en = 0;
+    int y = T.cy - R, z = T.cz - RZ;
+    uint32_t rb = g.cell_base + (uint32_t)((z * g.ny + y) * g.nx);  // wraps below 0 outside the grid (not read)
+    auto load_range = [&]() {
+      tn = en = 0;
+      if (T.live && (unsigned)y < (unsigned)g.ny && (unsigned)z < (unsigned)g.nz) {
+        tn = start[rb + T.x0];
+        en = start[rb + T.x1 + 1];
       }
     };
-    int row = -1, nxt = 0;
-    uint32_t t = 0, e = 0, tn, en;
-    row_range(0, tn, en);
-    while (true) {
-      while (t >= e && nxt < nrows) {
-        t = tn;
-        e = en;
-        row = nxt++;
-        if (nxt < nrows) row_range(nxt, tn, en);
-      }
-      if (t >= e) break;
-      // the batch's candidates that belong to the row, the target itself left out (the packs
-      // are padded by kPackPad records, so the loads need no clamp)
-      unsigned valid = e - t >= (uint32_t)kListBatch ? (1u << kListBatch) - 1 : (1u << (e - t)) - 1;
-      if (T.k - t < (uint32_t)kListBatch) valid &= ~(1u << (T.k - t));
-      const float4* __restrict__ pb = PF + t;
-      float4 pj[kListBatch];
-#pragma unroll
-      for (int b = 0; b < kListBatch; ++b) pj[b] = __ldg(pb + b);
-      unsigned hit = 0, below = 0;
-#pragma unroll
-      for (int b = 0; b < kListBatch; ++b) {
-        bool h, m;
-        classify<DIM, EXACT_PF, XD>(pi, pj[b], thr, thr_lo, h, m);
-        if (h) hit |= 1u << b;
-        if (m) below |= 1u << b;
-      }
-      hit &= valid;
-      if (XD >= 0) {
-        for (unsigned m = below & ~hit & valid; m; m &= m - 1) {
-          const int b = __ffs(m) - 1;
-          if (exact_neighbor<DIM>(X, T.k, t + b, K.d.four_h2)) hit |= 1u << b;
+    load_range();
+    Batch<DIM, B> batch;
+    bool loaded = false;  // batch holds the next row's first batch
+    for (int row = 0; row < nrows; ++row) {
+      uint32_t t = tn & ~3u;  // the batch's first slot, a multiple of 4
+      const uint32_t e = tn < en ? en : 0u;
+      unsigned lead = kAll >> (tn & 3u);  // valid bits of the batch's slots from the row's first on
+      if (!loaded && t < e) batch.load(PF, t);
+      loaded = false;
+      if (row + 1 < nrows) {
+        if (++y > T.cy + R) {
+          y = T.cy - R;
+          ++z;
+          rb += (uint32_t)((g.ny - 2 * R) * g.nx);
+        } else {
+          rb += (uint32_t)g.nx;
         }
+        load_range();
+      } else {
+        tn = en = 0;
       }
-      for (; hit; hit &= hit - 1) list_push(a, my, cnt, T.k, row, t + __ffs(hit) - 1);
-      t += kListBatch;
+      while (t < e) {
+        // the batch's candidates that belong to the row, the target itself left out
+        unsigned valid = lead;
+        if (e - t < (uint32_t)B) valid &= ~(kAll >> (e - t));
+        if (T.k - t < (uint32_t)B) valid &= ~((kAll + 1) / 2 >> (T.k - t));
+        unsigned open;
+        unsigned hit = screen_batch<DIM, B, !EXACT_PF, !EXACT_PF>(batch, S, open) & valid;
+        const uint32_t first = t;
+        lead = kAll;
+        t += B;
+        // the next batch (of this row, or the next row's first), in flight while the hits are stored
+        loaded = t >= e && tn < en;
+        if (t < e || loaded) batch.load(PF, t < e ? t : tn & ~3u);
+        open &= valid;
+        for (hit &= ~open; open; open &= open - 1) {
+          const int b = B - __ffs(open);
+          if (listed_slow<DIM, EXACT_PF, XD>(PF, X, T.k, first + b, thr, thr_lo, K.d.four_h2)) hit |= open & -open;
+        }
+        if (!hit) continue;
+        const uint32_t end = cnt + __popc(hit);
+        if (end <= a.cap) {
+          uint32_t* __restrict__ out = my + (size_t)cnt * kListTile;
+#pragma unroll
+          for (int b = 0; b < B; ++b)
+            if (hit >> (B - 1 - b) & 1u) {
+              *out = first + b;
+              out += kListTile;
+            }
+        } else {  // the list is full, or becomes so within this batch
+          for (uint32_t q = cnt; hit; ++q) {
+            const int b = 31 - __clz(hit);
+            hit ^= 1u << b;
+            const uint32_t c = first + B - 1 - b;
+            if (q < a.cap) {
+              my[(size_t)q * kListTile] = c;
+            } else if (q == a.cap) {
+              a.nresume[2 * (size_t)T.k] = (uint32_t)row;
+              a.nresume[2 * (size_t)T.k + 1] = c;
+            }
+          }
+        }
+        cnt = end;
+      }
     }
     if (T.live) a.nlen[T.k] = cnt;
   }
@@ -319,7 +327,7 @@ struct PrefetchPolicy<P, decltype((void)P::kPrefetch)> {
 // through their lists together; a list that overflowed is followed by the rest of the walk from
 // its resume point (lane 0).
 template <class Pairs, int DIM, bool EXACT_PF, int LANES = 1>
-__global__ void __launch_bounds__(kSphMaxThreads) sph_list_pass_kernel(SphArgs a, int pf_index) {
+__global__ void __launch_bounds__(kSphMaxThreads) sph_list_pass_kernel(SphArgs a) {
   static_assert(LANES == 1 || LANES == 2 || LANES == 4, "1, 2 or 4 lanes per slot");
   const int tid = threadIdx.x;
   const uint32_t cap = a.cap;
@@ -363,12 +371,12 @@ __global__ void __launch_bounds__(kSphMaxThreads) sph_list_pass_kernel(SphArgs a
     }
     if (cnt > cap && sub == 0) {
       // rare: continue the candidate walk where the list stopped
-      const float4* __restrict__ PF = (const float4*)a.s[pf_index];
+      const float* __restrict__ PF = a.pf;
       const SphK* Kp;
       const Target T = target_of(a, k0, &Kp, a.reach);
       const GridK& g = K.g;
       const int R = a.reach, RZ = DIM == 3 ? R : 0, side = 2 * R + 1, nrows = side * (2 * RZ + 1);
-      const float4 pi = PF[k];
+      const float4 pi = pf_at<DIM>(PF, k);
       const float thr = prefilter_threshold<EXACT_PF>(K, pi);
       const int row0 = (int)a.nresume[2 * (size_t)k];
       const uint32_t t0 = a.nresume[2 * (size_t)k + 1];
@@ -378,7 +386,7 @@ __global__ void __launch_bounds__(kSphMaxThreads) sph_list_pass_kernel(SphArgs a
         const uint32_t rb = g.cell_base + ((uint32_t)z * g.ny + (uint32_t)y) * g.nx;
         const uint32_t e = a.cell_start[rb + T.x1 + 1];
         for (uint32_t t = row == row0 ? t0 : a.cell_start[rb + T.x0]; t < e; ++t)
-          if (prefilter_hit<DIM, EXACT_PF>(pi, PF[t], thr)) P.pair(t);
+          if (prefilter_hit<DIM, EXACT_PF>(pi, pf_at<DIM>(PF, t), thr)) P.pair(t);
       }
     }
     if constexpr (LANES > 1) P.template reduce_lanes<LANES>();  // whole warps: the tile loop is uniform
