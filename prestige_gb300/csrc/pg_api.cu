@@ -205,6 +205,7 @@ NbrArgs nbr_args(pg_system* s) {
   a.sorted_id = s->nw.sorted_id;
   a.cell_start = s->nw.cell_start.as<uint32_t>();
   a.spos = s->spos.p;
+  a.pf = s->spf.as<float>();
   return a;
 }
 
@@ -1178,6 +1179,7 @@ int pg_build_neighbors(pg_system* s) {
   PG_TRY(check(s));
   PG_TRY(pg::enqueue_neighbors(s));
   PG_TRY(s->spos.ensure((s->f64 ? 32 : 16) * (s->n ? s->n : 1)));
+  PG_TRY(s->spf.ensure(4 * chunked_floats(s->n, s->dim)));
   NbrArgs a = pg::nbr_args(s);
   PG_TRY(pg::launch_sorted_positions(s->stream, a, s->pos.p, s->spos.p));
   PG_CUDA_TRY(cudaStreamSynchronize(s->stream));
@@ -1495,7 +1497,7 @@ int pg_memory_bytes(pg_system* s, size_t* bytes) {
                               &s->contacts, &s->err};
   for (const pg::DevBuf* d : bufs) b += d->bytes;
   for (int i = 0; i < 6; ++i) b += s->sorted[i].bytes;
-  b += s->pf.bytes;
+  b += s->pf.bytes + s->spf.bytes;
   b += s->nlist.bytes + s->nlen.bytes + s->nresume.bytes + s->fcache.bytes;
   for (auto& kv : s->user) b += kv.second->bytes;
   b += s->adjoint_bytes();

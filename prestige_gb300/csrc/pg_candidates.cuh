@@ -84,6 +84,23 @@ struct Batch {
   }
 };
 
+// Bounds on the FP32 r^2 of a candidate of a target at p (FP32 positions rounded from f64; reach: at
+// least the support radius in FP32):  |x_j - x_i| < reach in f64  =>  r^2 < outer_threshold, and
+// r^2 < inner_threshold  =>  |x_j - x_i| < reach in f64.  delta bounds the rounding of the
+// positions and of the FP32 arithmetic with a generous factor.
+__device__ __forceinline__ float outer_threshold(float reach, const float4& p) {
+  const float M = fmaxf(fmaxf(fabsf(p.x), fabsf(p.y)), fabsf(p.z)) + reach;
+  const float delta = 2.384185791015625e-07f * (2.f * M + reach);  // 4u (2M + reach)
+  const float rr = reach + 2.f * delta;
+  return rr * rr * 1.0000153f;
+}
+__device__ __forceinline__ float inner_threshold(float reach, const float4& p) {
+  const float M = fmaxf(fmaxf(fabsf(p.x), fabsf(p.y)), fabsf(p.z)) + reach;
+  const float delta = 2.384185791015625e-07f * (2.f * M + reach);
+  const float rr = fmaxf(reach - 2.f * delta, 0.f);
+  return rr * rr * 0.9999847f;
+}
+
 // The FP32 test of one target against thresholds on r^2.  With
 // s = r^2 / mid - 1 (RATIO) or r^2 - mid (exact sign), a candidate is inside when s < 0.  Candidates
 // with |r^2 s| <= tol are not decided by FP32 (r^2 close to mid, or zero, or tiny against it).

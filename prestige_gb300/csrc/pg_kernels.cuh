@@ -144,6 +144,7 @@ struct NbrArgs {
   const uint32_t* sorted_id;
   const uint32_t* cell_start;
   const void* spos;           // sorted positions: double4_32a or float4 (x, y, z, 0)
+  float* pf;                  // the same rounded to FP32, in chunks (pg_candidates.cuh)
 };
 
 int launch_sorted_positions(cudaStream_t st, const NbrArgs& a, const void* pos, void* spos);

@@ -70,16 +70,10 @@ __device__ __forceinline__ Target target_of(const SphArgs& a, uint32_t k0, const
   return T;
 }
 
-// FP32 threshold on r^2.  EXACT_PF (f32 systems): the exact test.  Otherwise a conservative
-// bound: |x_j - x_i| < 2h in f64  =>  the FP32 r^2 below is < thr (rounding of positions to
-// float and of the FP32 arithmetic bounded with a generous factor).
+// FP32 threshold on r^2.  EXACT_PF (f32 systems): the exact test.  Otherwise the conservative bound.
 template <bool EXACT_PF>
 __device__ __forceinline__ float prefilter_threshold(const SphK& K, const float4& pi) {
-  if (EXACT_PF) return K.f.four_h2;
-  const float M = fmaxf(fmaxf(fabsf(pi.x), fabsf(pi.y)), fabsf(pi.z)) + K.two_h_f;
-  const float delta = 2.384185791015625e-07f * (2.f * M + K.two_h_f);  // 4u (2M + 2h)
-  const float rr = K.two_h_f + 2.f * delta;
-  return rr * rr * 1.0000153f;
+  return EXACT_PF ? K.f.four_h2 : outer_threshold(K.two_h_f, pi);
 }
 
 template <int DIM, bool EXACT_PF>
@@ -100,15 +94,6 @@ __device__ __forceinline__ bool prefilter_hit(const float4& pi, const float4& pj
     r2 = fmaf(d2, d2, r2);
   }
   return r2 < thr;
-}
-
-// FP32 r^2 below which |x_j - x_i| < 2h holds in f64 for certain: the mirror image of
-// prefilter_threshold (same error bound delta, taken off instead of added).
-__device__ __forceinline__ float certain_threshold(const SphK& K, const float4& pi) {
-  const float M = fmaxf(fmaxf(fabsf(pi.x), fabsf(pi.y)), fabsf(pi.z)) + K.two_h_f;
-  const float delta = 2.384185791015625e-07f * (2.f * M + K.two_h_f);
-  const float rr = fmaxf(K.two_h_f - 2.f * delta, 0.f);
-  return rr * rr * 0.9999847f;
 }
 
 // The oracle's f64 neighbour test of slots k and t (positions X, double4 per slot); inline in
@@ -202,7 +187,7 @@ __global__ void __launch_bounds__(kSphMaxThreads) sph_list_kernel(SphArgs a) {
     const GridK& g = K.g;
     const float4 pi = pf_at<DIM>(PF, T.k);
     const float thr = prefilter_threshold<EXACT_PF>(K, pi);
-    const float thr_lo = XD < 0 ? thr : certain_threshold(K, pi);
+    const float thr_lo = XD < 0 ? thr : inner_threshold(K.two_h_f, pi);
     Screen S;
     screen_target(S, pi);
     if (EXACT_PF) screen_exact(S, thr);

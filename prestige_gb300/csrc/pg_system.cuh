@@ -47,7 +47,7 @@ struct pg_system {
   bool stage_pending = false;  // pg_step_stage(0) ran; pg_step_stage(1) may follow
   pg::DevBuf sorted[6];
   pg::DevBuf pf;                 // FP32 positions of the candidate walks, in chunks
-  pg::DevBuf spos;
+  pg::DevBuf spos, spf;
   pg::DevBuf tmp, tmp2, tmp3, tmp4;
   int pass_grid[3] = {0, 0, 0};  // per SphStage
   int list_grid = 0;

@@ -91,3 +91,37 @@ def test_nan_position_has_no_neighbours(pg, mode):
         assert 7 not in got
         if ids[k] == 7:
             assert lengths[k] == 0
+
+
+# (dim, offset of all positions, scale of positions and support): ordinary; FP32 positions that resolve
+# the support poorly or not at all; squares of the support outside the FP32 range
+_SCALES = [(2, 0.0, 1.0), (3, 0.0, 1.0), (3, 1e5, 1.0), (3, 1e8, 1.0), (2, 0.0, 1e-22), (3, 0.0, 1e22)]
+
+
+@pytest.mark.parametrize("f64", [True, False])
+@pytest.mark.parametrize("mult", [1.0, 0.5])
+@pytest.mark.parametrize("dim,offset,scale", _SCALES)
+def test_counts_lists_and_gather(pg, oracle, dim, offset, scale, mult, f64):
+    if not f64 and (offset or scale != 1.0):
+        pytest.skip("f32 systems use the IEEE FP32 test at any scale")
+    for n in (1, 4, 9, 17, 33, 64, 150):
+        rng = np.random.default_rng(n + dim)
+        side = max(0.3, (n / 30.0) ** (1.0 / dim) * 0.4)
+        pos = (rng.uniform(0.0, side, size=(n, dim)) + 0.05) * scale + offset
+        if n > 4:
+            pos[n - 1] = pos[2]
+        h = 0.1 * scale
+        lo, hi = [offset] * 3, [offset + 2.0 * scale] * 3
+        cfg = dict(model=0, dim=dim, precision=1 if f64 else 0, h=h, cell_multiplier=mult, domain_lo=lo, domain_hi=hi)
+        s = ParticleSystem(make_config(**cfg), n)
+        s.set("pos", pos)
+        src, dst = rng.normal(size=n), rng.normal(size=n)
+        s.set("src", src)
+        s.set("dst", dst)
+        assert np.array_equal(s.count_neighbors(), oracle.neighbor_counts(pos, lo, hi, 2.0 * h, mult, f64=f64))
+        offs, nbr = s.neighbor_list()
+        ro, rn = oracle.neighbor_list(pos, lo, hi, 2.0 * h, mult, f64=f64)
+        assert np.array_equal(offs, ro) and np.array_equal(nbr, rn)
+        s.gather_sum("dst", "src")
+        assert np.array_equal(s.get("dst"), oracle.gather_sum(pos, lo, hi, 2.0 * h, src, dst, mult, f64=f64))
+        s.close()
