@@ -696,7 +696,7 @@ int pg_backward(pg_system* s, const double* dL_dx, double* dL_dalpha, double* dL
         PG_CUDA_TRY(cudaMemcpyAsync(A->seg_id[b].as<uint32_t>() + (size_t)t * n, s->nw.sorted_id, 4 * n,
                                     cudaMemcpyDeviceToDevice, s->stream));
       }
-      PG_CUDA_TRY(cudaMemcpyAsync(A->seg_start[b].as<uint32_t>() + (size_t)t * ncp1, s->nw.cell_start.p, 4 * ncp1,
+      PG_CUDA_TRY(cudaMemcpyAsync(A->seg_start[b].as<uint32_t>() + (size_t)t * ncp1, s->nw.cell_start, 4 * ncp1,
                                   cudaMemcpyDeviceToDevice, s->stream));
     }
     PG_CUDA_TRY(cudaEventRecord(A->ev_rec[b], s->stream));

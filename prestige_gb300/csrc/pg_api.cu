@@ -155,7 +155,7 @@ int ensure_sorted_buffers(pg_system* s) {
   if (s->arith == ARITH_F64_EXACT) PG_TRY(s->fcache.ensure(sph_sym_entry_bytes() * entries));
   PG_TRY(s->nlen.ensure(4 * n));
   PG_TRY(s->nresume.ensure(8 * n));
-  PG_TRY(s->posmin.ensure(3 * sizeof(unsigned long long) * (size_t)s->nsys));
+  PG_TRY(s->posmin.ensure(2 * 3 * sizeof(unsigned long long) * (size_t)s->nsys));  // minima, accumulators
   return PG_OK;
 }
 
@@ -169,7 +169,8 @@ SphArgs sph_args(pg_system* s, int integrate, bool rates) {
   a.reach = s->grids[0].reach;
   a.sorted_cell = s->nw.sorted_cell;
   a.sorted_id = s->nw.sorted_id;
-  a.cell_start = s->nw.cell_start.as<uint32_t>();
+  a.cell_start = s->nw.cell_start;
+  a.order = nbr_order(s->nw);
   for (int i = 0; i < 6; ++i) a.s[i] = s->sorted[i].p;
   a.pf = s->pf.as<float>();
   a.s[6] = a.s[7] = nullptr;
@@ -203,32 +204,49 @@ NbrArgs nbr_args(pg_system* s) {
   a.f64 = s->f64;
   a.sorted_cell = s->nw.sorted_cell;
   a.sorted_id = s->nw.sorted_id;
-  a.cell_start = s->nw.cell_start.as<uint32_t>();
+  a.cell_start = s->nw.cell_start;
+  a.order = nbr_order(s->nw);
   a.spos = s->spos.p;
   a.pf = s->spf.as<float>();
   return a;
 }
 
-// Hash + stable sort + cell table for the current positions (enqueued on the stream).
+// Counts and minima of the neighbour search rest at zero and all ones between searches (each search
+// restores them, so a step needs no memsets).  Set here before the first search, and after one that
+// was not enqueued whole.
+int rest_neighbors(pg_system* s) {
+  NbrWork& w = s->nw;
+  if (w.clean) return PG_OK;
+  PG_CUDA_TRY(cudaMemsetAsync(w.rest, 0, 4 * w.rest_words, s->stream));
+  if (s->posmin.p) PG_CUDA_TRY(cudaMemsetAsync(s->posmin.p, 0xff, s->posmin.bytes, s->stream));
+  w.clean = true;
+  return PG_OK;
+}
+
+// Cells, cell table and the ids grouped by cell for the current positions (enqueued on the stream);
+// every caller goes on with a sorted gather, which puts each cell's ids in order (ordered_slot).
 int enqueue_neighbors(pg_system* s) {
   s->stage_pending = false;  // any neighbour search ends a pending pg_step_stage(0)
-  const void* pos = s->pos.p;
-  // the double-word packs need each system's minimum position of the step (sph_gather_df)
-  unsigned long long* posmin = nullptr;
-  if (s->model == PG_MODEL_SPH && s->arith == ARITH_F64_DF && s->posmin.p) {
-    posmin = s->posmin.as<unsigned long long>();
-    PG_CUDA_TRY(cudaMemsetAsync(posmin, 0xff, 3 * sizeof(unsigned long long) * (size_t)s->nsys, s->stream));
-  }
+  NbrWork& w = s->nw;
+  // the double-word packs need each system's minimum position of the step (sph_gather_df): folded
+  // into posacc by the hash, moved to posmin by the scan
+  const bool mins = s->model == PG_MODEL_SPH && s->arith == ARITH_F64_DF && s->posmin.p;
+  const uint32_t nmin = 3u * (uint32_t)s->nsys;
+  unsigned long long* posmin = mins ? s->posmin.as<unsigned long long>() : nullptr;
+  unsigned long long* posacc = mins ? posmin + nmin : nullptr;
+  PG_TRY(rest_neighbors(s));
+  w.clean = false;
   PG_TRY(launch_hash(s->stream, s->gridk.as<GridK>(), s->nsys > 1 ? s->sys_of_id.as<uint32_t>() : nullptr, s->f64,
-                     s->dim, pos, s->n, s->nw.keys[0].as<uint32_t>(), s->nw.vals[0].as<uint32_t>(), posmin));
-  PG_TRY(sort_and_table(s->stream, s->nw));
+                     s->dim, s->pos.p, w, posacc));
+  PG_TRY(launch_sort(s->stream, w, posacc, posmin, nmin));
+  w.clean = true;
   return PG_OK;
 }
 
 int mom_block(const pg_system* s) { return s->block_mom > 0 ? s->block_mom : s->block; }
 
-// Kernels enqueued by one neighbour search (hash, radix passes, cell-start table).
-long long neighbor_launches(const pg_system* s) { return 1 + 3LL * s->nw.passes + 1; }
+// Kernels enqueued by one neighbour search (hash, reduce, scan, scatter).
+long long neighbor_launches(const pg_system* s) { return s->nw.chunks > 1 ? 4 : 3; }
 
 // The continuity part of a step: neighbour search, sorted gather, neighbour lists and the
 // continuity pass (rho' into the canonical density and the sorted pack).  ev (optional): events
@@ -360,7 +378,8 @@ DemArgs dem_args(pg_system* s) {
   a.reach = s->grids[0].reach;
   a.sorted_cell = s->nw.sorted_cell;
   a.sorted_id = s->nw.sorted_id;
-  a.cell_start = s->nw.cell_start.as<uint32_t>();
+  a.cell_start = s->nw.cell_start;
+  a.order = nbr_order(s->nw);
   a.sA = s->sorted[0].as<double4_32a>();
   a.sB = s->sorted[1].as<double4_32a>();
   a.sW = s->sorted[2].as<double4_32a>();
@@ -442,6 +461,7 @@ int timing_collect(pg_system* s) {
 
 // One full step, enqueued; flips the DEM history buffers.
 int enqueue_step(pg_system* s) {
+  PG_TRY(rest_neighbors(s));
   cudaEvent_t* ev = nullptr;
   if (s->timing) PG_TRY(timing_events(s, &ev));
   if (s->model == PG_MODEL_DEM) {
@@ -490,6 +510,7 @@ void drop_graphs(pg_system* s) {
 
 int capture_graphs(pg_system* s) {
   drop_graphs(s);
+  PG_TRY(rest_neighbors(s));  // outside the captured step
   const int ngraphs = s->model == PG_MODEL_DEM ? 2 : 1;
   const int hsave = s->hcur;
   for (int gi = 0; gi < ngraphs; ++gi) {
@@ -1212,7 +1233,7 @@ int pg_get_neighbors(pg_system* s, uint32_t* cell_sorted, uint32_t* ids_sorted, 
     PG_CUDA_TRY(cudaMemcpy(cell_sorted, s->nw.sorted_cell, 4 * s->n, cudaMemcpyDeviceToHost));
   if (ids_sorted && s->n) PG_CUDA_TRY(cudaMemcpy(ids_sorted, s->nw.sorted_id, 4 * s->n, cudaMemcpyDeviceToHost));
   if (cell_start)
-    PG_CUDA_TRY(cudaMemcpy(cell_start, s->nw.cell_start.p, 4 * (s->ncells + 1), cudaMemcpyDeviceToHost));
+    PG_CUDA_TRY(cudaMemcpy(cell_start, s->nw.cell_start, 4 * (s->ncells + 1), cudaMemcpyDeviceToHost));
   return PG_OK;
 }
 

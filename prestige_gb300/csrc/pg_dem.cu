@@ -163,9 +163,10 @@ __device__ __forceinline__ void history_lookup(const uint32_t* hp, const double*
 }
 
 __global__ void dem_gather_kernel(DemArgs a) {
-  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= a.n) return;
-  const uint32_t id = a.sorted_id[k];
+  const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= a.n) return;
+  uint32_t id;
+  const uint32_t k = ordered_slot(a.order, s, id);
   const size_t o = (size_t)id * 3;
   a.sA[k] = make_double4_32a(a.pos[o], a.pos[o + 1], a.pos[o + 2], a.radius[id]);
   a.sB[k] = make_double4_32a(a.vel[o], a.vel[o + 1], a.vel[o + 2], a.mass[id]);

@@ -4,7 +4,7 @@
 // concatenated in id order):
 //   canonical state, particle-id order   pos[n*dim], vel[n*dim], rho[n], mass[n]   (SPH)
 //                                        pos, vel, omega[n*3], radius[n], mass[n]  (DEM)
-//   neighbour search, every step         cell of each id -> stable LSD radix sort by cell
+//   neighbour search, every step         cell of each id -> stable counting sort by cell
 //                                        -> sorted_cell[k], sorted_id[k] (slot k)
 //                                        cell_start[c], n_cells + 1 entries
 //   sorted packed copies, slot order     read by the pair kernels (coalesced, shared in L1)
@@ -94,29 +94,64 @@ struct GridK {
 GridK grid_k(const Grid& g, uint32_t cell_base);
 
 // ---------------------------------------------------------------------------------------
-// Neighbour-search workspace: stable LSD radix sort of (cell, id) and the cell table.
+// Neighbour-search workspace: stable counting sort of the particles by cell, and the cell table
+// (pg_sort.cu).
 // ---------------------------------------------------------------------------------------
+constexpr uint32_t kScanChunk = 8192;  // cells per block of the scan
+constexpr uint32_t kBigCell = 1024;    // particles of a cell that one block sorts (see pg_sort.cu)
+
 struct NbrWork {
   size_t n = 0;
   uint64_t ncells = 0;
-  int passes = 0;
-  int tiles = 0;
-  int items = 16;  // keys per thread of the radix kernels (tiles of 256 * items keys)
-  DevBuf keys[2], vals[2];  // u32
-  DevBuf hist;              // u32 [256 * tiles]
-  DevBuf digit_total;       // u32 [256]
-  DevBuf cell_start;        // u32 [ncells + 1]
-  uint32_t* sorted_cell = nullptr;
-  uint32_t* sorted_id = nullptr;
+  int passes = 0;      // 8-bit digits of a cell index
+  uint32_t chunks = 0; // scan chunks: cover ncells + 1 entries
+  DevBuf mem;          // all arrays below
+  uint32_t *key = nullptr, *rank = nullptr, *unsorted = nullptr;  // [n] cell and arrival rank of each id; ids by cell
+  uint32_t *sorted_cell = nullptr, *sorted_id = nullptr;          // [n] cell and id of each sorted slot
+  uint32_t* cell_start = nullptr;   // [ncells + 1], padded to whole chunks
+  uint32_t* chunk_total = nullptr;  // [chunks] particles per chunk
+  uint32_t* rest = nullptr;         // the arrays that are zero between searches, rest_words in all:
+  uint32_t* count = nullptr;        //   [chunks * kScanChunk] particles per cell
+  uint32_t* big = nullptr;          //   {cells listed, blocks done, cell indices ...}
+  size_t rest_words = 0;
+  bool clean = false;  // count, big and the position minima hold their rest values
   int init(size_t n, uint64_t ncells);
   size_t bytes() const;
 };
 
-// Cell key and id of every particle (id order) into w.keys[0] / w.vals[0].
+// What a sorted-gather kernel needs to finish the sort: ordered_slot() gives each thread the particle
+// and the final slot of one entry of `unsorted`, and records both.
+struct NbrOrder {
+  const uint32_t* unsorted;
+  const uint32_t* key;
+  const uint32_t* cell_start;
+  uint32_t* sorted_cell;
+  uint32_t* sorted_id;
+};
+NbrOrder nbr_order(const NbrWork& w);
+
+// Within a cell the scatter left the ids in arrival order: an id's slot is the cell's first plus the
+// number of smaller ids in the cell, so equal cells end up in id order (the stable order).  Cells of
+// more than kBigCell particles are in id order already.
+__device__ __forceinline__ uint32_t ordered_slot(const NbrOrder& o, uint32_t s, uint32_t& id) {
+  id = o.unsorted[s];
+  const uint32_t c = o.key[id];
+  const uint32_t b = o.cell_start[c], e = o.cell_start[c + 1];
+  uint32_t k = s;
+  if (e - b <= kBigCell) {
+    k = b;
+    for (uint32_t q = b; q < e; ++q) k += o.unsorted[q] < id ? 1u : 0u;
+  }
+  o.sorted_id[k] = id;
+  o.sorted_cell[k] = c;
+  return k;
+}
+
+// Cell of every particle (id order) with its arrival rank in the cell, counted into w.count.
 // posmin (optional, f64 positions only): per system and dimension ([3 sys + d]) the minimum
-// position, as ordered_code values, folded in with atomicMin (the caller presets it to all ones).
+// position, as ordered_code values, folded in with atomicMin (all ones before).
 int launch_hash(cudaStream_t st, const GridK* grid_dev, const uint32_t* sys_of_id, int f64, int dim,
-                const void* pos, size_t n, uint32_t* keys, uint32_t* vals, unsigned long long* posmin = nullptr);
+                const void* pos, NbrWork& w, unsigned long long* posmin = nullptr);
 
 // Order-preserving map of doubles to unsigned 64-bit integers (and back), for atomicMin.
 __device__ __forceinline__ unsigned long long ordered_code(double x) {
@@ -126,8 +161,10 @@ __device__ __forceinline__ unsigned long long ordered_code(double x) {
 __device__ __forceinline__ double ordered_value(unsigned long long u) {
   return __longlong_as_double((long long)((u >> 63) ? (u & 0x7fffffffffffffffull) : ~u));
 }
-// Sort (cell, id) pairs already in keys[0]/vals[0] and build cell_start.
-int sort_and_table(cudaStream_t st, NbrWork& w);
+// Cell table and the ids grouped by cell, from launch_hash's counts; the sorted gather that follows
+// orders the ids within each cell (ordered_slot).  nmin position minima move from minacc to minout
+// (both optional), minacc going back to all ones.
+int launch_sort(cudaStream_t st, NbrWork& w, unsigned long long* minacc, unsigned long long* minout, uint32_t nmin);
 // Exclusive scan of m u32 values into out[0..m] (out[m] = total).  tmp: scan_tmp_words(m).
 size_t scan_tmp_words(size_t m);
 int launch_exclusive_scan(cudaStream_t st, const uint32_t* in, uint32_t* out, size_t m, uint32_t* tmp);

@@ -589,7 +589,7 @@ int pg_run_equations(pg_system* s, const char* const* bodies, int n_bodies) {
   const void* spos = s->spos.p;
   const void* sid = s->nw.sorted_id;
   const void* scell = s->nw.sorted_cell;
-  const void* cstart = s->nw.cell_start.p;
+  const void* cstart = s->nw.cell_start;
   std::vector<void*> args = {grid_arg, (void*)&spos, (void*)&sid, (void*)&scell, (void*)&cstart};
   for (size_t f = 0; f < ptrs.size(); ++f) {
     args.push_back(&ptrs[f]);

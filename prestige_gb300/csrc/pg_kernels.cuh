@@ -64,6 +64,7 @@ struct SphArgs {
   const uint32_t* sorted_cell;
   const uint32_t* sorted_id;
   const uint32_t* cell_start;
+  NbrOrder order;            // for the sorted gather, which finishes the sort
   void* s[8];                // sorted packed arrays (layout per arithmetic mode)
   float* pf;                 // sorted FP32 positions of the candidate walks, in chunks (pg_candidates.cuh)
   void* pos;                 // canonical state, id order
@@ -143,6 +144,7 @@ struct NbrArgs {
   const uint32_t* sorted_cell;
   const uint32_t* sorted_id;
   const uint32_t* cell_start;
+  NbrOrder order;            // for the sorted gather, which finishes the sort
   const void* spos;           // sorted positions: double4_32a or float4 (x, y, z, 0)
   float* pf;                  // the same rounded to FP32, in chunks (pg_candidates.cuh)
 };
@@ -172,6 +174,7 @@ struct DemArgs {
   const uint32_t* sorted_cell;
   const uint32_t* sorted_id;
   const uint32_t* cell_start;
+  NbrOrder order;            // for the sorted gather, which finishes the sort
   double4_32a* sA;  // x, y, z, r
   double4_32a* sB;  // vx, vy, vz, m
   double4_32a* sW;  // wx, wy, wz, 0

@@ -157,15 +157,23 @@ __device__ __forceinline__ int cell_coord_f(float x, float lo, float inv, int n)
   return (int)t;
 }
 
-// Cell key and id of every particle.  MIN: also the minimum position per system and dimension
-// (posmin[3 sys + d]).  A single system: block reduction, one atomicMin per block and dimension
-// (blockDim.x == 256).  A batch: warp reduction where the warp's particles belong to one system
-// (ids are contiguous per system, so all warps but those at a system boundary), else one
-// atomicMin per particle.
+// *p = min(*p, v).  The value read first can only be too large (the minimum only falls), so the
+// atomic is left out only where it would change nothing; atomics on one address take about 5 ns each,
+// and all but the first blocks of a launch leave theirs out.
+__device__ __forceinline__ void fold_min(unsigned long long* p, unsigned long long v) {
+  if (v < *(volatile unsigned long long*)p) atomicMin(p, v);
+}
+
+// Cell and arrival rank of every particle (pg_sort.cu).  MIN: also the minimum position per system
+// and dimension (posmin[3 sys + d]): a block reduction and one fold per block and dimension
+// (blockDim.x == 256), or one per particle where a block spans systems of a batch (ids are
+// contiguous per system).
 template <class R, int DIM, bool MIN>
 __global__ void hash_kernel(const GridK* __restrict__ grid, const uint32_t* __restrict__ sys_of_id,
                             const R* __restrict__ pos, uint32_t n, uint32_t* __restrict__ keys,
-                            uint32_t* __restrict__ vals, unsigned long long* __restrict__ posmin) {
+                            uint32_t* __restrict__ rank, uint32_t* __restrict__ count,
+                            uint32_t* __restrict__ big,
+                            unsigned long long* __restrict__ posmin) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   unsigned long long m[3] = {~0ull, ~0ull, ~0ull};
   if (i < n) {
@@ -179,44 +187,44 @@ __global__ void hash_kernel(const GridK* __restrict__ grid, const uint32_t* __re
       else c[d] = cell_coord_f((float)x, g.lof[d], g.invf, nn[d]);
       if (MIN) m[d] = ordered_code((double)x);
     }
-    keys[i] = g.cell_base + ((uint32_t)c[2] * (uint32_t)g.ny + (uint32_t)c[1]) * (uint32_t)g.nx + (uint32_t)c[0];
-    vals[i] = i;
+    const uint32_t key =
+        g.cell_base + ((uint32_t)c[2] * (uint32_t)g.ny + (uint32_t)c[1]) * (uint32_t)g.nx + (uint32_t)c[0];
+    keys[i] = key;
+    const uint32_t r = atomicAdd(count + key, 1u);
+    rank[i] = r;
+    if (r == kBigCell) big[2 + atomicAdd(big, 1u)] = key;  // one thread per cell that large
   }
-  if (MIN && sys_of_id) {
-    const uint32_t s = i < n ? sys_of_id[i] : 0xffffffffu;
-    const uint32_t s0 = __shfl_sync(0xffffffffu, s, 0);
-    if (__all_sync(0xffffffffu, s == s0)) {
+  if (MIN) {
+    // the block's particles belong to one system unless its id range spans a boundary
+    const uint32_t i0 = blockIdx.x * blockDim.x, i1 = min(i0 + blockDim.x, n) - 1;
+    const uint32_t s0 = sys_of_id ? sys_of_id[i0] : 0u;
+    if (!sys_of_id || sys_of_id[i1] == s0) {
+      __shared__ unsigned long long part[DIM][8];
+      const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
       for (int d = 0; d < DIM; ++d) {
         for (int o = 16; o; o >>= 1) m[d] = min(m[d], __shfl_down_sync(0xffffffffu, m[d], o));
-        if ((threadIdx.x & 31) == 0 && s0 != 0xffffffffu) atomicMin(posmin + 3 * (size_t)s0 + d, m[d]);
+        if (lane == 0) part[d][warp] = m[d];
+      }
+      __syncthreads();
+      if (threadIdx.x < DIM) {
+        unsigned long long v = part[threadIdx.x][0];
+        for (int w = 1; w < 8; ++w) v = min(v, part[threadIdx.x][w]);
+        fold_min(posmin + 3 * (size_t)s0 + threadIdx.x, v);
       }
     } else if (i < n) {
 #pragma unroll
-      for (int d = 0; d < DIM; ++d) atomicMin(posmin + 3 * (size_t)s + d, m[d]);
-    }
-  } else if (MIN) {
-    __shared__ unsigned long long part[DIM][8];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int d = 0; d < DIM; ++d) {
-      for (int o = 16; o; o >>= 1) m[d] = min(m[d], __shfl_down_sync(0xffffffffu, m[d], o));
-      if (lane == 0) part[d][warp] = m[d];
-    }
-    __syncthreads();
-    if (threadIdx.x < DIM) {
-      unsigned long long v = part[threadIdx.x][0];
-      for (int w = 1; w < 8; ++w) v = min(v, part[threadIdx.x][w]);
-      atomicMin(posmin + threadIdx.x, v);
+      for (int d = 0; d < DIM; ++d) fold_min(posmin + 3 * (size_t)sys_of_id[i] + d, m[d]);
     }
   }
 }
 
 template <class R, int DIM>
 __global__ void sorted_positions_kernel(NbrArgs a, const R* __restrict__ pos, typename NbrV4<R>::T* spos) {
-  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= a.n) return;
-  const uint32_t id = a.sorted_id[k];
+  const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= a.n) return;
+  uint32_t id;
+  const uint32_t k = ordered_slot(a.order, s, id);
   typename NbrV4<R>::T p;
   p.x = pos[(size_t)id * DIM];
   p.y = pos[(size_t)id * DIM + 1];
@@ -368,20 +376,27 @@ inline unsigned blocks_for(size_t n, int t) { return (unsigned)((n + t - 1) / t)
 
 }  // namespace
 
+template <class R, int DIM>
+static void hash_dim(cudaStream_t st, const GridK* grid, const uint32_t* sys_of_id, const void* pos, NbrWork& w,
+                     unsigned long long* posmin) {
+  const unsigned b = blocks_for(w.n, 256);
+  if (sizeof(R) == 8 && posmin)
+    hash_kernel<R, DIM, true><<<b, 256, 0, st>>>(grid, sys_of_id, (const R*)pos, (uint32_t)w.n, w.key, w.rank,
+                                                 w.count, w.big, posmin);
+  else
+    hash_kernel<R, DIM, false><<<b, 256, 0, st>>>(grid, sys_of_id, (const R*)pos, (uint32_t)w.n, w.key, w.rank,
+                                                  w.count, w.big, nullptr);
+}
+
 int launch_hash(cudaStream_t st, const GridK* grid_dev, const uint32_t* sys_of_id, int f64, int dim, const void* pos,
-                size_t n, uint32_t* keys, uint32_t* vals, unsigned long long* posmin) {
-  if (n == 0) return PG_OK;
-  const unsigned b = blocks_for(n, 256);
-  const uint32_t m = (uint32_t)n;
-  if (f64 && posmin) {
-    if (dim == 2) hash_kernel<double, 2, true><<<b, 256, 0, st>>>(grid_dev, sys_of_id, (const double*)pos, m, keys, vals, posmin);
-    else hash_kernel<double, 3, true><<<b, 256, 0, st>>>(grid_dev, sys_of_id, (const double*)pos, m, keys, vals, posmin);
-  } else if (f64) {
-    if (dim == 2) hash_kernel<double, 2, false><<<b, 256, 0, st>>>(grid_dev, sys_of_id, (const double*)pos, m, keys, vals, nullptr);
-    else hash_kernel<double, 3, false><<<b, 256, 0, st>>>(grid_dev, sys_of_id, (const double*)pos, m, keys, vals, nullptr);
+                NbrWork& w, unsigned long long* posmin) {
+  if (w.n == 0) return PG_OK;
+  if (f64) {
+    if (dim == 2) hash_dim<double, 2>(st, grid_dev, sys_of_id, pos, w, posmin);
+    else hash_dim<double, 3>(st, grid_dev, sys_of_id, pos, w, posmin);
   } else {
-    if (dim == 2) hash_kernel<float, 2, false><<<b, 256, 0, st>>>(grid_dev, sys_of_id, (const float*)pos, m, keys, vals, nullptr);
-    else hash_kernel<float, 3, false><<<b, 256, 0, st>>>(grid_dev, sys_of_id, (const float*)pos, m, keys, vals, nullptr);
+    if (dim == 2) hash_dim<float, 2>(st, grid_dev, sys_of_id, pos, w, nullptr);
+    else hash_dim<float, 3>(st, grid_dev, sys_of_id, pos, w, nullptr);
   }
   PG_CUDA_TRY(cudaGetLastError());
   return PG_OK;

@@ -1,5 +1,5 @@
-// Neighbour-search integer stages: device exclusive scan, stable LSD radix sort of
-// (cell, particle id) pairs, and the cell-start table.
+// Neighbour-search integer stages: device exclusive scan, stable counting sort of the particles by
+// cell with its cell-start table, and the radix sort of the cell list without allocation.
 //
 // The reference executes an equation as `for i in 0..n { for j in 0..n { body } }`
 // (prestige/src/codegen/simple_cpu.rs:7-8).  These stages replace the inner all-pairs loop
@@ -7,12 +7,20 @@
 // cell_start[c] .. cell_start[c+1].  Everything here is integer work and bit-exact against
 // the oracle's stable counting sort.
 //
-// Sort: 8-bit digits, least significant first.  Each pass is three launches:
-//   digit_hist   per tile of 1024 keys (4096 without allocation), a 256-bin histogram
-//                                                                   -> hist[d * tiles + t]
-//   digit_scan   per digit, exclusive scan over tiles (in place)    -> digit_total[d]
-//   digit_scatter stable per-tile ranking with warp match masks, then scatter
-// Input order is id order, and every pass is stable, so equal cells stay in id order.
+// The sort of a handle takes three or four launches and a share of the sorted gather that follows:
+//   hash (pg_neighbors.cu)  cell of each id; an atomic on the cell's count gives the id its arrival
+//                rank there
+//   cell_reduce  totals per chunk of kScanChunk cells (grids of more than one chunk; adding them up by
+//                atomics in the hash took 5 ns per warp of particles: one address at a time)
+//   cell_scan    cell_start = exclusive scan of the counts: a block per chunk, its base the sum of
+//                the totals of the chunks before it; the counts go back to zero for the next search
+//   cell_scatter id -> slot cell_start[cell] + rank, so ids are grouped by cell in arrival order
+//   the gather   ranks each id among the few ids of its cell (ordered_slot): the stable order
+// It is bound by the latency of these few launches below about 1M particles and by the scattered
+// 4-byte writes and atomics above.  It replaced an LSD radix sort by 8-bit digits with a binary search
+// per cell for the table (3 launches per digit, 8 to 11 in all).  Search plus gather, ms, before and
+// after: 6.5k particles 0.049 / 0.025, 200k spheres 0.085 / 0.045, 262k 0.082 / 0.041, 700k f32
+// 0.073 / 0.050, 4M 0.409 / 0.254, 6.1M in 512 systems 0.589 / 0.401.
 #include <cuda_runtime.h>
 
 #include <mutex>
@@ -24,16 +32,7 @@ namespace pg {
 namespace {
 
 constexpr int kSortThreads = 256;
-// Keys per thread of the histogram and scatter kernels.  The handles' sorts use 4 (tiles of 1024
-// keys): against 16 (tiles of 4096) the 200,000-sphere DEM step went from 0.144 to 0.122 ms
-// (49 tiles had left most of the 152 SMs idle) and the 4M-particle neighbour search from 0.304
-// to 0.285 ms.  The no-allocation path keeps 16: its fixed scratch holds the histograms of
-// 4096-key tiles.  The sort result does not depend on the tile size.  Digits of 10 bits, which
-// sort the 19-bit DEM keys in two passes instead of three, were measured and dropped: the
-// 1024-bin tables made each pass dearer by as much (DEM step 0.099 against 0.097 ms).
-constexpr int kSortItems = 16;
-constexpr int kSortItemsSmall = 4;
-constexpr size_t kSmallSortN = ~size_t(0);
+constexpr int kSortItems = 16;  // keys per thread of the radix kernels: their scratch has a fixed size
 constexpr int kSortTile = kSortThreads * kSortItems;  // 4096 keys per tile
 constexpr int kSortWarps = kSortThreads / 32;
 constexpr int kRadix = 256;
@@ -225,20 +224,134 @@ __global__ void __launch_bounds__(kSortThreads) digit_scatter_kernel(
   }
 }
 
-// cell_start[c] = first sorted slot whose cell is >= c, for c = 0 .. ncells (so cell_start[ncells]
-// = n), by a binary search over the sorted cells: one kernel, no count buffer and no scan.  The
-// threads of a warp search for consecutive cells, so they load the same midpoints on most steps.
-__global__ void cell_start_kernel(const uint32_t* __restrict__ cell, uint32_t n, uint32_t ncells,
-                                  uint32_t* __restrict__ start) {
-  const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c > ncells) return;
-  uint32_t lo = 0, hi = n;
-  while (lo < hi) {
-    const uint32_t mid = lo + (hi - lo) / 2;
-    if (__ldg(cell + mid) < c) lo = mid + 1;
-    else hi = mid;
+// ---------------------------------------------------------------------------------------
+// Counting sort.
+// ---------------------------------------------------------------------------------------
+constexpr int kCellScanThreads = 1024;
+constexpr int kCellScanItems = kScanChunk / kCellScanThreads;
+static_assert(kCellScanItems == 8, "two 16-byte loads per thread");
+
+__global__ void __launch_bounds__(kCellScanThreads) cell_reduce_kernel(const uint32_t* __restrict__ count,
+                                                                       uint32_t* __restrict__ chunk_total) {
+  const uint4* cp = (const uint4*)(count + (size_t)blockIdx.x * kScanChunk) + 2 * threadIdx.x;
+  const uint4 a = cp[0], b = cp[1];
+  uint32_t total;
+  block_excl_scan(a.x + a.y + a.z + a.w + b.x + b.y + b.z + b.w, &total);
+  if (threadIdx.x == 0) chunk_total[blockIdx.x] = total;
+}
+
+__global__ void __launch_bounds__(kCellScanThreads) cell_scan_kernel(uint32_t* __restrict__ count,
+                                                                     const uint32_t* __restrict__ chunk_total,
+                                                                     uint32_t* __restrict__ start,
+                                                                     unsigned long long* minacc,
+                                                                     unsigned long long* minout, uint32_t nmin) {
+  __shared__ uint32_t base;
+  const uint32_t tid = threadIdx.x;
+  // cells of the chunks before this one
+  uint32_t before = 0;
+  for (uint32_t c = tid; c < blockIdx.x; c += kCellScanThreads) before += chunk_total[c];
+  uint32_t total;
+  block_excl_scan(before, &total);
+  if (tid == 0) base = total;
+  uint4* cp = (uint4*)(count + (size_t)blockIdx.x * kScanChunk) + 2 * tid;
+  const uint4 a = cp[0], b = cp[1];
+  if (a.x | a.y | a.z | a.w) cp[0] = make_uint4(0, 0, 0, 0);
+  if (b.x | b.y | b.z | b.w) cp[1] = make_uint4(0, 0, 0, 0);
+  uint32_t ex = block_excl_scan(a.x + a.y + a.z + a.w + b.x + b.y + b.z + b.w, &total) + base;
+  uint4 o, p;
+  o.x = ex;
+  o.y = o.x + a.x;
+  o.z = o.y + a.y;
+  o.w = o.z + a.z;
+  p.x = o.w + a.w;
+  p.y = p.x + b.x;
+  p.z = p.y + b.y;
+  p.w = p.z + b.z;
+  uint4* sp = (uint4*)(start + (size_t)blockIdx.x * kScanChunk) + 2 * tid;
+  sp[0] = o;
+  sp[1] = p;
+  if (blockIdx.x == 0)
+    for (uint32_t i = tid; i < nmin; i += kCellScanThreads) {
+      minout[i] = minacc[i];
+      minacc[i] = ~0ull;
+    }
+}
+
+// Sort the m distinct ids of one cell ascending, by one block of kSortThreads threads: LSD radix by
+// 8-bit digits, tile after tile, between ids and tmp (m values each).
+__device__ __noinline__ void sort_segment(uint32_t* ids, uint32_t* tmp, uint32_t m, int bits) {
+  __shared__ uint32_t wcnt[kSortWarps][kRadix];
+  __shared__ uint32_t next[kRadix];  // next free position of each digit
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  uint32_t *src = ids, *dst = tmp;
+  for (int shift = 0; shift < bits; shift += 8) {
+    next[tid] = 0;
+    __syncthreads();
+    for (uint32_t i = tid; i < m; i += kSortThreads) atomicAdd(&next[(src[i] >> shift) & 0xffu], 1u);
+    __syncthreads();
+    uint32_t total;
+    const uint32_t first = block_excl_scan(next[tid], &total);
+    next[tid] = first;
+    __syncthreads();
+    for (uint32_t t0 = 0; t0 < m; t0 += kSortThreads) {
+#pragma unroll
+      for (int w = 0; w < kSortWarps; ++w) wcnt[w][tid] = 0;
+      __syncthreads();
+      const uint32_t i = t0 + tid;
+      const bool valid = i < m;
+      const uint32_t v = valid ? src[i] : 0u;
+      const uint32_t d = valid ? ((v >> shift) & 0xffu) : 0x100u;
+      const uint32_t peers = __match_any_sync(0xffffffffu, d);
+      const uint32_t below = __popc(peers & ((1u << lane) - 1u));
+      if (valid && below == 0) wcnt[warp][d] = __popc(peers);
+      __syncthreads();
+      uint32_t run = next[tid];  // per digit: positions of the warps' runs
+#pragma unroll
+      for (int w = 0; w < kSortWarps; ++w) {
+        const uint32_t c = wcnt[w][tid];
+        wcnt[w][tid] = run;
+        run += c;
+      }
+      next[tid] = run;
+      __syncthreads();
+      if (valid) dst[wcnt[warp][d] + below] = v;
+      __syncthreads();
+    }
+    uint32_t* t = src;
+    src = dst;
+    dst = t;
   }
-  start[c] = lo;
+  if (src != ids) {
+    for (uint32_t i = tid; i < m; i += kSortThreads) ids[i] = src[i];
+    __syncthreads();
+  }
+}
+
+// ids to their cell's slots in arrival order.  Ranking an id among the ids of its cell costs the gather
+// as many reads as the cell holds, so the cells of more than kBigCell particles (a degenerate
+// distribution: the hash listed them) are sorted here, by the block that finishes last; it waits
+// for nothing, and a search without such cells has no last block.
+__global__ void __launch_bounds__(kSortThreads) cell_scatter_kernel(const uint32_t* __restrict__ key,
+                                                                    uint32_t* rank,
+                                                                    const uint32_t* __restrict__ start, uint32_t n,
+                                                                    uint32_t* unsorted, uint32_t* big, int id_bits) {
+  const uint32_t i = blockIdx.x * kSortThreads + threadIdx.x;
+  if (i < n) unsorted[start[key[i]] + rank[i]] = i;
+  const uint32_t nbig = ((volatile uint32_t*)big)[0];
+  if (nbig == 0) return;
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(&big[1], 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  for (uint32_t b = 0; b < nbig; ++b) {
+    const uint32_t c = big[2 + b];
+    const uint32_t s0 = start[c];
+    sort_segment(unsorted + s0, rank + s0, start[c + 1] - s0, id_bits);  // the ranks are done with
+  }
+  if (threadIdx.x == 0) big[0] = big[1] = 0;
 }
 
 int bits_needed(uint64_t v) {
@@ -270,56 +383,51 @@ int launch_exclusive_scan(cudaStream_t st, const uint32_t* in, uint32_t* out, si
 int NbrWork::init(size_t n_, uint64_t ncells_) {
   n = n_;
   ncells = ncells_;
-  const int bits = bits_needed(ncells ? ncells - 1 : 0);
-  passes = (bits + 7) / 8;
-  items = n <= kSmallSortN ? kSortItemsSmall : kSortItems;
-  const size_t tile = (size_t)kSortThreads * items;
-  tiles = (int)((n + tile - 1) / tile);
-  if (tiles < 1) tiles = 1;
-  const size_t nn = n ? n : 1;
-  PG_TRY(keys[0].ensure(nn * 4));
-  PG_TRY(keys[1].ensure(nn * 4));
-  PG_TRY(vals[0].ensure(nn * 4));
-  PG_TRY(vals[1].ensure(nn * 4));
-  PG_TRY(hist.ensure((size_t)kRadix * tiles * 4));
-  PG_TRY(digit_total.ensure(kRadix * 4));
-  PG_TRY(cell_start.ensure((ncells + 1) * 4));
+  passes = (bits_needed(ncells ? ncells - 1 : 0) + 7) / 8;
+  chunks = (uint32_t)(ncells / kScanChunk + 1);
+  const size_t nn = n ? n : 1, cells = (size_t)chunks * kScanChunk;
+  rest_words = cells + 2 + nn / kBigCell;
+  struct {
+    uint32_t** p;
+    size_t words;
+  } parts[] = {{&key, nn},           {&rank, nn},          {&unsorted, nn},       {&sorted_cell, nn},
+               {&sorted_id, nn},     {&cell_start, cells}, {&chunk_total, chunks}, {&rest, rest_words}};
+  size_t words = 0;
+  for (auto& part : parts) words += (part.words + 63) / 64 * 64;  // each from a 256-byte boundary
+  PG_TRY(mem.ensure(words * 4));
+  uint32_t* at = mem.as<uint32_t>();
+  for (auto& part : parts) {
+    *part.p = at;
+    at += (part.words + 63) / 64 * 64;
+  }
+  count = rest;
+  big = rest + cells;
+  clean = false;
   return PG_OK;
 }
 
-size_t NbrWork::bytes() const {
-  return keys[0].bytes + keys[1].bytes + vals[0].bytes + vals[1].bytes + hist.bytes + digit_total.bytes +
-         cell_start.bytes;
+size_t NbrWork::bytes() const { return mem.bytes; }
+
+NbrOrder nbr_order(const NbrWork& w) {
+  NbrOrder o;
+  o.unsorted = w.unsorted;
+  o.key = w.key;
+  o.cell_start = w.cell_start;
+  o.sorted_cell = w.sorted_cell;
+  o.sorted_id = w.sorted_id;
+  return o;
 }
 
-int sort_and_table(cudaStream_t st, NbrWork& w) {
-  const size_t n = w.n;
-  int cur = 0;
-  for (int p = 0; p < w.passes; ++p) {
-    const int shift = 8 * p;
-    if (w.items == kSortItemsSmall)
-      digit_hist_kernel<kSortItemsSmall><<<w.tiles, kSortThreads, 0, st>>>(w.keys[cur].as<uint32_t>(), n, shift,
-                                                                          w.tiles, w.hist.as<uint32_t>());
-    else
-      digit_hist_kernel<kSortItems><<<w.tiles, kSortThreads, 0, st>>>(w.keys[cur].as<uint32_t>(), n, shift, w.tiles,
-                                                                     w.hist.as<uint32_t>());
-    digit_scan_kernel<<<kRadix, kSortThreads, 0, st>>>(w.hist.as<uint32_t>(), w.tiles, w.digit_total.as<uint32_t>());
-    if (w.items == kSortItemsSmall)
-      digit_scatter_kernel<kSortItemsSmall><<<w.tiles, kSortThreads, 0, st>>>(
-          w.keys[cur].as<uint32_t>(), w.vals[cur].as<uint32_t>(), w.keys[cur ^ 1].as<uint32_t>(),
-          w.vals[cur ^ 1].as<uint32_t>(), n, shift, w.tiles, w.hist.as<uint32_t>(), w.digit_total.as<uint32_t>());
-    else
-      digit_scatter_kernel<kSortItems><<<w.tiles, kSortThreads, 0, st>>>(
-          w.keys[cur].as<uint32_t>(), w.vals[cur].as<uint32_t>(), w.keys[cur ^ 1].as<uint32_t>(),
-          w.vals[cur ^ 1].as<uint32_t>(), n, shift, w.tiles, w.hist.as<uint32_t>(), w.digit_total.as<uint32_t>());
-    cur ^= 1;
-  }
-  w.sorted_cell = w.keys[cur].as<uint32_t>();
-  w.sorted_id = w.vals[cur].as<uint32_t>();
-  // cell table: start[c] = first slot of cell c (start[ncells] = n)
-  cell_start_kernel<<<(unsigned)((w.ncells + 1 + 255) / 256), 256, 0, st>>>(w.sorted_cell, (uint32_t)n,
-                                                                          (uint32_t)w.ncells,
-                                                                          w.cell_start.as<uint32_t>());
+int launch_sort(cudaStream_t st, NbrWork& w, unsigned long long* minacc, unsigned long long* minout, uint32_t nmin) {
+  if (w.chunks > 1)
+    cell_reduce_kernel<<<w.chunks, kCellScanThreads, 0, st>>>(w.count, w.chunk_total);
+  cell_scan_kernel<<<w.chunks, kCellScanThreads, 0, st>>>(w.count, w.chunk_total,
+                                                          w.cell_start, minacc, minout,
+                                                          minacc ? nmin : 0u);
+  if (w.n)
+    cell_scatter_kernel<<<(unsigned)((w.n + kSortThreads - 1) / kSortThreads), kSortThreads, 0, st>>>(
+        w.key, w.rank, w.cell_start, (uint32_t)w.n,
+        w.unsorted, w.big, bits_needed(w.n - 1));
   PG_CUDA_TRY(cudaGetLastError());
   return PG_OK;
 }
@@ -327,10 +435,9 @@ int sort_and_table(cudaStream_t st, NbrWork& w) {
 // =========================================================================================
 // Cell list without device allocation (pg_cell_list_noalloc).
 //
-// The radix sort above needs scratch beyond its inputs and outputs: a second key/value buffer
-// for the ping-pong passes, the per-tile digit histograms and the digit totals.  Handles get
-// that scratch from cudaMalloc when they are created.  This variant takes it from one
-// file-scope device array instead, so a call allocates nothing.  Its size fixes the largest
+// The radix sort (digit_hist, digit_scan, digit_scatter above) needs scratch beyond its inputs and
+// outputs: a second key/value buffer for the ping-pong passes, the per-tile digit histograms and
+// the digit totals.  It comes from one file-scope device array, so a call allocates nothing.  Its size fixes the largest
 // system it accepts (kNoAllocMaxParticles).
 //
 // The array is shared by every call on a device and keeps the previous call's contents.

@@ -48,16 +48,18 @@ template <> __device__ __forceinline__ double2 make2<double>(double a, double b)
 template <> __device__ __forceinline__ float2 make2<float>(float a, float b) { return make_float2(a, b); }
 
 // ---------------------------------------------------------------------------------------
-// Sorted gather: slot k <- particle sorted_id[k]; precomputes P = p / rho^2.
+// Sorted gather: the final order of the neighbour search (ordered_slot), then slot k <- particle
+// sorted_id[k]; precomputes P = p / rho^2.
 //   IEEE modes:   s0 {x, y, z, m}   s1 {vx, vy, vz, 0}   s2 {rho, P}   (pf: FP32 x, y, z)
 // ---------------------------------------------------------------------------------------
 template <class Ops, int DIM>
 __global__ void sph_gather_real(SphArgs a) {
   typedef typename Ops::R R;
   typedef typename V4<R>::T R4;
-  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= a.n) return;
-  const uint32_t id = a.sorted_id[k];
+  const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= a.n) return;
+  uint32_t id;
+  const uint32_t k = ordered_slot(a.order, s, id);
   const SphK& K = a.sys[sys_of_slot(a, id)];
   const R* pos = (const R*)a.pos;
   const R* vel = (const R*)a.vel;
@@ -141,9 +143,10 @@ struct __align__(64) DfRecord {
 // the other systems of a batch; the f64 array for the exact test keeps the unshifted positions.
 template <int DIM>
 __global__ void sph_gather_df(SphArgs a) {
-  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= a.n) return;
-  const uint32_t id = a.sorted_id[k];
+  const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= a.n) return;
+  uint32_t id;
+  const uint32_t k = ordered_slot(a.order, s, id);
   const uint32_t sys = sys_of_slot(a, id);
   const SphK& K = a.sys[sys];
   const double* pos = (const double*)a.pos;

@@ -63,7 +63,7 @@ struct pg_system {
   cudaEvent_t ov_ev[2] = {nullptr, nullptr};
   pg::DevBuf nlist, nlen, nresume;
   pg::DevBuf fcache;             // f64 modes: pair values per list entry (continuity -> momentum)
-  pg::DevBuf posmin;             // 3 x u64, double-word mode (pos_min_kernel)
+  pg::DevBuf posmin;             // per system 3 x u64 minima, then as many accumulators (double-word mode)
 
   // DEM contact history, id order, double buffered
   pg::DevBuf hpid[2], hxi[2];
