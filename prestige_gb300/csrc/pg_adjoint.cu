@@ -138,9 +138,9 @@ __global__ void adjoint_prep_kernel(SphArgs a) {
   const double rr = rho * K.d.inv_rho0;
   double pw = rr;
   for (int e = 1; e < K.gamma; ++e) pw *= rr;
-  const double inv_r2 = 1.0 / (rho * rho);
+  const double inv_r2 = soft_div(1.0, rho * rho);
   const double P = tait_pterm<OpsD>(K.d, K.gamma, rho);
-  const double Pd = K.d.B * ((double)(K.gamma - 2) * pw + 2.0) * inv_r2 / rho;
+  const double Pd = soft_div(K.d.B * ((double)(K.gamma - 2) * pw + 2.0) * inv_r2, rho);
   const double PB = (pw - 1.0) * inv_r2;
   ((double4_32a*)a.s[0])[k] = make_double4_32a(x[0], x[1], x[2], m);
   ((double4_32a*)a.s[1])[k] = make_double4_32a(v[0], v[1], v[2], rho);
@@ -204,9 +204,9 @@ __global__ void adjoint_prep_f_kernel(SphArgs a) {
   const double rr = rho * K.d.inv_rho0;
   double pw = rr;
   for (int e = 1; e < K.gamma; ++e) pw *= rr;
-  const double inv_r2 = 1.0 / (rho * rho);
+  const double inv_r2 = soft_div(1.0, rho * rho);
   const double P = tait_pterm<OpsD>(K.d, K.gamma, rho);
-  const double Pd = K.d.B * ((double)(K.gamma - 2) * pw + 2.0) * inv_r2 / rho;
+  const double Pd = soft_div(K.d.B * ((double)(K.gamma - 2) * pw + 2.0) * inv_r2, rho);
   const double PB = (pw - 1.0) * inv_r2;
   ((float4*)a.s[0])[k] = make_float4(hx[0], hx[1], hx[2], (float)m);
   pf_store<DIM>(a.pf, k, hx[0], hx[1], hx[2]);

@@ -119,7 +119,7 @@ __device__ __forceinline__ Geo<DIM> geometry(const SphC<double>& c, const double
   g.d[2] = DIM == 3 ? xk.z - xt.z : 0.0;
   g.r2 = __dadd_rn(__dmul_rn(g.d[0], g.d[0]), __dmul_rn(g.d[1], g.d[1]));
   if (DIM == 3) g.r2 = __dadd_rn(g.r2, __dmul_rn(g.d[2], g.d[2]));
-  const double inv_r = rsqrt(g.r2);  // one FP64 sequence in place of a square root and a division
+  const double inv_r = soft_div(1.0, soft_sqrt(g.r2));  // off the FP64 pipe (pg_softf64.cuh)
   const double r = g.r2 * inv_r;
   const double q = r * c.inv_h;
   if (q < 1.0) {
@@ -167,7 +167,7 @@ __device__ __forceinline__ MomTerms<DIM> mom_terms(const SphK& K, const Packs& P
   const double rb = vk.w + vt.w;
   const double e = g.r2 + c.eps_h2;
   // one reciprocal serves the four quotients of the terms
-  const double inv_erb = __drcp_rn(e * rb);
+  const double inv_erb = soft_div(1.0, e * rb);
   const double inv_e = rb * inv_erb, inv_rb = e * inv_erb;
   double c1 = 0.0, c1a = 0.0;
   if (g.w < 0.0) {

@@ -1,7 +1,8 @@
 // Arithmetic policies for the pair kernels.
 //
-//   OpsD  IEEE double, one rounding per operation, never contracted (__dadd_rn, ...).  With
-//         the oracle's operation order this reproduces the CPU oracle bit for bit.
+//   OpsD  IEEE double, one rounding per operation, never contracted (__dadd_rn, ...; division and
+//         square root on the integer pipe, pg_softf64.cuh).  With the oracle's operation order this
+//         reproduces the CPU oracle bit for bit.
 //   OpsF  the same in IEEE single precision.
 //   OpsFF single precision with contraction allowed (fast f32 mode).
 //   df    double-word ("double-float") arithmetic on the FP32 pipe: a value is hi + lo with
@@ -41,6 +42,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "pg_softf64.cuh"
+
 namespace pg {
 
 struct OpsD {
@@ -48,8 +51,8 @@ struct OpsD {
   static __device__ __forceinline__ R add(R a, R b) { return __dadd_rn(a, b); }
   static __device__ __forceinline__ R sub(R a, R b) { return __dsub_rn(a, b); }
   static __device__ __forceinline__ R mul(R a, R b) { return __dmul_rn(a, b); }
-  static __device__ __forceinline__ R div(R a, R b) { return __ddiv_rn(a, b); }
-  static __device__ __forceinline__ R sqrt(R a) { return __dsqrt_rn(a); }
+  static __device__ __forceinline__ R div(R a, R b) { return soft_div(a, b); }
+  static __device__ __forceinline__ R sqrt(R a) { return soft_sqrt(a); }
 };
 
 struct OpsF {

@@ -20,6 +20,7 @@
 
 #include "pg_internal.cuh"
 #include "pg_kernels.cuh"
+#include "pg_softf64.cuh"
 
 namespace pg {
 
@@ -31,7 +32,7 @@ constexpr uint32_t kWallId = 0xFFFFFFF0u;
 __device__ __forceinline__ double dadd(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double dsub(double a, double b) { return __dsub_rn(a, b); }
 __device__ __forceinline__ double dmul(double a, double b) { return __dmul_rn(a, b); }
-__device__ __forceinline__ double ddiv(double a, double b) { return __ddiv_rn(a, b); }
+__device__ __forceinline__ double ddiv(double a, double b) { return soft_div(a, b); }
 
 // +-0 and 0 < x < inf, tested on the bit pattern.
 __device__ __forceinline__ bool is_zero(double x) { return ((unsigned long long)__double_as_longlong(x) << 1) == 0; }
@@ -60,7 +61,7 @@ __device__ __forceinline__ void contact_terms(const DemK& K, const Contact& ct, 
   double vt[3];
 #pragma unroll
   for (int c = 0; c < 3; ++c) vt[c] = dsub(ct.vr[c], dmul(vn, n[c]));
-  const double gn = dmul(K.gcoef, __dsqrt_rn(dmul(ct.meff, K.kn)));
+  const double gn = dmul(K.gcoef, soft_sqrt(dmul(ct.meff, K.kn)));
   const double fn = dsub(dmul(K.kn, ct.delta), dmul(gn, vn));
   const double xdn = dadd(dadd(dmul(xo[0], n[0]), dmul(xo[1], n[1])), dmul(xo[2], n[2]));
   double xi[3], ft[3];
@@ -71,7 +72,7 @@ __device__ __forceinline__ void contact_terms(const DemK& K, const Contact& ct, 
   const double ft2 = dadd(dadd(dmul(ft[0], ft[0]), dmul(ft[1], ft[1])), dmul(ft[2], ft[2]));
   const double lim = dmul(K.mu, fabs(fn));
   if (ft2 > dmul(lim, lim)) {
-    const double scale = ddiv(lim, __dsqrt_rn(ft2));
+    const double scale = ddiv(lim, soft_sqrt(ft2));
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       ft[c] = dmul(ft[c], scale);
@@ -114,7 +115,7 @@ __device__ __forceinline__ void contact_geometry(const DemArgs& a, const DemK& K
     const double d[3] = {dsub(me.x[0], Aj.x), dsub(me.x[1], Aj.y), dsub(me.x[2], Aj.z)};
     const double d2 = dadd(dadd(dmul(d[0], d[0]), dmul(d[1], d[1])), dmul(d[2], d[2]));
     const double rs = dadd(me.r, Aj.w);
-    const double dist = __dsqrt_rn(d2);
+    const double dist = soft_sqrt(d2);
 #pragma unroll
     for (int cc = 0; cc < 3; ++cc) ct.nrm[cc] = ddiv(d[cc], dist);
     ct.delta = dsub(rs, dist);
