@@ -36,7 +36,6 @@ namespace {
 
 using namespace sphpass;
 
-constexpr uint32_t kNoMirror = 0xFFFFFFFFu;
 constexpr int kPlanes = 15;  // doubles per list entry (plus one u32)
 // the partner's momentum share (Vx, Vv, F x.E, Pi / rho_ij); for the continuity pass, the pair's
 // vectors U1 = G w x + F v and U2 = F x and the partner's mass (own entries above the slot)
@@ -65,31 +64,6 @@ __device__ __forceinline__ size_t entry(uint32_t k, uint32_t q, uint32_t cap) {
 __device__ __forceinline__ bool holds(const SphArgs& a, uint32_t t, uint32_t k) {
   if (a.nlen[t] <= a.cap) return true;
   return a.nlist[entry(t, a.cap - 1, a.cap)] >= k;
-}
-
-// Position of k in slot t's stored (ascending) list, or kNoMirror.
-__device__ __forceinline__ uint32_t find_in_list(const SphArgs& a, uint32_t t, uint32_t k) {
-  const uint32_t L = min(a.nlen[t], a.cap);
-  const uint32_t* __restrict__ lt = a.nlist + list_base(t, a.cap);
-  uint32_t lo = 0, hi = L;
-  while (lo < hi) {
-    const uint32_t mid = (lo + hi) >> 1;
-    if (lt[(size_t)mid * kListTile] < k) lo = mid + 1;
-    else hi = mid;
-  }
-  return lo < L && lt[(size_t)lo * kListTile] == k ? lo : kNoMirror;
-}
-
-// Index of the first entry above slot k in its ascending list of L entries (binary search):
-// the entries before it are the ones below k.
-__device__ __forceinline__ uint32_t first_above(const uint32_t* __restrict__ my, uint32_t L, uint32_t k) {
-  uint32_t lo = 0, hi = L;
-  while (lo < hi) {
-    const uint32_t mid = (lo + hi) >> 1;
-    if (my[(size_t)mid * kListTile] < k) lo = mid + 1;
-    else hi = mid;
-  }
-  return lo;
 }
 
 // The slot-ordered packs of the adjoint step (adjoint_prep_kernel):
@@ -285,9 +259,14 @@ __global__ void __launch_bounds__(kSphMaxThreads) adj_mirror_kernel(SphArgs a) {
   if (!slot_of(a, s)) return;
   const Planes E = planes_of(a);
   const uint32_t* __restrict__ my = a.nlist + list_base(s.k, a.cap);
-  for (uint32_t q = 0; q < s.L; ++q) {
-    const uint32_t t = my[(size_t)q * kListTile];
-    if (t > s.k) E.mirror(entry(s.k, q, a.cap)) = find_in_list(a, t, s.k);
+  for (uint32_t q = lower_bound(my, s.L, s.k); q < s.L; q += kSearch) {
+    uint32_t t[kSearch], m[kSearch];
+#pragma unroll
+    for (int i = 0; i < kSearch; ++i) t[i] = my[(size_t)min(q + i, s.L - 1) * kListTile];
+    find_in_lists(a, t, s.k, m);
+#pragma unroll
+    for (int i = 0; i < kSearch; ++i)
+      if (q + i < s.L) E.mirror(entry(s.k, q + i, a.cap)) = m[i];
   }
 }
 
@@ -304,7 +283,7 @@ __global__ void __launch_bounds__(kSphMaxThreads) adj_a1_kernel(SphArgs a) {
   Sums sum = {{0, 0, 0}, {0, 0, 0}, 0, 0, 0};
   // each lane from its own first entry above the slot, so the lanes of a warp evaluate their
   // pairs in the same iterations
-  for (uint32_t q = first_above(my, s.L, s.k); q < s.L; ++q) {
+  for (uint32_t q = lower_bound(my, s.L, s.k); q < s.L; ++q) {
     const uint32_t t = my[(size_t)q * kListTile];
     const MomTerms<DIM> m = mom_terms<DIM>(K, P, s.k, t, xk, vk);
     const size_t e = entry(s.k, q, a.cap);
@@ -341,7 +320,7 @@ __global__ void __launch_bounds__(kSphMaxThreads) adj_a2_kernel(SphArgs a) {
   const double Pdk = P.Q[s.k].y;
   const uint32_t* __restrict__ my = a.nlist + list_base(s.k, a.cap);
   Sums sum = load_sums(a, P, s.k, kSlotSums);
-  const uint32_t below = first_above(my, s.L, s.k);  // the entries below the slot come first
+  const uint32_t below = lower_bound(my, s.L, s.k);  // the entries below the slot come first
   for (uint32_t q = 0; q < below; ++q) {
     const uint32_t t = my[(size_t)q * kListTile];
     if (holds(a, t, s.k)) {  // t's share of the pair was written here by t: negate it
@@ -443,7 +422,7 @@ __global__ void __launch_bounds__(kSphMaxThreads) adj_c2_kernel(SphArgs a) {
   const double4_32a xk = P.X[s.k], vk = P.V[s.k];
   const uint32_t* __restrict__ my = a.nlist + list_base(s.k, a.cap);
   Sums sum = load_sums(a, P, s.k, 6);
-  const uint32_t below = first_above(my, s.L, s.k);
+  const uint32_t below = lower_bound(my, s.L, s.k);
   for (uint32_t q = 0; q < below; ++q) {
     const uint32_t t = my[(size_t)q * kListTile];
     if (holds(a, t, s.k)) {

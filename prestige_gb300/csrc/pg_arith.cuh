@@ -55,6 +55,11 @@ struct OpsD {
   static __device__ __forceinline__ R sqrt(R a) { return soft_sqrt(a); }
 };
 
+// The same results with multiplications on the integer pipe as well (kernels bound by the FP64 pipe).
+struct OpsDI : OpsD {
+  static __device__ __forceinline__ R mul(R a, R b) { return soft_mul(a, b); }
+};
+
 struct OpsF {
   typedef float R;
   static __device__ __forceinline__ R add(R a, R b) { return __fadd_rn(a, b); }

@@ -1,4 +1,4 @@
-// Correctly rounded f64 division and square root on the integer and FP32 pipes.
+// Correctly rounded f64 division, square root and multiplication on the integer and FP32 pipes.
 //
 // GB300 issues FP64 at 1/64 of the FP32 rate, so a division or square root in FP64 instructions
 // (about 9 and 10 FP64 operations by measured throughput) occupies its pipe as long as about 600
@@ -27,6 +27,8 @@ namespace pg {
 
 static __device__ __noinline__ double div_f64_call(double a, double b) { return __ddiv_rn(a, b); }
 static __device__ __noinline__ double sqrt_f64_call(double x) { return __dsqrt_rn(x); }
+// (inline, the compiler multiplies always and selects)
+static __device__ __noinline__ double mul_f64_call(double a, double b) { return __dmul_rn(a, b); }
 
 // d, with m = fl(d + 1.5 2^23), is far enough from a rounding boundary: |d - rint(d)| + 2^-21 |d| < 1/2 -
 // 2^-19, and |d| < 512.
@@ -94,6 +96,33 @@ __device__ __forceinline__ double soft_sqrt(double x) {
   const unsigned long long res = s + (unsigned long long)(long long)(__float_as_int(m) - 0x4b400000);
   const unsigned hi = (unsigned)(res >> 32) + (((e + 1023u) >> 1) - 1u << 20);
   return __hiloint2double((int)hi, (int)(unsigned)res);
+}
+
+// a b, rounded to nearest even: the 106-bit product of the significands by four 32 x 32 bit multiplications,
+// its leading 53 bits rounded on the bits below.  About 32 integer instructions against one FP64 one,
+// that is about half of the FP64 pipe's time but on another pipe: for kernels whose FP64 pipe is full
+// and whose other pipes are not.  Operands outside 2^-255 .. 2^257 (zeros among them) and possible ties
+// take the FP64 instruction, out of line.
+__device__ __forceinline__ double soft_mul(double a, double b) {
+  const unsigned ah = (unsigned)__double2hiint(a), al = (unsigned)__double2loint(a);
+  const unsigned bh = (unsigned)__double2hiint(b), bl = (unsigned)__double2loint(b);
+  const unsigned am = (ah & 0xfffffu) | 0x100000u, bm = (bh & 0xfffffu) | 0x100000u;
+  // A in [2^52, 2^53) times B 2^11 in [2^63, 2^64): 2^115 .. 2^117, the high 64 bits h in [2^51, 2^53)
+  const unsigned cl = bl << 11, ch = __funnelshift_l(bl, bm, 11);
+  const unsigned long long m0 = (unsigned long long)al * cl;
+  const unsigned long long m1 = (unsigned long long)am * cl + (unsigned)(m0 >> 32);
+  const unsigned long long m2 = (unsigned long long)al * ch + (unsigned)m1;
+  const unsigned long long h = (unsigned long long)am * ch + (unsigned)(m1 >> 32) + (unsigned)(m2 >> 32);
+  const unsigned hl = (unsigned)h, hh = (unsigned)(h >> 32), below = (unsigned)m2;
+  const unsigned s = ~(hh >> 20) & 1u;  // one bit to the left where h < 2^52
+  const unsigned rh = __funnelshift_l(hl, hh, s), rl = __funnelshift_l(below, hl, s), rest = below << s;
+  const unsigned long long r = (((unsigned long long)rh << 32) | rl) + (rest >> 31);
+  // both exponents in 768 .. 1279 where neither difference has one of its two top bits set
+  const bool in = ((((ah << 1) - 0x60000000u) | ((bh << 1) - 0x60000000u)) & 0xc0000000u) == 0;
+  const unsigned e = (ah & 0x7ff00000u) + (bh & 0x7ff00000u) - ((1023u << 20) + (s << 20));  // r has the leading bit
+  const unsigned hi = ((unsigned)(r >> 32) + e) | ((ah ^ bh) & 0x80000000u);
+  if (!in || rest == 0x80000000u) return mul_f64_call(a, b);
+  return __hiloint2double((int)hi, (int)(unsigned)r);
 }
 
 }  // namespace pg

@@ -275,6 +275,60 @@ __global__ void __launch_bounds__(kSphMaxThreads) sph_list_kernel(SphArgs a) {
   }
 }
 
+// ---------------------------------------------------------------------------------------
+// Mirror entries of the pair-once kernels: the position of a slot in another slot's stored list
+// (lists ascend).
+// ---------------------------------------------------------------------------------------
+constexpr uint32_t kNoMirror = 0xFFFFFFFFu;
+constexpr int kSearch = 4;  // searches in flight per thread
+
+// First of the L entries of an ascending tiled list that is not below k.
+__device__ __forceinline__ uint32_t lower_bound(const uint32_t* __restrict__ list, uint32_t L, uint32_t k) {
+  uint32_t lo = 0, hi = L;
+  while (lo < hi) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (list[(size_t)mid * kListTile] < k) lo = mid + 1;
+    else hi = mid;
+  }
+  return lo;
+}
+
+// pos[i] = position of slot k in the stored list of slot t[i], or kNoMirror.  The searches run in step, so
+// each round has kSearch loads in flight in place of one.
+__device__ __forceinline__ void find_in_lists(const SphArgs& a, const uint32_t (&t)[kSearch], uint32_t k,
+                                              uint32_t (&pos)[kSearch]) {
+  uint32_t hi[kSearch], L[kSearch];
+  const uint32_t* lt[kSearch];
+  bool more = false;
+#pragma unroll
+  for (int i = 0; i < kSearch; ++i) {
+    L[i] = hi[i] = min(a.nlen[t[i]], a.cap);
+    lt[i] = a.nlist + list_base(t[i], a.cap);
+    pos[i] = 0;
+    more = more || hi[i] > 0;
+  }
+  while (more) {
+    more = false;
+    uint32_t v[kSearch], mid[kSearch];
+#pragma unroll
+    for (int i = 0; i < kSearch; ++i) {
+      mid[i] = (pos[i] + hi[i]) >> 1;
+      v[i] = pos[i] < hi[i] ? lt[i][(size_t)mid[i] * kListTile] : 0u;
+    }
+#pragma unroll
+    for (int i = 0; i < kSearch; ++i) {
+      if (pos[i] < hi[i]) {
+        if (v[i] < k) pos[i] = mid[i] + 1;
+        else hi[i] = mid[i];
+      }
+      more = more || pos[i] < hi[i];
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < kSearch; ++i)
+    if (pos[i] >= L[i] || lt[i][(size_t)pos[i] * kListTile] != k) pos[i] = kNoMirror;
+}
+
 // L2 prefetch hint for one address (PTX prefetch.global.L2; a hint, it returns nothing).
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 

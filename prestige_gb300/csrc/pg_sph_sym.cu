@@ -15,9 +15,9 @@
 //
 // Lists (sph_list_kernel) hold each slot's neighbours in ascending slot order: the entries below
 // the slot's own index come first.  Per step:
-//   sym_c1  for the entries above the slot (partner t > k): r^2, F, w, w F and r^2 + eps h^2 into
-//           the slot's entry planes; the position of k in t's list (binary search: t's list is
-//           ascending) into the mirror-index plane, and w F into t's entry there.
+//   sym_c1  for the entries above the slot (partner t > k): F, w, w F and r^2 + eps h^2 into the
+//           slot's entry planes; t and the position of k in t's list (binary search: t's list is
+//           ascending) into the mirror plane, and w F into t's entry there.
 //   sym_c2  every entry in order: w F from the entry (own, or the mirror t wrote), times m_t,
 //           into the continuity sum; then rho' and the packed {rho', P'} (the oracle's rho
 //           update and Tait term).
@@ -30,6 +30,15 @@
 // list reached its capacity before this slot) is evaluated in full where it is read, and an
 // overflowed list is followed by the rest of its candidate walk, evaluated in full, as in the
 // other modes.
+//
+// The kernels are bound by the FP64 pipe and, beside it, by the latency of their loads.  Against FP64
+// instructions for everything and all lanes of a warp at the same entry index (1M particles, ms: c1
+// 4.6, c2 0.44, m1 1.56, m2 1.58): divisions and roots on the integer pipe 2.95 / 0.41 / 0.94 / 1.57,
+// each lane from its own first entry above the slot, multiplications on the integer pipe and the
+// loads pipelined 2.0 / 0.40 / 0.91 / 1.09 (FP64 pipe 64 / 34 / 35 / 71 % busy, issue slots 40 to 60 %).
+// Below about 16,000 particles, where a warp or two share a scheduler and latency decides, the FP64
+// multiplication is the faster one (6.5k particles: 0.118 ms a step against 0.153), so the two-sided
+// passes and the DEM pass keep it.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -43,11 +52,13 @@ namespace {
 
 using namespace sphpass;
 
-typedef OpsD D;
-constexpr uint32_t kNoMirror = 0xFFFFFFFFu;
+typedef OpsDI D;  // multiplications, divisions and roots on the integer pipe
 
 // Entry planes of the per-entry store (a.fcache): doubles F, w, r^2 + eps h^2, S (w F after
-// sym_c1, X after sym_m1), then the u32 mirror index, each plane in the tiled list layout.
+// sym_c1, X after sym_m1), then the u32 pairs {mirror index, partner}, each plane in the tiled list
+// layout.  S is indexed like the list; the others, which only the slot itself reads, by the number
+// of the entry among those above the slot, so a warp whose lanes each start at their own first
+// entry above the slot still reads and writes whole rows of them.
 struct Planes {
   double* base;
   size_t plane;  // entries per plane
@@ -55,7 +66,7 @@ struct Planes {
   __device__ __forceinline__ double* W(size_t e) const { return base + plane + e; }
   __device__ __forceinline__ double* R(size_t e) const { return base + 2 * plane + e; }
   __device__ __forceinline__ double* S(size_t e) const { return base + 3 * plane + e; }
-  __device__ __forceinline__ uint32_t* M(size_t e) const { return (uint32_t*)(base + 4 * plane) + e; }
+  __device__ __forceinline__ uint2* M(size_t e) const { return (uint2*)(base + 4 * plane) + e; }
 };
 
 __device__ __forceinline__ Planes planes_of(const SphArgs& a) {
@@ -136,31 +147,21 @@ __device__ __forceinline__ void resume_walk(const SphArgs& a, const SphK& K, uin
   }
 }
 
-// Slot t's list holds slot k (a neighbour above t) as a stored entry, so t wrote the pair's
-// value into k's entry: t's list did not reach capacity before k (the list is ascending, so
-// then its last stored entry is at least k).
-__device__ __forceinline__ bool holds(const SphArgs& a, uint32_t t, uint32_t k) {
-  if (a.nlen[t] <= a.cap) return true;
-  return a.nlist[entry(t, a.cap - 1, a.cap)] >= k;
+// A pair without a stored value (a list at its capacity), everything from the packs; out of line, so the
+// passes' common path does not hold its registers.
+template <int DIM>
+__device__ __noinline__ double full_wF(const SphC<double>* c, const double4_32a* A, const double4_32a* B, uint32_t k,
+                                       uint32_t t) {
+  double d[3], r2, F, w;
+  pair_geometry<DIM>(*c, A[k], B[k], A[t], B[t], d, r2, F, w);
+  return D::mul(w, F);
 }
-
-// First of the L entries of an ascending tiled list that is not below k.
-__device__ __forceinline__ uint32_t lower_bound(const uint32_t* __restrict__ list, uint32_t L, uint32_t k) {
-  uint32_t lo = 0, hi = L;
-  while (lo < hi) {
-    const uint32_t mid = (lo + hi) >> 1;
-    if (list[(size_t)mid * kListTile] < k) lo = mid + 1;
-    else hi = mid;
-  }
-  return lo;
-}
-
-// Position of k in slot t's stored list, or kNoMirror.
-__device__ __forceinline__ uint32_t find_in_list(const SphArgs& a, uint32_t t, uint32_t k) {
-  const uint32_t L = min(a.nlen[t], a.cap);
-  const uint32_t* __restrict__ lt = a.nlist + list_base(t, a.cap);
-  const uint32_t q = lower_bound(lt, L, k);
-  return q < L && lt[(size_t)q * kListTile] == k ? q : kNoMirror;
+template <int DIM>
+__device__ __noinline__ double full_X(const SphC<double>* c, const double4_32a* A, const double4_32a* B,
+                                      const double2* Q, uint32_t k, uint32_t t) {
+  double d[3], r2, F, w;
+  pair_geometry<DIM>(*c, A[k], B[k], A[t], B[t], d, r2, F, w);
+  return momentum_factor(*c, F, w, D::add(r2, c->eps_h2), Q[k], Q[t]);
 }
 
 struct Slot {
@@ -196,22 +197,41 @@ __global__ void __launch_bounds__(kSphMaxThreads) sym_c1_kernel(SphArgs a, uint3
   const double4_32a* __restrict__ B = (const double4_32a*)a.s[1];
   const Planes P = planes_of(a);
   const double4_32a Ai = A[s.k], Bi = B[s.k];
-  // all lanes at the same entry index, so the entry-plane stores coalesce (starting each lane at
-  // its own first upper entry, found by binary search, measured the same)
-  for (uint32_t q = 0; q < s.L; ++q) {
-    const uint32_t t = my[(size_t)q * kListTile];
-    if (t < s.k) continue;
+  // each lane from its own first entry above the slot: with all lanes at the same entry index a third
+  // of them idled (21 of 32 active), while the FP64 pipe takes as long for 21 lanes as for 32
+  const uint32_t q0 = lower_bound(my, s.L, s.k), U = s.L - q0;
+  my += (size_t)q0 * kListTile;
+  // the positions of k in the partners' lists first, kSearch searches at a time (each is a chain of
+  // dependent loads)
+  for (uint32_t j = 0; j < U; j += kSearch) {
+    uint32_t t[kSearch], m[kSearch];
+#pragma unroll
+    for (int i = 0; i < kSearch; ++i) t[i] = my[(size_t)min(j + i, U - 1) * kListTile];
+    find_in_lists(a, t, s.k, m);
+#pragma unroll
+    for (int i = 0; i < kSearch; ++i)
+      if (j + i < U) *P.M(entry(s.k, j + i, a.cap)) = make_uint2(m[i], t[i]);
+  }
+  if (U == 0) return;
+  // software pipeline: entries two ahead, the partner's records one ahead
+  uint2 m = *P.M(entry(s.k, 0, a.cap)), mn = *P.M(entry(s.k, min(1u, U - 1), a.cap));
+  double4_32a Aj = A[m.y], Bj = B[m.y];
+  for (uint32_t j = 0; j < U; ++j) {
+    const uint2 mnn = *P.M(entry(s.k, min(j + 2, U - 1), a.cap));
+    const double4_32a An = A[mn.y], Bn = B[mn.y];
     double d[3], r2, F, w;
-    pair_geometry<DIM>(K.d, Ai, Bi, A[t], B[t], d, r2, F, w);
+    pair_geometry<DIM>(K.d, Ai, Bi, Aj, Bj, d, r2, F, w);
     const double wF = D::mul(w, F);
-    const size_t e = entry(s.k, q, a.cap);
+    const size_t e = entry(s.k, j, a.cap);
     *P.F(e) = F;
     *P.W(e) = w;
     *P.R(e) = D::add(r2, K.d.eps_h2);
-    *P.S(e) = wF;
-    const uint32_t m = find_in_list(a, t, s.k);
-    *P.M(e) = m;
-    if (m != kNoMirror) *P.S(entry(t, m, a.cap)) = wF;
+    *P.S(entry(s.k, q0 + j, a.cap)) = wF;
+    if (m.x != kNoMirror) *P.S(entry(m.y, m.x, a.cap)) = wF;
+    m = mn;
+    mn = mnn;
+    Aj = An;
+    Bj = Bn;
   }
 }
 
@@ -224,13 +244,9 @@ __global__ void __launch_bounds__(kSphMaxThreads) sym_c2_kernel(SphArgs a) {
   const double4_32a* __restrict__ A = (const double4_32a*)a.s[0];
   const double4_32a* __restrict__ B = (const double4_32a*)a.s[1];
   const Planes P = planes_of(a);
-  const double4_32a Ai = A[s.k], Bi = B[s.k];
+  const double4_32a Ai = A[s.k];
   const uint32_t* __restrict__ my = a.nlist + list_base(s.k, a.cap);
-  auto full = [&](uint32_t t) {
-    double d[3], r2, F, w;
-    pair_geometry<DIM>(c, Ai, Bi, A[t], B[t], d, r2, F, w);
-    return D::mul(w, F);
-  };
+  auto full = [&](uint32_t t) { return full_wF<DIM>(&c, A, B, s.k, t); };
   // software pipeline: list entries two ahead, the partner's mass and list length and the
   // entry's stored value one ahead (the pass waits on these loads; its FP64 work is two
   // operations per entry, summed in list order)
@@ -242,12 +258,16 @@ __global__ void __launch_bounds__(kSphMaxThreads) sym_c2_kernel(SphArgs a) {
   uint32_t nl = L > 0 ? a.nlen[t] : 0u;
   double sv = L > 0 ? *P.S(entry(s.k, 0, a.cap)) : 0.0;
   for (uint32_t q = 0; q < L; ++q) {
+    if (q + kL2Ahead < L) {
+      prefetch_l2(my + (size_t)(q + kL2Ahead) * kListTile);
+      prefetch_l2(P.S(entry(s.k, q + kL2Ahead, a.cap)));
+    }
     const uint32_t tnn = q + 2 < L ? my[(size_t)(q + 2) * kListTile] : 0u;
     const double mtn = q + 1 < L ? A[tn].w : 0.0;
     const uint32_t nln = q + 1 < L ? a.nlen[tn] : 0u;
     const double svn = q + 1 < L ? *P.S(entry(s.k, q + 1, a.cap)) : 0.0;
-    // the value is in the entry unless the partner below is one whose list did not reach this
-    // slot (holds())
+    // the value is in the entry unless the partner below is one whose list reached its capacity before
+    // this slot (lists ascend: then its last stored entry is below the slot)
     const bool stored = t > s.k || nl <= a.cap || a.nlist[entry(t, a.cap - 1, a.cap)] >= s.k;
     dr = D::add(dr, D::mul(mt, stored ? sv : full(t)));
     t = tn;
@@ -260,7 +280,7 @@ __global__ void __launch_bounds__(kSphMaxThreads) sym_c2_kernel(SphArgs a) {
   double* rho = (double*)a.rho;
   const double rn = D::add(rho[s.id], D::mul(c.dt, dr));
   rho[s.id] = rn;
-  ((double2*)a.s[2])[s.k] = make_double2(rn, tait_pterm<D>(c, K.gamma, rn));
+  ((double2*)a.s[2])[s.k] = make_double2(rn, tait_pterm<OpsD>(c, K.gamma, rn));
 }
 
 template <int DIM>
@@ -272,17 +292,28 @@ __global__ void __launch_bounds__(kSphMaxThreads) sym_m1_kernel(SphArgs a) {
   const Planes P = planes_of(a);
   const double2 qk = Q[s.k];
   const uint32_t* __restrict__ my = a.nlist + list_base(s.k, a.cap);
-  // all lanes at the same entry index, so the loads of the entry planes coalesce (this pass does
-  // little FP64 work per pair; starting each lane at its own first upper entry spread them over
-  // the lines of different entry rows and the pass took 20 % longer)
-  for (uint32_t q = 0; q < s.L; ++q) {
-    const uint32_t t = my[(size_t)q * kListTile];
-    if (t < s.k) continue;
-    const size_t e = entry(s.k, q, a.cap);
-    const double X = momentum_factor(K.d, *P.F(e), *P.W(e), *P.R(e), qk, Q[t]);
-    *P.S(e) = X;
-    const uint32_t m = *P.M(e);
-    if (m != kNoMirror) *P.S(entry(t, m, a.cap)) = X;
+  // each lane from its own first entry above the slot, as in sym_c1; the pass waits on its loads, so
+  // the partner's index is loaded two entries ahead and everything else one ahead
+  const uint32_t q0 = lower_bound(my, s.L, s.k), U = s.L - q0;
+  if (U == 0) return;
+  uint2 m = *P.M(entry(s.k, 0, a.cap)), mn = *P.M(entry(s.k, min(1u, U - 1), a.cap));
+  size_t e = entry(s.k, 0, a.cap);
+  double F = *P.F(e), w = *P.W(e), r2e = *P.R(e);
+  double2 qt = Q[m.y];
+  for (uint32_t j = 0; j < U; ++j) {
+    const uint2 mnn = *P.M(entry(s.k, min(j + 2, U - 1), a.cap));
+    e = entry(s.k, min(j + 1, U - 1), a.cap);
+    const double Fn = *P.F(e), wn = *P.W(e), rn = *P.R(e);
+    const double2 qn = Q[mn.y];
+    const double X = momentum_factor(K.d, F, w, r2e, qk, qt);
+    *P.S(entry(s.k, q0 + j, a.cap)) = X;
+    if (m.x != kNoMirror) *P.S(entry(m.y, m.x, a.cap)) = X;
+    m = mn;
+    mn = mnn;
+    F = Fn;
+    w = wn;
+    r2e = rn;
+    qt = qn;
   }
 }
 
@@ -297,30 +328,38 @@ __global__ void __launch_bounds__(kSphMaxThreads) sym_m2_kernel(SphArgs a) {
   const double2* __restrict__ Q = (const double2*)a.s[2];
   const Planes P = planes_of(a);
   const double4_32a Ai = A[s.k];
-  const double2 qk = Q[s.k];
   const uint32_t* __restrict__ my = a.nlist + list_base(s.k, a.cap);
   double acc[3] = {0.0, 0.0, 0.0};
-  // a pair without a stored X: everything from the packs
-  auto full = [&](uint32_t t, const double4_32a& Aj) {
-    double d[3], r2, F, w;
-    pair_geometry<DIM>(c, Ai, B[s.k], Aj, B[t], d, r2, F, w);
-    return momentum_factor(c, F, w, D::add(r2, c.eps_h2), qk, Q[t]);
-  };
+  auto full = [&](uint32_t t) { return full_X<DIM>(&c, A, B, Q, s.k, t); };
   auto add = [&](const double4_32a& Aj, double X) {
     const double coef = D::mul(Aj.w, X);
     acc[0] = D::sub(acc[0], D::mul(coef, D::sub(Ai.x, Aj.x)));
     acc[1] = D::sub(acc[1], D::mul(coef, D::sub(Ai.y, Aj.y)));
     if (DIM == 3) acc[2] = D::sub(acc[2], D::mul(coef, D::sub(Ai.z, Aj.z)));
   };
-  for (uint32_t q = 0; q < s.L; ++q) {
-    const uint32_t t = my[(size_t)q * kListTile];
-    const double4_32a Aj = A[t];
-    add(Aj, t > s.k || holds(a, t, s.k) ? *P.S(entry(s.k, q, a.cap)) : full(t, Aj));
+  // software pipeline: list entries two ahead; the partner's record and list length and the entry's
+  // stored value one ahead
+  const uint32_t L = s.L;
+  if (L > 0) {
+    uint32_t t = my[0], tn = my[(size_t)min(1u, L - 1) * kListTile];
+    double4_32a Aj = A[t];
+    uint32_t nl = a.nlen[t];
+    double X = *P.S(entry(s.k, 0, a.cap));
+    for (uint32_t q = 0; q < L; ++q) {
+      const uint32_t tnn = my[(size_t)min(q + 2, L - 1) * kListTile];
+      const double4_32a An = A[tn];
+      const uint32_t nln = a.nlen[tn];
+      const double Xn = *P.S(entry(s.k, min(q + 1, L - 1), a.cap));
+      const bool stored = t > s.k || nl <= a.cap || a.nlist[entry(t, a.cap - 1, a.cap)] >= s.k;  // as in sym_c2
+      add(Aj, stored ? X : full(t));
+      t = tn;
+      tn = tnn;
+      Aj = An;
+      nl = nln;
+      X = Xn;
+    }
   }
-  if (s.overflow) resume_walk<DIM>(a, K, s.k, Ai, [&](uint32_t t) {
-      const double4_32a Aj = A[t];
-      add(Aj, full(t, Aj));
-    });
+  if (s.overflow) resume_walk<DIM>(a, K, s.k, Ai, [&](uint32_t t) { add(A[t], full(t)); });
   if (s.id < K.fluid_end) {
     double* pos = (double*)a.pos;
     double* vel = (double*)a.vel;
@@ -348,7 +387,7 @@ SymKernel sym_kernel(int part) {
 
 }  // namespace
 
-size_t sph_sym_entry_bytes() { return 4 * sizeof(double) + sizeof(uint32_t); }
+size_t sph_sym_entry_bytes() { return 4 * sizeof(double) + 2 * sizeof(uint32_t); }
 
 int launch_sph_sym(cudaStream_t st, const SphArgs& a, int part, int block, uint32_t split, int second) {
   SymKernel kern = a.dim == 2 ? sym_kernel<2>(part) : sym_kernel<3>(part);

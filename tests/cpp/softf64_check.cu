@@ -1,5 +1,5 @@
-// soft_div and soft_sqrt (prestige_gb300/csrc/pg_softf64.cuh) against the IEEE operations of the
-// device (__ddiv_rn, __dsqrt_rn), bit for bit (NaNs as NaNs).  Run by tests/test_gpu_softf64.py.
+// soft_div, soft_sqrt and soft_mul (prestige_gb300/csrc/pg_softf64.cuh) against the IEEE operations of
+// the device (__ddiv_rn, __dsqrt_rn, __dmul_rn), bit for bit (NaNs as NaNs).  Run by tests/test_gpu_softf64.py.
 //   random bit patterns (every exponent, subnormals, infinities, NaNs)
 //   random significands with exponents near zero, and few-bit significands (exact quotients and roots)
 //   operands whose quotient or root lies next to a representable number or next to a midpoint of two
@@ -41,7 +41,7 @@ __device__ bool same(double a, double b) {
   return (a != a && b != b) || __double_as_longlong(a) == __double_as_longlong(b);
 }
 
-// bad[0..1]: mismatches of the division and of the root; ex: the first mismatching operands
+// bad[0..2]: mismatches of the division, the root and the product; ex: the first mismatching operands
 __global__ void check(uint64_t seed, int iters, unsigned long long* bad, double* ex) {
   const uint64_t id = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   for (int i = 0; i < iters; ++i) {
@@ -70,22 +70,34 @@ __global__ void check(uint64_t seed, int iters, unsigned long long* bad, double*
     if (!same(soft_sqrt(x), __dsqrt_rn(x))) {
       if (atomicAdd(bad + 1, 1ull) == 0) ex[2] = x;
     }
+    if (kind == 5) {  // factors of about 27 bits: products next to a tie
+      a = as_double((uint64_t)__double_as_longlong(operand(1, r)) & ~0ull << (24 + (r3 >> 12) % 4));
+      b = as_double((uint64_t)__double_as_longlong(operand(1, r2)) & ~0ull << (24 + (r3 >> 14) % 4));
+      if ((r3 >> 57) & 1) b = as_double((uint64_t)__double_as_longlong(b) + 1);
+    }
+    if (!same(soft_mul(a, b), __dmul_rn(a, b))) {
+      if (atomicAdd(bad + 2, 1ull) == 0) {
+        ex[3] = a;
+        ex[4] = b;
+      }
+    }
   }
 }
 
 int main() {
   unsigned long long* bad;
   double* ex;
-  if (cudaMallocManaged(&bad, 16) != cudaSuccess || cudaMallocManaged(&ex, 24) != cudaSuccess) return 2;
-  bad[0] = bad[1] = 0;
+  if (cudaMallocManaged(&bad, 24) != cudaSuccess || cudaMallocManaged(&ex, 40) != cudaSuccess) return 2;
+  bad[0] = bad[1] = bad[2] = 0;
   for (int rep = 0; rep < 4; ++rep) check<<<1024, 256>>>(1234567ull + ((uint64_t)rep << 40), 256, bad, ex);
   const cudaError_t e = cudaDeviceSynchronize();
   if (e != cudaSuccess) {
     fprintf(stderr, "%s\n", cudaGetErrorString(e));
     return 2;
   }
-  printf("268M operand pairs: %llu quotients and %llu roots differ\n", bad[0], bad[1]);
+  printf("268M operand pairs: %llu quotients, %llu roots and %llu products differ\n", bad[0], bad[1], bad[2]);
   if (bad[0]) fprintf(stderr, "division: %a / %a\n", ex[0], ex[1]);
   if (bad[1]) fprintf(stderr, "root: %a\n", ex[2]);
-  return bad[0] || bad[1] ? 1 : 0;
+  if (bad[2]) fprintf(stderr, "product: %a * %a\n", ex[3], ex[4]);
+  return bad[0] || bad[1] || bad[2] ? 1 : 0;
 }
