@@ -36,17 +36,22 @@ namespace {
 
 using namespace sphpass;
 
-constexpr int kPlanes = 15;  // doubles per list entry (plus one u32)
+constexpr int kPlanes = 15;  // doubles per list entry (plus the mirror index and the partner)
 // the partner's momentum share (Vx, Vv, F x.E, Pi / rho_ij); for the continuity pass, the pair's
-// vectors U1 = G w x + F v and U2 = F x and the partner's mass (own entries above the slot)
+// vectors U1 = G w x + F v and U2 = F x and the partner's mass (own entries above the slot).  The first
+// group is indexed like the list; the second and {mirror index, partner}, which only the slot
+// itself reads, by the number of the entry among those above the slot, so lanes that each start at
+// their own first entry above the slot read and write whole rows of them.
 enum { kMx = 0, kMv = 3, kFxE = 6, kPIrb = 7, kU1 = 8, kU2 = 11, kMt = 14 };
+constexpr int kAdjBlock = 128;
+constexpr int kAdjLanes = 4;  // threads per slot
 constexpr int kSlotSums = 9;  // per-slot partial sums: gx (3), gv (3), gr, gal, gB
 
 struct Planes {
   double* base;
   size_t plane;  // entries per plane
   __device__ __forceinline__ double& at(int j, size_t e) const { return base[j * plane + e]; }
-  __device__ __forceinline__ uint32_t& mirror(size_t e) const { return ((uint32_t*)(base + kPlanes * plane))[e]; }
+  __device__ __forceinline__ uint2& mirror(size_t e) const { return ((uint2*)(base + kPlanes * plane))[e]; }
 };
 
 __device__ __forceinline__ Planes planes_of(const SphArgs& a) {
@@ -217,13 +222,19 @@ __device__ __forceinline__ void resume_walk(const SphArgs& a, const SphK& K, con
   }
 }
 
+// LANES threads share a slot: thread `sub` takes every LANES-th entry of its loops and the
+// partial sums are added at the end in a fixed order.
+template <int LANES>
 struct Slot {
-  uint32_t k, id, L;
+  uint32_t k, id, L, sub;
   bool overflow;
 };
 
-__device__ __forceinline__ bool slot_of(const SphArgs& a, Slot& s) {
-  s.k = blockIdx.x * blockDim.x + threadIdx.x;
+template <int LANES>
+__device__ __forceinline__ bool slot_of(const SphArgs& a, Slot<LANES>& s) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  s.k = i / LANES;
+  s.sub = i % LANES;
   if (s.k >= a.n) return false;
   s.id = a.sorted_id[s.k];
   const uint32_t cnt = a.nlen[s.k];
@@ -232,47 +243,74 @@ __device__ __forceinline__ bool slot_of(const SphArgs& a, Slot& s) {
   return true;
 }
 
+// v summed over the threads of the slot (all of them call this; every one gets the sum).
+template <int LANES>
+__device__ __forceinline__ double lane_sum(double v) {
+  if (LANES == 1) return v;
+  const int lane = threadIdx.x & 31;
+  const unsigned group = ((1u << LANES) - 1u) << (lane & ~(LANES - 1));
+#pragma unroll
+  for (int o = 1; o < LANES; o <<= 1) v += __shfl_xor_sync(group, v, o);
+  return v;
+}
+
+template <int LANES>
+__device__ __forceinline__ void lane_sums(Sums& s, int count) {
+  if (LANES == 1) return;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    s.gx[c] = lane_sum<LANES>(s.gx[c]);
+    s.gv[c] = lane_sum<LANES>(s.gv[c]);
+  }
+  if (count > 6) {
+    s.gr = lane_sum<LANES>(s.gr);
+    s.gal = lane_sum<LANES>(s.gal);
+    s.gB = lane_sum<LANES>(s.gB);
+  }
+}
+
 __device__ __forceinline__ void store_sums(const SphArgs& a, const Packs& P, uint32_t k, const Sums& s, int count) {
   const double v[kSlotSums] = {s.gx[0], s.gx[1], s.gx[2], s.gv[0], s.gv[1], s.gv[2], s.gr, s.gal, s.gB};
   for (int j = 0; j < count; ++j) P.PS[(size_t)j * a.n + k] = v[j];
 }
 
-__device__ __forceinline__ Sums load_sums(const SphArgs& a, const Packs& P, uint32_t k, int count) {
+__device__ __forceinline__ void add_stored_sums(const SphArgs& a, const Packs& P, uint32_t k, Sums& s, int count) {
   double v[kSlotSums] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
   for (int j = 0; j < count; ++j) v[j] = P.PS[(size_t)j * a.n + k];
-  Sums s;
   for (int c = 0; c < 3; ++c) {
-    s.gx[c] = v[c];
-    s.gv[c] = v[3 + c];
+    s.gx[c] += v[c];
+    s.gv[c] += v[3 + c];
   }
-  s.gr = v[6];
-  s.gal = v[7];
-  s.gB = v[8];
-  return s;
+  s.gr += v[6];
+  s.gal += v[7];
+  s.gB += v[8];
 }
 
 // The mirror index of every entry above its slot: the position of the slot in the partner's
 // list (a binary search, latency-bound; apart from the FP64 work of adj_a1 it runs at full
 // occupancy).
+template <int LANES>
 __global__ void __launch_bounds__(kSphMaxThreads) adj_mirror_kernel(SphArgs a) {
-  Slot s;
+  Slot<LANES> s;
   if (!slot_of(a, s)) return;
   const Planes E = planes_of(a);
   const uint32_t* __restrict__ my = a.nlist + list_base(s.k, a.cap);
-  for (uint32_t q = lower_bound(my, s.L, s.k); q < s.L; q += kSearch) {
+  const uint32_t q0 = lower_bound(my, s.L, s.k), U = s.L - q0;
+  my += (size_t)q0 * kListTile;
+  for (uint32_t j = s.sub * kSearch; j < U; j += LANES * kSearch) {
     uint32_t t[kSearch], m[kSearch];
 #pragma unroll
-    for (int i = 0; i < kSearch; ++i) t[i] = my[(size_t)min(q + i, s.L - 1) * kListTile];
+    for (int i = 0; i < kSearch; ++i) t[i] = my[(size_t)min(j + i, U - 1) * kListTile];
     find_in_lists(a, t, s.k, m);
 #pragma unroll
     for (int i = 0; i < kSearch; ++i)
-      if (q + i < s.L) E.mirror(entry(s.k, q + i, a.cap)) = m[i];
+      if (j + i < U) E.mirror(entry(s.k, j + i, a.cap)) = make_uint2(m[i], t[i]);
   }
 }
 
-template <int DIM>
+template <int DIM, int LANES>
 __global__ void __launch_bounds__(kSphMaxThreads) adj_a1_kernel(SphArgs a) {
-  Slot s;
+  Slot<LANES> s;
   if (!slot_of(a, s)) return;
   const SphK& K = a.sys[0];
   const Packs P(a);
@@ -283,35 +321,36 @@ __global__ void __launch_bounds__(kSphMaxThreads) adj_a1_kernel(SphArgs a) {
   Sums sum = {{0, 0, 0}, {0, 0, 0}, 0, 0, 0};
   // each lane from its own first entry above the slot, so the lanes of a warp evaluate their
   // pairs in the same iterations
-  for (uint32_t q = lower_bound(my, s.L, s.k); q < s.L; ++q) {
-    const uint32_t t = my[(size_t)q * kListTile];
-    const MomTerms<DIM> m = mom_terms<DIM>(K, P, s.k, t, xk, vk);
-    const size_t e = entry(s.k, q, a.cap);
+  const uint32_t U = s.L - lower_bound(my, s.L, s.k);
+  for (uint32_t j = s.sub; j < U; j += LANES) {
+    const size_t e = entry(s.k, j, a.cap);
+    const uint2 mt = E.mirror(e);
+    const MomTerms<DIM> m = mom_terms<DIM>(K, P, s.k, mt.y, xk, vk);
 #pragma unroll
     for (int cc = 0; cc < DIM; ++cc) {
       E.at(kU1 + cc, e) = m.U1[cc];
       E.at(kU2 + cc, e) = m.U2[cc];
     }
     E.at(kMt, e) = m.mt;
-    const uint32_t mt = E.mirror(e);
-    if (mt != kNoMirror) {
-      const size_t f = entry(t, mt, a.cap);
+    if (mt.x != kNoMirror) {
+      const size_t f = entry(mt.y, mt.x, a.cap);
 #pragma unroll
-      for (int cc = 0; cc < 3; ++cc) {
+      for (int cc = 0; cc < DIM; ++cc) {
         E.at(kMx + cc, f) = m.Vx[cc];
         E.at(kMv + cc, f) = m.Vv[cc];
       }
       E.at(kFxE, f) = m.FxE;
       E.at(kPIrb, f) = m.PIrb;
     }
-    add_own<DIM>(sum, m, Pdk, mt != kNoMirror ? 1.0 : 0.5);
+    add_own<DIM>(sum, m, Pdk, mt.x != kNoMirror ? 1.0 : 0.5);
   }
-  store_sums(a, P, s.k, sum, kSlotSums);
+  lane_sums<LANES>(sum, kSlotSums);
+  if (s.sub == 0) store_sums(a, P, s.k, sum, kSlotSums);
 }
 
-template <int DIM>
+template <int DIM, int LANES>
 __global__ void __launch_bounds__(kSphMaxThreads) adj_a2_kernel(SphArgs a) {
-  Slot s;
+  Slot<LANES> s;
   if (!slot_of(a, s)) return;
   const SphK& K = a.sys[0];
   const Packs P(a);
@@ -319,9 +358,9 @@ __global__ void __launch_bounds__(kSphMaxThreads) adj_a2_kernel(SphArgs a) {
   const double4_32a xk = P.X[s.k], vk = P.V[s.k];
   const double Pdk = P.Q[s.k].y;
   const uint32_t* __restrict__ my = a.nlist + list_base(s.k, a.cap);
-  Sums sum = load_sums(a, P, s.k, kSlotSums);
+  Sums sum = {{0, 0, 0}, {0, 0, 0}, 0, 0, 0};
   const uint32_t below = lower_bound(my, s.L, s.k);  // the entries below the slot come first
-  for (uint32_t q = 0; q < below; ++q) {
+  for (uint32_t q = s.sub; q < below; q += LANES) {
     const uint32_t t = my[(size_t)q * kListTile];
     if (holds(a, t, s.k)) {  // t's share of the pair was written here by t: negate it
       const size_t e = entry(s.k, q, a.cap);
@@ -335,9 +374,12 @@ __global__ void __launch_bounds__(kSphMaxThreads) adj_a2_kernel(SphArgs a) {
       add_own<DIM>(sum, mom_terms<DIM>(K, P, s.k, t, xk, vk), Pdk, 0.5);
     }
   }
-  if (s.overflow)
+  if (s.overflow && s.sub == 0)
     resume_walk<DIM>(a, K, P, s.k, xk,
                      [&](uint32_t t) { add_own<DIM>(sum, mom_terms<DIM>(K, P, s.k, t, xk, vk), Pdk, 0.5); });
+  lane_sums<LANES>(sum, kSlotSums);
+  if (s.sub != 0) return;
+  add_stored_sums(a, P, s.k, sum, kSlotSums);
   // the momentum adjoint's update: lx += gx, lv += dt lx' (fluid) + gv, lr += gr, dbar = dt lr for
   // the continuity pass, and the parameter sums
   double* lx = (double*)a.lam[0];
@@ -375,55 +417,75 @@ __device__ __forceinline__ void cont_full(const SphK& K, const Packs& P, uint32_
   }
 }
 
-template <int DIM>
+template <int DIM, int LANES>
 __global__ void __launch_bounds__(kSphMaxThreads) adj_c1_kernel(SphArgs a) {
-  Slot s;
+  Slot<LANES> s;
   if (!slot_of(a, s)) return;
   const Packs P(a);
   const Planes E = planes_of(a);
   const double mk = P.X[s.k].w, dbk = P.DB[s.k];
   const uint32_t* __restrict__ my = a.nlist + list_base(s.k, a.cap);
   Sums sum = {{0, 0, 0}, {0, 0, 0}, 0, 0, 0};
-  // all lanes at the same entry index, so the entry-plane loads coalesce (this pass waits on its
-  // loads; starting each lane at its own first upper entry made it slower)
-  for (uint32_t q = 0; q < s.L; ++q) {
-    const uint32_t t = my[(size_t)q * kListTile];
-    if (t < s.k) continue;
-    const size_t e = entry(s.k, q, a.cap);
-    const double D = dbk * E.at(kMt, e) + P.DB[t] * mk;
-    double Vx[3] = {0, 0, 0}, Vv[3] = {0, 0, 0};
+  // this pass waits on its loads: the partner two entries ahead, everything else one ahead
+  const uint32_t U = s.L - lower_bound(my, s.L, s.k);
+  if (s.sub < U) {
+    auto row = [&](uint32_t j) { return entry(s.k, min(j, U - 1), a.cap); };
+    struct Vals {
+      double u1[DIM], u2[DIM], mt, db;
+    };
+    auto load = [&](size_t e, uint32_t t, Vals& v) {
 #pragma unroll
-    for (int cc = 0; cc < DIM; ++cc) {
-      Vx[cc] = D * E.at(kU1 + cc, e);
-      Vv[cc] = D * E.at(kU2 + cc, e);
-      sum.gx[cc] += Vx[cc];
-      sum.gv[cc] += Vv[cc];
-    }
-    const uint32_t mt = E.mirror(e);
-    if (mt != kNoMirror) {
-      const size_t f = entry(t, mt, a.cap);
-#pragma unroll
-      for (int cc = 0; cc < 3; ++cc) {
-        E.at(kMx + cc, f) = Vx[cc];
-        E.at(kMv + cc, f) = Vv[cc];
+      for (int cc = 0; cc < DIM; ++cc) {
+        v.u1[cc] = E.at(kU1 + cc, e);
+        v.u2[cc] = E.at(kU2 + cc, e);
       }
+      v.mt = E.at(kMt, e);
+      v.db = P.DB[t];
+    };
+    uint2 m = E.mirror(row(s.sub)), mn = E.mirror(row(s.sub + LANES));
+    Vals v, vn;
+    load(row(s.sub), m.y, v);
+    for (uint32_t j = s.sub; j < U; j += LANES) {
+      const uint2 mnn = E.mirror(row(j + 2 * LANES));
+      load(row(j + LANES), mn.y, vn);
+      const double D = dbk * v.mt + v.db * mk;
+      double Vx[DIM], Vv[DIM];
+#pragma unroll
+      for (int cc = 0; cc < DIM; ++cc) {
+        Vx[cc] = D * v.u1[cc];
+        Vv[cc] = D * v.u2[cc];
+        sum.gx[cc] += Vx[cc];
+        sum.gv[cc] += Vv[cc];
+      }
+      if (m.x != kNoMirror) {
+        const size_t f = entry(m.y, m.x, a.cap);
+#pragma unroll
+        for (int cc = 0; cc < DIM; ++cc) {
+          E.at(kMx + cc, f) = Vx[cc];
+          E.at(kMv + cc, f) = Vv[cc];
+        }
+      }
+      m = mn;
+      mn = mnn;
+      v = vn;
     }
   }
-  store_sums(a, P, s.k, sum, 6);
+  lane_sums<LANES>(sum, 6);
+  if (s.sub == 0) store_sums(a, P, s.k, sum, 6);
 }
 
-template <int DIM>
+template <int DIM, int LANES>
 __global__ void __launch_bounds__(kSphMaxThreads) adj_c2_kernel(SphArgs a) {
-  Slot s;
+  Slot<LANES> s;
   if (!slot_of(a, s)) return;
   const SphK& K = a.sys[0];
   const Packs P(a);
   const Planes E = planes_of(a);
   const double4_32a xk = P.X[s.k], vk = P.V[s.k];
   const uint32_t* __restrict__ my = a.nlist + list_base(s.k, a.cap);
-  Sums sum = load_sums(a, P, s.k, 6);
+  Sums sum = {{0, 0, 0}, {0, 0, 0}, 0, 0, 0};
   const uint32_t below = lower_bound(my, s.L, s.k);
-  for (uint32_t q = 0; q < below; ++q) {
+  for (uint32_t q = s.sub; q < below; q += LANES) {
     const uint32_t t = my[(size_t)q * kListTile];
     if (holds(a, t, s.k)) {
       const size_t e = entry(s.k, q, a.cap);
@@ -436,7 +498,11 @@ __global__ void __launch_bounds__(kSphMaxThreads) adj_c2_kernel(SphArgs a) {
       cont_full<DIM>(K, P, s.k, t, xk, vk, sum);
     }
   }
-  if (s.overflow) resume_walk<DIM>(a, K, P, s.k, xk, [&](uint32_t t) { cont_full<DIM>(K, P, s.k, t, xk, vk, sum); });
+  if (s.overflow && s.sub == 0)
+    resume_walk<DIM>(a, K, P, s.k, xk, [&](uint32_t t) { cont_full<DIM>(K, P, s.k, t, xk, vk, sum); });
+  lane_sums<LANES>(sum, 6);
+  if (s.sub != 0) return;
+  add_stored_sums(a, P, s.k, sum, 6);
   double* lx = (double*)a.lam[0];
   double* lv = (double*)a.lam[1];
 #pragma unroll
@@ -449,31 +515,32 @@ __global__ void __launch_bounds__(kSphMaxThreads) adj_c2_kernel(SphArgs a) {
 
 typedef void (*AdjSymKernel)(SphArgs);
 
-template <int DIM>
+template <int DIM, int LANES>
 AdjSymKernel adj_sym_kernel(int part) {
   switch (part) {
-    case 0: return adj_mirror_kernel;
-    case 1: return adj_a1_kernel<DIM>;
-    case 2: return adj_a2_kernel<DIM>;
-    case 3: return adj_c1_kernel<DIM>;
-    case 4: return adj_c2_kernel<DIM>;
+    case 0: return adj_mirror_kernel<LANES>;
+    case 1: return adj_a1_kernel<DIM, LANES>;
+    case 2: return adj_a2_kernel<DIM, LANES>;
+    case 3: return adj_c1_kernel<DIM, LANES>;
+    case 4: return adj_c2_kernel<DIM, LANES>;
     default: return nullptr;
   }
 }
 
 }  // namespace
 
-size_t adjoint_sym_entry_bytes() { return kPlanes * sizeof(double) + sizeof(uint32_t); }
+size_t adjoint_sym_entry_bytes() { return kPlanes * sizeof(double) + 2 * sizeof(uint32_t); }
 size_t adjoint_sym_slot_bytes() { return kSlotSums * sizeof(double); }
 
 int launch_adjoint_sym(cudaStream_t st, const SphArgs& a, int part) {
-  AdjSymKernel kern = a.dim == 2 ? adj_sym_kernel<2>(part) : adj_sym_kernel<3>(part);
+  AdjSymKernel kern = a.dim == 2 ? adj_sym_kernel<2, kAdjLanes>(part) : adj_sym_kernel<3, kAdjLanes>(part);
   if (!kern) {
     set_error("unknown part %d of the pair-once adjoint", part);
     return PG_EINVAL;
   }
   if (a.n == 0) return PG_OK;
-  kern<<<(a.n + kSphThreads - 1) / kSphThreads, kSphThreads, 0, st>>>(a);
+  const unsigned blocks = (unsigned)(((size_t)a.n * kAdjLanes + kAdjBlock - 1) / kAdjBlock);
+  kern<<<blocks, kAdjBlock, 0, st>>>(a);
   PG_CUDA_TRY(cudaGetLastError());
   return PG_OK;
 }

@@ -252,12 +252,11 @@ long long neighbor_launches(const pg_system* s) { return s->nw.chunks > 1 ? 4 : 
 // continuity pass (rho' into the canonical density and the sorted pack).  ev (optional): events
 // 0-4 of a step (start, after the neighbour search, after the sorted gather, after the lists,
 // after the continuity pass).
-// The IEEE f64 step evaluates each pair once (pg_sph_sym.cu: four kernels) from 16,384 particles;
-// below, where the step is bound by the latency of its launches, the two-sided passes (two
-// kernels) are faster: the 6,518-particle dam break took 0.149 against 0.125 ms per step.  Both
-// give the oracle's bits.
-constexpr size_t kPairOnceMin = 16384;
-bool pair_once(const pg_system* s) { return s->arith == ARITH_F64_EXACT && s->n >= kPairOnceMin; }
+// The IEEE f64 step evaluates each pair once (pg_sph_sym.cu: four kernels) at every size.  The two-sided
+// passes (two launches) were the faster ones below 16,384 particles while a slot's pairs ran on one
+// thread; with four threads per slot the 2D dam break of 6,518 particles takes 72 us a step
+// pair-once against 92 two-sided, 4,000 particles in 3D 162 against 266.  Both give the oracle's bits.
+bool pair_once(const pg_system* s) { return s->arith == ARITH_F64_EXACT; }
 
 int enqueue_sph_front(pg_system* s, cudaEvent_t* ev) {
   if (ev) PG_CUDA_TRY(cudaEventRecord(ev[0], s->stream));
@@ -615,7 +614,12 @@ int choose_pass_grid(pg_system* s) {
   PG_CUDA_TRY(cudaGetDevice(&dev));
   PG_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   for (int st = 0; st < 3; ++st) {
-    const int occ = sph_list_occupancy(s->arith, s->dim, s->grids[0].reach, st, st == SPH_MOM ? mom_block(s) : s->block, s->lanes);
+    const int block = st == SPH_MOM ? mom_block(s) : s->block;
+    if (st != SPH_RATES && pair_once(s)) {  // one block per tile
+      s->pass_grid[st] = (int)((s->n + block - 1) / block);
+      continue;
+    }
+    const int occ = sph_list_occupancy(s->arith, s->dim, s->grids[0].reach, st, block, s->lanes);
     s->pass_grid[st] = occ > 0 ? occ * sms : 0;  // persistent: one resident wave
   }
   const int locc = sph_list_occupancy(s->arith, s->dim, s->grids[0].reach, -1, s->block);

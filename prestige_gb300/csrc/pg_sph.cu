@@ -538,8 +538,9 @@ PassKernel list_pass_for(int arith, int lanes) {
   if (lanes == 2) return list_pass_lanes<DIM, STAGE, 2>(arith);
   if (lanes == 4) return list_pass_lanes<DIM, STAGE, 4>(arith);
   switch (arith) {
-    case ARITH_F64_EXACT:
-      return sph_list_pass_kernel<RealPairs<OpsD, DIM, true, STAGE>, DIM, false>;
+    case ARITH_F64_EXACT:  // (the step's passes: pg_sph_sym.cu)
+      if constexpr (STAGE == SPH_RATES) return sph_list_pass_kernel<RealPairs<OpsD, DIM, true, STAGE>, DIM, false>;
+      else return nullptr;
     case ARITH_F64_DF:
       return sph_list_pass_kernel<DfPairs<DIM, STAGE>, DIM, false>;
     case ARITH_F32_EXACT:

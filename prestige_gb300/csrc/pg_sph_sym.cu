@@ -33,12 +33,13 @@
 //
 // The kernels are bound by the FP64 pipe and, beside it, by the latency of their loads.  Against FP64
 // instructions for everything and all lanes of a warp at the same entry index (1M particles, ms: c1
-// 4.6, c2 0.44, m1 1.56, m2 1.58): divisions and roots on the integer pipe 2.95 / 0.41 / 0.94 / 1.57,
+// 4.6, c2 0.44, m1 1.56, m2 1.58): divisions and roots on the integer pipe 2.95 / 0.41 / 0.94 / 1.57;
 // each lane from its own first entry above the slot, multiplications on the integer pipe and the
-// loads pipelined 2.0 / 0.40 / 0.91 / 1.09 (FP64 pipe 64 / 34 / 35 / 71 % busy, issue slots 40 to 60 %).
-// Below about 16,000 particles, where a warp or two share a scheduler and latency decides, the FP64
-// multiplication is the faster one (6.5k particles: 0.118 ms a step against 0.153), so the two-sided
-// passes and the DEM pass keep it.
+// loads pipelined 2.0 / 0.40 / 0.91 / 1.09 (FP64 pipe 64 / 34 / 35 / 71 % busy, issue slots 40 to 60 %);
+// four threads per slot in c1 and m1 another 0.25 less together.
+// Where a warp or two share a scheduler and latency decides, the FP64 multiplication is the faster
+// one (two-sided passes at 6.5k particles: 0.118 ms a step against 0.153 with soft_mul; the dense DEM
+// pass 0.296 against 0.368), so only these kernels use the integer one.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -164,13 +165,21 @@ __device__ __noinline__ double full_X(const SphC<double>* c, const double4_32a* 
   return momentum_factor(*c, F, w, D::add(r2, c->eps_h2), Q[k], Q[t]);
 }
 
+// LANES threads share a slot in the pair-value kernels: thread `sub` takes every LANES-th entry (the values
+// do not depend on who evaluates them).  With 8 slots to a warp the slots' entry counts differ less
+// than with 32, and a small system fills more of the chip.
+constexpr int kPairLanes = 4;
+
 struct Slot {
-  uint32_t k, id, L;
+  uint32_t k, id, L, sub;
   bool overflow;
 };
 
+template <int LANES = 1>
 __device__ __forceinline__ bool slot_of(const SphArgs& a, Slot& s) {
-  s.k = a.k_begin + blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  s.k = a.k_begin + i / LANES;
+  s.sub = i % LANES;
   if (s.k >= a.k_end) return false;
   s.id = a.sorted_id[s.k];
   const uint32_t cnt = a.nlen[s.k];
@@ -186,7 +195,7 @@ __device__ __forceinline__ bool slot_of(const SphArgs& a, Slot& s) {
 template <int DIM>
 __global__ void __launch_bounds__(kSphMaxThreads) sym_c1_kernel(SphArgs a, uint32_t split, int second) {
   Slot s;
-  if (!slot_of(a, s)) return;
+  if (!slot_of<kPairLanes>(a, s)) return;
   const uint32_t* __restrict__ my = a.nlist + list_base(s.k, a.cap);
   if (split) {
     const bool early = s.k < split && (s.L == 0 || my[(size_t)(s.L - 1) * kListTile] < split);
@@ -203,21 +212,24 @@ __global__ void __launch_bounds__(kSphMaxThreads) sym_c1_kernel(SphArgs a, uint3
   my += (size_t)q0 * kListTile;
   // the positions of k in the partners' lists first, kSearch searches at a time (each is a chain of
   // dependent loads)
-  for (uint32_t j = 0; j < U; j += kSearch) {
+  for (uint32_t j = s.sub; j < U; j += kPairLanes * kSearch) {
     uint32_t t[kSearch], m[kSearch];
 #pragma unroll
-    for (int i = 0; i < kSearch; ++i) t[i] = my[(size_t)min(j + i, U - 1) * kListTile];
+    for (int i = 0; i < kSearch; ++i) t[i] = my[(size_t)min(j + i * kPairLanes, U - 1) * kListTile];
     find_in_lists(a, t, s.k, m);
 #pragma unroll
     for (int i = 0; i < kSearch; ++i)
-      if (j + i < U) *P.M(entry(s.k, j + i, a.cap)) = make_uint2(m[i], t[i]);
+      if (j + i * kPairLanes < U) *P.M(entry(s.k, j + i * kPairLanes, a.cap)) = make_uint2(m[i], t[i]);
   }
-  if (U == 0) return;
-  // software pipeline: entries two ahead, the partner's records one ahead
-  uint2 m = *P.M(entry(s.k, 0, a.cap)), mn = *P.M(entry(s.k, min(1u, U - 1), a.cap));
+  if (s.sub >= U) return;
+  // software pipeline: entries two ahead, the partner's records one ahead (each thread reads back the
+  // entries it wrote above)
+  constexpr uint32_t N = kPairLanes;
+  const uint32_t last = s.sub + (U - 1 - s.sub) / N * N;  // the thread's last entry
+  uint2 m = *P.M(entry(s.k, s.sub, a.cap)), mn = *P.M(entry(s.k, min(s.sub + N, last), a.cap));
   double4_32a Aj = A[m.y], Bj = B[m.y];
-  for (uint32_t j = 0; j < U; ++j) {
-    const uint2 mnn = *P.M(entry(s.k, min(j + 2, U - 1), a.cap));
+  for (uint32_t j = s.sub; j < U; j += N) {
+    const uint2 mnn = *P.M(entry(s.k, min(j + 2 * N, last), a.cap));
     const double4_32a An = A[mn.y], Bn = B[mn.y];
     double d[3], r2, F, w;
     pair_geometry<DIM>(K.d, Ai, Bi, Aj, Bj, d, r2, F, w);
@@ -286,7 +298,7 @@ __global__ void __launch_bounds__(kSphMaxThreads) sym_c2_kernel(SphArgs a) {
 template <int DIM>
 __global__ void __launch_bounds__(kSphMaxThreads) sym_m1_kernel(SphArgs a) {
   Slot s;
-  if (!slot_of(a, s)) return;
+  if (!slot_of<kPairLanes>(a, s)) return;
   const SphK& K = a.sys[sys_of_slot(a, s.id)];
   const double2* __restrict__ Q = (const double2*)a.s[2];
   const Planes P = planes_of(a);
@@ -295,14 +307,15 @@ __global__ void __launch_bounds__(kSphMaxThreads) sym_m1_kernel(SphArgs a) {
   // each lane from its own first entry above the slot, as in sym_c1; the pass waits on its loads, so
   // the partner's index is loaded two entries ahead and everything else one ahead
   const uint32_t q0 = lower_bound(my, s.L, s.k), U = s.L - q0;
-  if (U == 0) return;
-  uint2 m = *P.M(entry(s.k, 0, a.cap)), mn = *P.M(entry(s.k, min(1u, U - 1), a.cap));
-  size_t e = entry(s.k, 0, a.cap);
+  if (s.sub >= U) return;
+  constexpr uint32_t N = kPairLanes;
+  uint2 m = *P.M(entry(s.k, s.sub, a.cap)), mn = *P.M(entry(s.k, min(s.sub + N, U - 1), a.cap));
+  size_t e = entry(s.k, s.sub, a.cap);
   double F = *P.F(e), w = *P.W(e), r2e = *P.R(e);
   double2 qt = Q[m.y];
-  for (uint32_t j = 0; j < U; ++j) {
-    const uint2 mnn = *P.M(entry(s.k, min(j + 2, U - 1), a.cap));
-    e = entry(s.k, min(j + 1, U - 1), a.cap);
+  for (uint32_t j = s.sub; j < U; j += N) {
+    const uint2 mnn = *P.M(entry(s.k, min(j + 2 * N, U - 1), a.cap));
+    e = entry(s.k, min(j + N, U - 1), a.cap);
     const double Fn = *P.F(e), wn = *P.W(e), rn = *P.R(e);
     const double2 qn = Q[mn.y];
     const double X = momentum_factor(K.d, F, w, r2e, qk, qt);
@@ -400,7 +413,8 @@ int launch_sph_sym(cudaStream_t st, const SphArgs& a, int part, int block, uint3
     return PG_EINVAL;
   }
   if (a.k_end <= a.k_begin) return PG_OK;
-  const unsigned blocks = (unsigned)((a.k_end - a.k_begin + block - 1) / block);
+  const int lanes = part == 0 || part == 2 ? kPairLanes : 1;
+  const unsigned blocks = (unsigned)(((size_t)(a.k_end - a.k_begin) * lanes + block - 1) / block);
   if (part == 0) {
     if (a.dim == 2) sym_c1_kernel<2><<<blocks, block, 0, st>>>(a, split, second);
     else sym_c1_kernel<3><<<blocks, block, 0, st>>>(a, split, second);
