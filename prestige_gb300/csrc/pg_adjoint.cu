@@ -115,6 +115,7 @@ using namespace sphpass;
 //   X4 {x, y, z, m}   V4 {vx, vy, vz, rho'}   Q4 {P, P'(rho'), P/B, 0}   A4 {abar, 0}   pf FP32 x
 template <int DIM>
 __global__ void adjoint_prep_kernel(SphArgs a) {
+  chain_begin();
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= a.n) return;
   const uint32_t id = a.sorted_id[k];
@@ -180,6 +181,7 @@ __device__ __noinline__ bool approaches_f64(const float4* XH, const float4* XL, 
 
 template <int DIM>
 __global__ void adjoint_prep_f_kernel(SphArgs a) {
+  chain_begin();
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= a.n) return;
   const uint32_t id = a.sorted_id[k];
@@ -416,11 +418,11 @@ int launch_adjoint_prep(cudaStream_t st, const SphArgs& a, bool fp32) {
   if (a.n == 0) return PG_OK;
   const unsigned b = (a.n + 255) / 256;
   if (fp32) {
-    if (a.dim == 2) adjoint_prep_f_kernel<2><<<b, 256, 0, st>>>(a);
-    else adjoint_prep_f_kernel<3><<<b, 256, 0, st>>>(a);
+    if (a.dim == 2) PG_CUDA_TRY(launch_chained(st, a.chained != 0, adjoint_prep_f_kernel<2>, b, 256, a));
+    else PG_CUDA_TRY(launch_chained(st, a.chained != 0, adjoint_prep_f_kernel<3>, b, 256, a));
   } else {
-    if (a.dim == 2) adjoint_prep_kernel<2><<<b, 256, 0, st>>>(a);
-    else adjoint_prep_kernel<3><<<b, 256, 0, st>>>(a);
+    if (a.dim == 2) PG_CUDA_TRY(launch_chained(st, a.chained != 0, adjoint_prep_kernel<2>, b, 256, a));
+    else PG_CUDA_TRY(launch_chained(st, a.chained != 0, adjoint_prep_kernel<3>, b, 256, a));
   }
   PG_CUDA_TRY(cudaGetLastError());
   return PG_OK;
@@ -449,7 +451,7 @@ int launch_adjoint_pass(cudaStream_t st, const SphArgs& a, int stage, int grid, 
   if (a.n == 0) return PG_OK;
   const uint32_t ntiles = (a.n + kSphThreads - 1) / kSphThreads;
   if (grid <= 0 || (uint32_t)grid > ntiles) grid = (int)ntiles;
-  adjoint_kernel(a.dim, stage, fp32)<<<grid, kSphThreads, 0, st>>>(a);
+  PG_CUDA_TRY(launch_chained(st, a.chained != 0, adjoint_kernel(a.dim, stage, fp32), (unsigned)grid, kSphThreads, a));
   PG_CUDA_TRY(cudaGetLastError());
   return PG_OK;
 }
@@ -717,7 +719,9 @@ int pg_backward(pg_system* s, const double* dL_dx, double* dL_dalpha, double* dL
       a.sorted_cell = A->seg_cell[b].as<uint32_t>() + (size_t)t * n;
       a.sorted_id = A->seg_id[b].as<uint32_t>() + (size_t)t * n;
       a.cell_start = A->seg_start[b].as<uint32_t>() + (size_t)t * ncp1;
+      a.chained = t < steps - 1;  // the segment's first launch follows an event
       PG_TRY(pg::launch_adjoint_prep(st, a, fp32));
+      a.chained = 1;
       if (fp32) {
         PG_TRY(pg::launch_sph_list_pf(st, a, 0, pg::kSphThreads));
         PG_TRY(pg::launch_adjoint_pass(st, a, pg::SPH_MOM, A->pass_grid[pg::SPH_MOM], fp32));

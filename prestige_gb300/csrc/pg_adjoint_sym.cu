@@ -291,6 +291,7 @@ __device__ __forceinline__ void add_stored_sums(const SphArgs& a, const Packs& P
 // occupancy).
 template <int LANES>
 __global__ void __launch_bounds__(kSphMaxThreads) adj_mirror_kernel(SphArgs a) {
+  chain_begin();
   Slot<LANES> s;
   if (!slot_of(a, s)) return;
   const Planes E = planes_of(a);
@@ -310,6 +311,7 @@ __global__ void __launch_bounds__(kSphMaxThreads) adj_mirror_kernel(SphArgs a) {
 
 template <int DIM, int LANES>
 __global__ void __launch_bounds__(kSphMaxThreads) adj_a1_kernel(SphArgs a) {
+  chain_begin();
   Slot<LANES> s;
   if (!slot_of(a, s)) return;
   const SphK& K = a.sys[0];
@@ -350,6 +352,7 @@ __global__ void __launch_bounds__(kSphMaxThreads) adj_a1_kernel(SphArgs a) {
 
 template <int DIM, int LANES>
 __global__ void __launch_bounds__(kSphMaxThreads) adj_a2_kernel(SphArgs a) {
+  chain_begin();
   Slot<LANES> s;
   if (!slot_of(a, s)) return;
   const SphK& K = a.sys[0];
@@ -419,6 +422,7 @@ __device__ __forceinline__ void cont_full(const SphK& K, const Packs& P, uint32_
 
 template <int DIM, int LANES>
 __global__ void __launch_bounds__(kSphMaxThreads) adj_c1_kernel(SphArgs a) {
+  chain_begin();
   Slot<LANES> s;
   if (!slot_of(a, s)) return;
   const Packs P(a);
@@ -476,6 +480,7 @@ __global__ void __launch_bounds__(kSphMaxThreads) adj_c1_kernel(SphArgs a) {
 
 template <int DIM, int LANES>
 __global__ void __launch_bounds__(kSphMaxThreads) adj_c2_kernel(SphArgs a) {
+  chain_begin();
   Slot<LANES> s;
   if (!slot_of(a, s)) return;
   const SphK& K = a.sys[0];
@@ -540,8 +545,7 @@ int launch_adjoint_sym(cudaStream_t st, const SphArgs& a, int part) {
   }
   if (a.n == 0) return PG_OK;
   const unsigned blocks = (unsigned)(((size_t)a.n * kAdjLanes + kAdjBlock - 1) / kAdjBlock);
-  kern<<<blocks, kAdjBlock, 0, st>>>(a);
-  PG_CUDA_TRY(cudaGetLastError());
+  PG_CUDA_TRY(launch_chained(st, a.chained != 0, kern, blocks, kAdjBlock, a));
   return PG_OK;
 }
 

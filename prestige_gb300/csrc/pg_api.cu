@@ -190,6 +190,7 @@ SphArgs sph_args(pg_system* s, int integrate, bool rates) {
   a.posmin = s->posmin.as<unsigned long long>();
   a.k_begin = 0;
   a.k_end = (uint32_t)s->n;
+  a.chained = 0;
   return a;
 }
 
@@ -258,14 +259,18 @@ long long neighbor_launches(const pg_system* s) { return s->nw.chunks > 1 ? 4 : 
 // pair-once against 92 two-sided, 4,000 particles in 3D 162 against 266.  Both give the oracle's bits.
 bool pair_once(const pg_system* s) { return s->arith == ARITH_F64_EXACT; }
 
+bool overlapped(const pg_system* s) { return s->ov_split > 0 && s->ov_split < s->n; }
+
 int enqueue_sph_front(pg_system* s, cudaEvent_t* ev) {
   if (ev) PG_CUDA_TRY(cudaEventRecord(ev[0], s->stream));
   PG_TRY(enqueue_neighbors(s));
   if (ev) PG_CUDA_TRY(cudaEventRecord(ev[1], s->stream));
   SphArgs a = sph_args(s, 1, false);
+  a.chained = !ev;
   PG_TRY(launch_sph_gather(s->stream, a, s->arith));
   if (ev) PG_CUDA_TRY(cudaEventRecord(ev[2], s->stream));
-  if (s->arith == ARITH_F64_EXACT && s->ov_split > 0 && s->ov_split < s->n) {
+  if (overlapped(s)) a.chained = 0;  // events between the launches
+  if (s->arith == ARITH_F64_EXACT && overlapped(s)) {
     // each pair once (pg_sph_sym.cu); the lists of [split, n) on the auxiliary stream beside the
     // lists of [0, split), then the pair values of the slots whose partners all lie below split,
     // the rest once every list is built
@@ -298,7 +303,7 @@ int enqueue_sph_front(pg_system* s, cudaEvent_t* ev) {
     s->launches += neighbor_launches(s) + 4;
     return PG_OK;
   }
-  if (s->ov_split > 0 && s->ov_split < s->n) {
+  if (overlapped(s)) {
     // lists of [0, split) first; then the continuity pass over them runs beside the lists of
     // [split, n) on the auxiliary stream, which goes on with the continuity pass over
     // [split, n) (neither continuity launch reads the packed rho' the other writes); the
@@ -330,11 +335,13 @@ int enqueue_sph_front(pg_system* s, cudaEvent_t* ev) {
 }
 
 // The momentum part of a step: the momentum pass with the packed rho' (velocity and position
-// update).  ev (optional): event 5 of a step (end).
-int enqueue_sph_momentum(pg_system* s, cudaEvent_t* ev) {
+// update).  chained: directly after the continuity part.  ev (optional): event 5 of a step (end).
+int enqueue_sph_momentum(pg_system* s, bool chained, cudaEvent_t* ev) {
   SphArgs a = sph_args(s, 1, false);
+  a.chained = chained && !ev && !overlapped(s);
   if (pair_once(s)) {
     PG_TRY(launch_sph_sym(s->stream, a, 2, mom_block(s)));
+    a.chained = !ev;
     PG_TRY(launch_sph_sym(s->stream, a, 3, mom_block(s)));
     s->launches += 2;
     if (ev) PG_CUDA_TRY(cudaEventRecord(ev[5], s->stream));
@@ -351,12 +358,13 @@ int enqueue_sph_momentum(pg_system* s, cudaEvent_t* ev) {
 int enqueue_sph_step(pg_system* s, bool rates, int integrate, cudaEvent_t* ev) {
   if (!rates) {
     PG_TRY(enqueue_sph_front(s, ev));
-    return enqueue_sph_momentum(s, ev);
+    return enqueue_sph_momentum(s, true, ev);
   }
   if (ev) PG_CUDA_TRY(cudaEventRecord(ev[0], s->stream));
   PG_TRY(enqueue_neighbors(s));
   if (ev) PG_CUDA_TRY(cudaEventRecord(ev[1], s->stream));
   SphArgs a = sph_args(s, integrate, rates);
+  a.chained = !ev;
   PG_TRY(launch_sph_gather(s->stream, a, s->arith));
   if (ev) PG_CUDA_TRY(cudaEventRecord(ev[2], s->stream));
   PG_TRY(launch_sph_list(s->stream, a, s->arith, s->list_grid, s->block));
@@ -402,8 +410,8 @@ int enqueue_dem_step(pg_system* s, cudaEvent_t* ev) {
   PG_TRY(enqueue_neighbors(s));
   if (ev) PG_CUDA_TRY(cudaEventRecord(ev[1], s->stream));
   DemArgs a = dem_args(s);
+  a.chained = !ev;
   PG_TRY(launch_dem_gather(s->stream, a));
-  PG_CUDA_TRY(cudaMemsetAsync(s->contacts.p, 0, sizeof(unsigned long long), s->stream));
   if (ev) PG_CUDA_TRY(cudaEventRecord(ev[2], s->stream));
   if (ev) PG_CUDA_TRY(cudaEventRecord(ev[3], s->stream));
   PG_TRY(launch_dem_pass(s->stream, a));
@@ -1412,7 +1420,7 @@ int pg_step_stage(pg_system* s, int stage) {
   SphArgs a = pg::sph_args(s, 1, false);
   PG_TRY(pg::launch_sph_repack_rho(s->stream, a, s->arith));
   s->launches += 1;
-  PG_TRY(pg::enqueue_sph_momentum(s, nullptr));
+  PG_TRY(pg::enqueue_sph_momentum(s, false, nullptr));
   return pg::sync_and_check(s);
 }
 

@@ -164,7 +164,9 @@ __device__ __forceinline__ void history_lookup(const uint32_t* hp, const double*
 }
 
 __global__ void dem_gather_kernel(DemArgs a) {
+  chain_begin();
   const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s == 0) *a.contacts = 0;  // the contact pass that follows adds to it
   if (s >= a.n) return;
   uint32_t id;
   const uint32_t k = ordered_slot(a.order, s, id);
@@ -220,6 +222,7 @@ __global__ void __launch_bounds__(kDemThreads) dem_pass_kernel(DemArgs a) {
   __shared__ uint32_t s_buf[kDemBuf][kDemThreads];   // [q][thread]: slot of a partner, or kWallId + face
   __shared__ uint16_t s_owner[kDemWarps][32 * kDemBuf];  // warp contact c -> (owner lane << 8) | q
   __shared__ DemTerm s_term[kDemWarps][32];
+  chain_begin();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t k = blockIdx.x * blockDim.x + tid;
   const bool live = k < a.n;
@@ -440,14 +443,14 @@ __global__ void __launch_bounds__(kDemThreads) dem_pass_kernel(DemArgs a) {
 
 int launch_dem_gather(cudaStream_t st, const DemArgs& a) {
   if (a.n == 0) return PG_OK;
-  dem_gather_kernel<<<(a.n + 255) / 256, 256, 0, st>>>(a);
+  PG_CUDA_TRY(launch_chained(st, a.chained != 0, dem_gather_kernel, (a.n + 255) / 256, 256, a));
   PG_CUDA_TRY(cudaGetLastError());
   return PG_OK;
 }
 
 int launch_dem_pass(cudaStream_t st, const DemArgs& a) {
   if (a.n == 0) return PG_OK;
-  dem_pass_kernel<<<(a.n + kDemThreads - 1) / kDemThreads, kDemThreads, 0, st>>>(a);
+  PG_CUDA_TRY(launch_chained(st, a.chained != 0, dem_pass_kernel, (a.n + kDemThreads - 1) / kDemThreads, kDemThreads, a));
   PG_CUDA_TRY(cudaGetLastError());
   return PG_OK;
 }

@@ -88,6 +88,7 @@ struct SphArgs {
                              // of the block size; the whole system is [0, n))
   unsigned* err;             // device error word (ERR_* bits)
   int integrate;
+  int chained;               // launched directly after another kernel of the step (launch_chained)
 };
 
 int launch_sph_gather(cudaStream_t st, const SphArgs& a, int arith);
@@ -188,8 +189,9 @@ struct DemArgs {
   const double* hxi_old;
   uint32_t* hpid_new;
   double* hxi_new;
-  unsigned long long* contacts;
+  unsigned long long* contacts;  // zeroed by the gather, counted by the pass
   unsigned* err;
+  int chained;               // launched directly after another kernel of the step (launch_chained)
 };
 
 int launch_dem_gather(cudaStream_t st, const DemArgs& a);

@@ -174,6 +174,7 @@ __global__ void hash_kernel(const GridK* __restrict__ grid, const uint32_t* __re
                             uint32_t* __restrict__ rank, uint32_t* __restrict__ count,
                             uint32_t* __restrict__ big,
                             unsigned long long* __restrict__ posmin) {
+  chain_begin();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   unsigned long long m[3] = {~0ull, ~0ull, ~0ull};
   if (i < n) {
@@ -221,6 +222,7 @@ __global__ void hash_kernel(const GridK* __restrict__ grid, const uint32_t* __re
 
 template <class R, int DIM>
 __global__ void sorted_positions_kernel(NbrArgs a, const R* __restrict__ pos, typename NbrV4<R>::T* spos) {
+  chain_begin();
   const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= a.n) return;
   uint32_t id;
@@ -406,11 +408,11 @@ int launch_sorted_positions(cudaStream_t st, const NbrArgs& a, const void* pos, 
   if (a.n == 0) return PG_OK;
   const unsigned b = blocks_for(a.n, 256);
   if (a.f64) {
-    if (a.dim == 2) sorted_positions_kernel<double, 2><<<b, 256, 0, st>>>(a, (const double*)pos, (double4_32a*)spos);
-    else sorted_positions_kernel<double, 3><<<b, 256, 0, st>>>(a, (const double*)pos, (double4_32a*)spos);
+    if (a.dim == 2) PG_CUDA_TRY(launch_chained(st, true, sorted_positions_kernel<double, 2>, b, 256, a, (const double*)pos, (double4_32a*)spos));
+    else PG_CUDA_TRY(launch_chained(st, true, sorted_positions_kernel<double, 3>, b, 256, a, (const double*)pos, (double4_32a*)spos));
   } else {
-    if (a.dim == 2) sorted_positions_kernel<float, 2><<<b, 256, 0, st>>>(a, (const float*)pos, (float4*)spos);
-    else sorted_positions_kernel<float, 3><<<b, 256, 0, st>>>(a, (const float*)pos, (float4*)spos);
+    if (a.dim == 2) PG_CUDA_TRY(launch_chained(st, true, sorted_positions_kernel<float, 2>, b, 256, a, (const float*)pos, (float4*)spos));
+    else PG_CUDA_TRY(launch_chained(st, true, sorted_positions_kernel<float, 3>, b, 256, a, (const float*)pos, (float4*)spos));
   }
   PG_CUDA_TRY(cudaGetLastError());
   return PG_OK;

@@ -233,6 +233,7 @@ static_assert(kCellScanItems == 8, "two 16-byte loads per thread");
 
 __global__ void __launch_bounds__(kCellScanThreads) cell_reduce_kernel(const uint32_t* __restrict__ count,
                                                                        uint32_t* __restrict__ chunk_total) {
+  chain_begin();
   const uint4* cp = (const uint4*)(count + (size_t)blockIdx.x * kScanChunk) + 2 * threadIdx.x;
   const uint4 a = cp[0], b = cp[1];
   uint32_t total;
@@ -246,6 +247,7 @@ __global__ void __launch_bounds__(kCellScanThreads) cell_scan_kernel(uint32_t* _
                                                                      unsigned long long* minacc,
                                                                      unsigned long long* minout, uint32_t nmin) {
   __shared__ uint32_t base;
+  chain_begin();
   const uint32_t tid = threadIdx.x;
   // cells of the chunks before this one
   uint32_t before = 0;
@@ -335,6 +337,7 @@ __global__ void __launch_bounds__(kSortThreads) cell_scatter_kernel(const uint32
                                                                     uint32_t* rank,
                                                                     const uint32_t* __restrict__ start, uint32_t n,
                                                                     uint32_t* unsorted, uint32_t* big, int id_bits) {
+  chain_begin();
   const uint32_t i = blockIdx.x * kSortThreads + threadIdx.x;
   if (i < n) unsorted[start[key[i]] + rank[i]] = i;
   const uint32_t nbig = ((volatile uint32_t*)big)[0];
@@ -420,14 +423,13 @@ NbrOrder nbr_order(const NbrWork& w) {
 
 int launch_sort(cudaStream_t st, NbrWork& w, unsigned long long* minacc, unsigned long long* minout, uint32_t nmin) {
   if (w.chunks > 1)
-    cell_reduce_kernel<<<w.chunks, kCellScanThreads, 0, st>>>(w.count, w.chunk_total);
-  cell_scan_kernel<<<w.chunks, kCellScanThreads, 0, st>>>(w.count, w.chunk_total,
-                                                          w.cell_start, minacc, minout,
-                                                          minacc ? nmin : 0u);
+    PG_CUDA_TRY(launch_chained(st, w.n > 0, cell_reduce_kernel, w.chunks, kCellScanThreads, w.count, w.chunk_total));
+  PG_CUDA_TRY(launch_chained(st, w.n > 0 || w.chunks > 1, cell_scan_kernel, w.chunks, kCellScanThreads, w.count,
+                             w.chunk_total, w.cell_start, minacc, minout, minacc ? nmin : 0u));
   if (w.n)
-    cell_scatter_kernel<<<(unsigned)((w.n + kSortThreads - 1) / kSortThreads), kSortThreads, 0, st>>>(
-        w.key, w.rank, w.cell_start, (uint32_t)w.n,
-        w.unsorted, w.big, bits_needed(w.n - 1));
+    PG_CUDA_TRY(launch_chained(st, true, cell_scatter_kernel, (unsigned)((w.n + kSortThreads - 1) / kSortThreads),
+                               kSortThreads, w.key, w.rank, w.cell_start, (uint32_t)w.n, w.unsorted, w.big,
+                               bits_needed(w.n - 1)));
   PG_CUDA_TRY(cudaGetLastError());
   return PG_OK;
 }

@@ -56,6 +56,7 @@ template <class Ops, int DIM>
 __global__ void sph_gather_real(SphArgs a) {
   typedef typename Ops::R R;
   typedef typename V4<R>::T R4;
+  chain_begin();
   const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= a.n) return;
   uint32_t id;
@@ -143,6 +144,7 @@ struct __align__(64) DfRecord {
 // the other systems of a batch; the f64 array for the exact test keeps the unshifted positions.
 template <int DIM>
 __global__ void sph_gather_df(SphArgs a) {
+  chain_begin();
   const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= a.n) return;
   uint32_t id;
@@ -606,7 +608,7 @@ int launch_table(cudaStream_t st, const SphArgs& a, PassKernel kern, int grid, i
   const uint32_t spb = (uint32_t)(block / lanes);
   const uint32_t ntiles = (a.k_end + spb - 1) / spb - a.k_begin / spb;
   if (grid <= 0 || (uint32_t)grid > ntiles) grid = (int)ntiles;
-  kern<<<grid, block, 0, st>>>(a);
+  PG_CUDA_TRY(launch_chained(st, a.chained != 0, kern, (unsigned)grid, (unsigned)block, a));
   PG_CUDA_TRY(cudaGetLastError());
   return PG_OK;
 }
@@ -635,20 +637,20 @@ int launch_sph_gather(cudaStream_t st, const SphArgs& a, int arith) {
   const int dim = a.dim;
   switch (arith) {
     case ARITH_F64_EXACT:
-      if (dim == 2) sph_gather_real<OpsD, 2><<<blocks, 256, 0, st>>>(a);
-      else sph_gather_real<OpsD, 3><<<blocks, 256, 0, st>>>(a);
+      if (dim == 2) PG_CUDA_TRY(launch_chained(st, a.chained != 0, sph_gather_real<OpsD, 2>, blocks, 256, a));
+      else PG_CUDA_TRY(launch_chained(st, a.chained != 0, sph_gather_real<OpsD, 3>, blocks, 256, a));
       break;
     case ARITH_F64_DF:  // a.posmin was filled by the step's hash kernel
-      if (dim == 2) sph_gather_df<2><<<blocks, 256, 0, st>>>(a);
-      else sph_gather_df<3><<<blocks, 256, 0, st>>>(a);
+      if (dim == 2) PG_CUDA_TRY(launch_chained(st, a.chained != 0, sph_gather_df<2>, blocks, 256, a));
+      else PG_CUDA_TRY(launch_chained(st, a.chained != 0, sph_gather_df<3>, blocks, 256, a));
       break;
     case ARITH_F32_EXACT:
-      if (dim == 2) sph_gather_real<OpsF, 2><<<blocks, 256, 0, st>>>(a);
-      else sph_gather_real<OpsF, 3><<<blocks, 256, 0, st>>>(a);
+      if (dim == 2) PG_CUDA_TRY(launch_chained(st, a.chained != 0, sph_gather_real<OpsF, 2>, blocks, 256, a));
+      else PG_CUDA_TRY(launch_chained(st, a.chained != 0, sph_gather_real<OpsF, 3>, blocks, 256, a));
       break;
     case ARITH_F32_FAST:
-      if (dim == 2) sph_gather_real<OpsFF, 2><<<blocks, 256, 0, st>>>(a);
-      else sph_gather_real<OpsFF, 3><<<blocks, 256, 0, st>>>(a);
+      if (dim == 2) PG_CUDA_TRY(launch_chained(st, a.chained != 0, sph_gather_real<OpsFF, 2>, blocks, 256, a));
+      else PG_CUDA_TRY(launch_chained(st, a.chained != 0, sph_gather_real<OpsFF, 3>, blocks, 256, a));
       break;
     default:
       set_error("unknown arithmetic mode %d", arith);

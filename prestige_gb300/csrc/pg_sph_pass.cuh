@@ -169,6 +169,7 @@ __device__ __forceinline__ size_t list_base(uint32_t k, uint32_t cap) {
 
 template <int DIM, bool EXACT_PF, int XD, int B>
 __global__ void __launch_bounds__(kSphMaxThreads) sph_list_kernel(SphArgs a) {
+  chain_begin();
   const int tid = threadIdx.x;
   const float* __restrict__ PF = a.pf;
   const double4_32a* __restrict__ X = (const double4_32a*)a.s[XD < 0 ? 0 : XD];
@@ -368,6 +369,7 @@ struct PrefetchPolicy<P, decltype((void)P::kPrefetch)> {
 template <class Pairs, int DIM, bool EXACT_PF, int LANES = 1>
 __global__ void __launch_bounds__(kSphMaxThreads) sph_list_pass_kernel(SphArgs a) {
   static_assert(LANES == 1 || LANES == 2 || LANES == 4, "1, 2 or 4 lanes per slot");
+  chain_begin();
   const int tid = threadIdx.x;
   const uint32_t cap = a.cap;
   const uint32_t spb = blockDim.x / LANES;  // slots per block

@@ -194,6 +194,7 @@ __device__ __forceinline__ bool slot_of(const SphArgs& a, Slot& s) {
 // last stored entry decides) and the second launch, after all lists, the others.
 template <int DIM>
 __global__ void __launch_bounds__(kSphMaxThreads) sym_c1_kernel(SphArgs a, uint32_t split, int second) {
+  chain_begin();
   Slot s;
   if (!slot_of<kPairLanes>(a, s)) return;
   const uint32_t* __restrict__ my = a.nlist + list_base(s.k, a.cap);
@@ -249,6 +250,7 @@ __global__ void __launch_bounds__(kSphMaxThreads) sym_c1_kernel(SphArgs a, uint3
 
 template <int DIM>
 __global__ void __launch_bounds__(kSphMaxThreads) sym_c2_kernel(SphArgs a) {
+  chain_begin();
   Slot s;
   if (!slot_of(a, s)) return;
   const SphK& K = a.sys[sys_of_slot(a, s.id)];
@@ -297,6 +299,7 @@ __global__ void __launch_bounds__(kSphMaxThreads) sym_c2_kernel(SphArgs a) {
 
 template <int DIM>
 __global__ void __launch_bounds__(kSphMaxThreads) sym_m1_kernel(SphArgs a) {
+  chain_begin();
   Slot s;
   if (!slot_of<kPairLanes>(a, s)) return;
   const SphK& K = a.sys[sys_of_slot(a, s.id)];
@@ -332,6 +335,7 @@ __global__ void __launch_bounds__(kSphMaxThreads) sym_m1_kernel(SphArgs a) {
 
 template <int DIM>
 __global__ void __launch_bounds__(kSphMaxThreads) sym_m2_kernel(SphArgs a) {
+  chain_begin();
   Slot s;
   if (!slot_of(a, s)) return;
   const SphK& K = a.sys[sys_of_slot(a, s.id)];
@@ -416,12 +420,11 @@ int launch_sph_sym(cudaStream_t st, const SphArgs& a, int part, int block, uint3
   const int lanes = part == 0 || part == 2 ? kPairLanes : 1;
   const unsigned blocks = (unsigned)(((size_t)(a.k_end - a.k_begin) * lanes + block - 1) / block);
   if (part == 0) {
-    if (a.dim == 2) sym_c1_kernel<2><<<blocks, block, 0, st>>>(a, split, second);
-    else sym_c1_kernel<3><<<blocks, block, 0, st>>>(a, split, second);
+    PG_CUDA_TRY(launch_chained(st, a.chained != 0, a.dim == 2 ? sym_c1_kernel<2> : sym_c1_kernel<3>, blocks,
+                               (unsigned)block, a, split, second));
   } else {
-    kern<<<blocks, block, 0, st>>>(a);
+    PG_CUDA_TRY(launch_chained(st, a.chained != 0, kern, blocks, (unsigned)block, a));
   }
-  PG_CUDA_TRY(cudaGetLastError());
   return PG_OK;
 }
 

@@ -110,7 +110,7 @@ SphArgs sph_args(pg_system* s, int integrate, bool rates);
 int enqueue_neighbors(pg_system* s);
 int enqueue_sph_step(pg_system* s, bool rates, int integrate, cudaEvent_t* ev);
 int enqueue_sph_front(pg_system* s, cudaEvent_t* ev);
-int enqueue_sph_momentum(pg_system* s, cudaEvent_t* ev);
+int enqueue_sph_momentum(pg_system* s, bool chained, cudaEvent_t* ev);
 long long neighbor_launches(const pg_system* s);
 int sync_and_check(pg_system* s);
 int choose_pass_grid(pg_system* s);
