@@ -203,23 +203,9 @@ __device__ __forceinline__ void add_own(Sums& s, const MomTerms<DIM>& m, double 
 template <int DIM, class OnPair>
 __device__ __forceinline__ void resume_walk(const SphArgs& a, const SphK& K, const Packs& P, uint32_t k,
                                             const double4_32a& xk, OnPair&& on_pair) {
-  const float* __restrict__ PF = a.pf;
-  const SphK* Kp;
-  const Target T = target_of(a, k, &Kp, a.reach);
-  const GridK& g = K.g;
-  const int R = a.reach, RZ = DIM == 3 ? R : 0, side = 2 * R + 1, nrows = side * (2 * RZ + 1);
-  const float4 pi = pf_at<DIM>(PF, k);
-  const float thr = prefilter_threshold<false>(K, pi);
-  const int row0 = (int)a.nresume[2 * (size_t)k];
-  const uint32_t t0 = a.nresume[2 * (size_t)k + 1];
-  for (int row = row0; row < nrows; ++row) {
-    const int z = T.cz + row / side - RZ, y = T.cy + row % side - R;
-    if (z < 0 || z >= g.nz || y < 0 || y >= g.ny) continue;
-    const uint32_t rb = g.cell_base + ((uint32_t)z * g.ny + (uint32_t)y) * g.nx;
-    const uint32_t e = a.cell_start[rb + T.x1 + 1];
-    for (uint32_t t = row == row0 ? t0 : a.cell_start[rb + T.x0]; t < e; ++t)
-      if (prefilter_hit<DIM, false>(pi, pf_at<DIM>(PF, t), thr) && is_neighbor<DIM>(K.d, xk, P.X[t])) on_pair(t);
-  }
+  continue_walk<DIM, false>(a, k, [&](uint32_t t) {
+    if (is_neighbor<DIM>(K.d, xk, P.X[t])) on_pair(t);
+  });
 }
 
 // LANES threads share a slot: thread `sub` takes every LANES-th entry of its loops and the

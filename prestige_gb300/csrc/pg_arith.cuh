@@ -42,6 +42,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "pg_f32x2.cuh"
 #include "pg_softf64.cuh"
 
 namespace pg {
@@ -291,5 +292,76 @@ __device__ __forceinline__ dfacc dfacc_add(dfacc a, dfacc b) {
 }
 
 __device__ __forceinline__ double dfacc_to_double(dfacc a) { return __dadd_rn((double)a.hi, (double)a.lo); }
+
+// ---------------------------------------------------------------------------------------
+// The same operations on two double-words at once (packed f32x2 instructions): each half gives the
+// bits of the scalar operation above (products that an addition takes are rounded on their own).
+// ---------------------------------------------------------------------------------------
+struct df2 {
+  f2 hi, lo;
+};
+
+__device__ __forceinline__ df2 df2_make(f2 h, f2 l) {
+  df2 r;
+  r.hi = h;
+  r.lo = l;
+  return r;
+}
+__device__ __forceinline__ df2 df2_dup(df a) { return df2_make(f2_dup(a.hi), f2_dup(a.lo)); }
+__device__ __forceinline__ df2 df2_pair(df a, df b) { return df2_make(f2_make(a.hi, b.hi), f2_make(a.lo, b.lo)); }
+__device__ __forceinline__ df df2_first(df2 v) { return df_make(f2_split(v.hi).x, f2_split(v.lo).x); }
+__device__ __forceinline__ df df2_second(df2 v) { return df_make(f2_split(v.hi).y, f2_split(v.lo).y); }
+__device__ __forceinline__ df2 df2_neg(df2 a) { return df2_make(f2_neg(a.hi), f2_neg(a.lo)); }
+
+__device__ __forceinline__ df2 two_sum2(f2 a, f2 b) {
+  const f2 s = f2_add(a, b);
+  const f2 bb = f2_sub(s, a);
+  return df2_make(s, f2_add(f2_sub(a, f2_sub(s, bb)), f2_sub(b, bb)));
+}
+__device__ __forceinline__ df2 fast_two_sum2(f2 a, f2 b) {
+  const f2 s = f2_add(a, b);
+  return df2_make(s, f2_sub(b, f2_sub(s, a)));
+}
+__device__ __forceinline__ df2 df2_sub_close(df2 x, df2 y) {
+  return fast_two_sum2(f2_sub(x.hi, y.hi), f2_sub(x.lo, y.lo));
+}
+__device__ __forceinline__ df2 df2_add_raw(df2 x, df2 y) {
+  const df2 s = two_sum2(x.hi, y.hi);
+  return df2_make(s.hi, f2_add(s.lo, f2_add(x.lo, y.lo)));
+}
+__device__ __forceinline__ df2 df2_sub(df2 x, df2 y) {
+  const df2 s = two_sum2(x.hi, f2_neg(y.hi));
+  return fast_two_sum2(s.hi, f2_add(s.lo, f2_sub(x.lo, y.lo)));
+}
+__device__ __forceinline__ df2 df2_mul(df2 x, df2 y) {
+  const f2 p = f2_mul_rn(x.hi, y.hi);
+  const f2 e = f2_fma(x.hi, y.hi, f2_neg(p));
+  const f2 t = f2_fma(x.lo, y.hi, f2_fma(x.hi, y.lo, f2_mul(x.lo, y.lo)));
+  return fast_two_sum2(p, f2_add(e, t));
+}
+__device__ __forceinline__ df2 df2_mul_f(df2 x, f2 y) {
+  const f2 p = f2_mul_rn(x.hi, y);
+  return fast_two_sum2(p, f2_fma(x.lo, y, f2_fma(x.hi, y, f2_neg(p))));
+}
+__device__ __forceinline__ df2 df2_div(df2 x, df2 y) {
+  const float2 yh = f2_split(y.hi);
+  const f2 t = f2_make(rcp_approx(yh.x), rcp_approx(yh.y));
+  const f2 q1 = f2_mul_rn(x.hi, t);
+  const df2 r = df2_sub(x, df2_mul_f(y, q1));
+  return fast_two_sum2(q1, f2_mul_rn(r.hi, t));
+}
+
+// a += first x y, then a += second x y: the products packed, the sums in order, so the bits are those of two
+// dfacc_add_prod.
+__device__ __forceinline__ void dfacc_add_prod2(dfacc& a, df2 x, df2 y) {
+  const f2 p = f2_mul_rn(x.hi, y.hi);
+  const f2 e = f2_fma(x.hi, y.hi, f2_neg(p));
+  const f2 pl = f2_fma(x.hi, y.lo, f2_fma(x.lo, y.hi, e));
+  const float2 ps = f2_split(p), ls = f2_split(pl);
+  const df s = two_sum(a.hi, ps.x);
+  const df t = two_sum(s.hi, ps.y);
+  a.hi = t.hi;
+  a.lo = (a.lo + (s.lo + ls.x)) + (t.lo + ls.y);
+}
 
 }  // namespace pg

@@ -11,36 +11,9 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "pg_f32x2.cuh"
+
 namespace pg {
-
-typedef unsigned long long f2;  // two floats: .lo is the low word
-
-__device__ __forceinline__ f2 f2_make(float lo, float hi) {
-  f2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ f2 f2_dup(float v) { return f2_make(v, v); }
-__device__ __forceinline__ float2 f2_split(f2 v) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r;
-}
-__device__ __forceinline__ f2 f2_add(f2 a, f2 b) {
-  f2 r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ f2 f2_mul(f2 a, f2 b) {
-  f2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) {
-  f2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
 
 // min(m, |a|, |b|); NaNs are ignored.
 __device__ __forceinline__ float min3_abs(float m, float a, float b) {
@@ -147,11 +120,11 @@ __device__ __forceinline__ unsigned screen_batch(const Batch<DIM, B>& C, const S
   for (int i = 0; i < B / 2; ++i) {
     const int c = i / 2;
     const f2 dx = f2_add(i & 1 ? C.v[c][0].y : C.v[c][0].x, S.nx), dy = f2_add(i & 1 ? C.v[c][1].y : C.v[c][1].x, S.ny);
-    f2 r2 = f2_mul(dx, dx);
-    r2 = CONTRACT ? f2_fma(dy, dy, r2) : f2_add(r2, f2_mul(dy, dy));
+    f2 r2 = CONTRACT ? f2_mul(dx, dx) : f2_mul_rn(dx, dx);
+    r2 = CONTRACT ? f2_fma(dy, dy, r2) : f2_add(r2, f2_mul_rn(dy, dy));
     if (DIM == 3) {
       const f2 dz = f2_add(i & 1 ? C.v[c][DIM - 1].y : C.v[c][DIM - 1].x, S.nz);
-      r2 = CONTRACT ? f2_fma(dz, dz, r2) : f2_add(r2, f2_mul(dz, dz));
+      r2 = CONTRACT ? f2_fma(dz, dz, r2) : f2_add(r2, f2_mul_rn(dz, dz));
     }
     const f2 s = RATIO ? f2_fma(r2, S.a, S.b) : f2_add(r2, S.b);
     const float2 sv = f2_split(s), qv = f2_split(f2_mul(r2, s));

@@ -83,9 +83,10 @@ __global__ void sph_gather_real(SphArgs a) {
 
 // Packs of the f64 fast (double-word) mode:
 //   pf x.hi, y.hi, z.hi (the list kernel's FP32 positions)
-//   s1 DfRecord {x,y,z,m}.hi, {x,y,z,m}.lo, {vx,vy,vz,0}.hi, {vx,vy,vz,0}.lo (the pair passes)
+//   s0 DfHalf {x,y,z,m}.hi, {x,y,z,m}.lo (momentum pass)
+//   s1 DfRecord the same and {vx,vy,vz,0}.hi, {vx,vy,vz,0}.lo (continuity pass, rates)
 //   s4 {rho.hi, rho.lo, P.hi, P.lo}   s5 double {x,y,z} for the exact neighbour test near 2h.
-// Positions in pf and s1 are shifted (see sph_gather_df).
+// Positions in pf, s0 and s1 are shifted (see sph_gather_df).
 
 // p / rho^2 of the Tait law in double-word arithmetic on the FP32 pipe (relative error about
 // 1e-12: (rho/rho0)^gamma - 1 loses the digits its cancellation takes).
@@ -129,13 +130,20 @@ __global__ void sph_repack_rho_df(SphArgs a) {
   ((float4*)a.s[4])[k] = df_pack_rho(K.w, K.gamma, ((const double*)a.rho)[id]);
 }
 
-// The pair passes' per-slot record in the double-word mode: positions and mass (hi, lo) and
-// velocities (hi, lo), 64 bytes, so the four loads of a neighbour touch two sectors of one line.
+// The pair passes' per-slot records in the double-word mode.  The continuity pass reads positions, mass
+// and velocities (hi, lo) from one 64-byte record, half a line; the momentum pass, which needs no
+// velocities, reads its own 32-byte copy of the first half: one sector, one load, and the
+// records of consecutive slots, which the lanes of a warp mostly read, side by side (4M
+// particles, momentum pass 2.14 ms from the 64-byte records, 1.97 from these; the gather pays 0.014
+// for the copy; the continuity pass gained nothing from two 32-byte arrays).
+struct __align__(32) DfHalf {
+  float4 hi, lo;
+};
 struct __align__(64) DfRecord {
-  float4 ah, al, bh, bl;
+  DfHalf x, v;  // {x, y, z, m}, {vx, vy, vz, 0}
 };
 
-// Packs of the double-word mode.  Positions in the record and in the FP32 array are shifted by
+// Packs of the double-word mode.  Positions in the records and in the FP32 array are shifted by
 // pos_pad - min (per system and dimension, pos_pad = 8h of the system), so every packed coordinate
 // is at least 8h: the hi parts of two particles closer than 2h are then within a factor 2 of each
 // other and the pair passes take differences with df_sub_close.  The shift is common to all
@@ -174,11 +182,15 @@ __global__ void sph_gather_df(SphArgs a) {
   df_split_fast(v[2], &bh.z, &bl.z);
   bh.w = bl.w = 0.f;
   pf_store<DIM>(a.pf, k, ah.x, ah.y, ah.z);
+  DfHalf xm, vv;
+  xm.hi = ah;
+  xm.lo = al;
+  vv.hi = bh;
+  vv.lo = bl;
   DfRecord rec;
-  rec.ah = ah;
-  rec.al = al;
-  rec.bh = bh;
-  rec.bl = bl;
+  rec.x = xm;
+  rec.v = vv;
+  ((DfHalf*)a.s[0])[k] = xm;
   ((DfRecord*)a.s[1])[k] = rec;
   ((float4*)a.s[4])[k] = df_pack_rho(K.w, K.gamma, rho);
   ((double4_32a*)a.s[5])[k] = make_double4_32a(x[0], x[1], x[2], 0.0);
@@ -320,6 +332,7 @@ template <int DIM, int STAGE>
 struct DfPairs {
   static constexpr bool kCont = STAGE != SPH_MOM;
   static constexpr bool kMom = STAGE != SPH_CONT;
+  const DfHalf* Xm;     // momentum pass of a step
   const DfRecord* Rec;
   const float4* RP;
   const double4_32a* Xd;
@@ -333,14 +346,15 @@ struct DfPairs {
   static constexpr bool kCacheF = STAGE == SPH_CONT || STAGE == SPH_MOM;
 
   __device__ __forceinline__ void begin(const SphArgs& a, const SphK& K, uint32_t k) {
+    Xm = (const DfHalf*)a.s[0];
     Rec = (const DfRecord*)a.s[1];
     RP = (const float4*)a.s[4];
     Xd = (const double4_32a*)a.s[5];
     w = K.w;
     four_h2 = K.d.four_h2;
-    const float4 ah = Rec[k].ah, al = Rec[k].al, bh = Rec[k].bh, bl = Rec[k].bl;
+    const float4 ah = STAGE == SPH_MOM ? Xm[k].hi : Rec[k].x.hi, al = STAGE == SPH_MOM ? Xm[k].lo : Rec[k].x.lo;
     xi[0] = df_make(ah.x, al.x); xi[1] = df_make(ah.y, al.y); xi[2] = df_make(ah.z, al.z);
-    vi[0] = df_make(bh.x, bl.x); vi[1] = df_make(bh.y, bl.y); vi[2] = df_make(bh.z, bl.z);
+    if (STAGE != SPH_MOM) load_velocity(k);
     rhoi = Pi = df_make(0.f, 0.f);
     if (kMom) {
       const float4 rp = RP[k];
@@ -348,9 +362,14 @@ struct DfPairs {
       Pi = df_make(rp.z, rp.w);
     }
     kself = k;
-    fc = kCacheF && a.fcache ? (float4*)a.fcache + list_base(k, a.cap) : nullptr;
+    fc = kCacheF ? (float4*)a.fcache + list_base(k, a.cap) : nullptr;
     acc[0] = acc[1] = acc[2] = dfacc_zero();
     dr = dfacc_zero();
+  }
+
+  __device__ __forceinline__ void load_velocity(uint32_t k) {
+    const float4 bh = Rec[k].v.hi, bl = Rec[k].v.lo;
+    vi[0] = df_make(bh.x, bl.x); vi[1] = df_make(bh.y, bl.y); vi[2] = df_make(bh.z, bl.z);
   }
 
   // Geometry of pair (k, t): x_ij, r^2, F = (dW/dr)/r and w = v_ij . x_ij.  CHECK: false when t is
@@ -362,73 +381,59 @@ struct DfPairs {
     float4 ah, al, bh, bl, rp, fw;
   };
   static constexpr bool kPrefetch = true;
+  static constexpr bool kTwo = STAGE == SPH_MOM;  // two list entries at a time (pair_two)
 
-  __device__ __forceinline__ Pre fetch(uint32_t t, uint32_t q) const { return fetch_entry(t, q, STAGE == SPH_MOM && fc); }
+  __device__ __forceinline__ Pre fetch(uint32_t t, uint32_t q) const { return fetch_entry(t, q, STAGE == SPH_MOM); }
 
   // the momentum pass's cache entries are a DRAM stream like the lists (sph_list_pass_kernel)
   static constexpr bool kL2Entry = STAGE == SPH_MOM;
   __device__ __forceinline__ void prefetch_entry(uint32_t q) const {
-    if (fc) prefetch_l2(fc + (size_t)q * kListTile);
+    prefetch_l2(fc + (size_t)q * kListTile);
   }
 
   // cached: list entry q of a momentum pass that reads G = m_j F and u from the continuity pass
   __device__ __forceinline__ Pre fetch_entry(uint32_t t, uint32_t q, bool cached) const {
     Pre p;
-    p.ah = Rec[t].ah;
-    p.al = Rec[t].al;
     // the momentum pass takes w from the cache and needs no velocities of the neighbour
-    p.bh = cached ? make_float4(0.f, 0.f, 0.f, 0.f) : Rec[t].bh;
-    p.bl = cached ? make_float4(0.f, 0.f, 0.f, 0.f) : Rec[t].bl;
+    load_32b(cached ? &Xm[t].hi : &Rec[t].x.hi, p.ah, p.al);
+    p.bh = p.bl = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (!cached) load_32b(&Rec[t].v.hi, p.bh, p.bl);
     p.rp = kMom ? RP[t] : make_float4(0.f, 0.f, 0.f, 0.f);
     p.fw = cached ? fc[q * kListTile] : make_float4(0.f, 0.f, 0.f, 0.f);
     return p;
   }
 
-  // CACHED: F holds G = m_j F and wv holds u = w / (r^2 + eps h^2), both from the continuity pass
-  // (list entries of a step's momentum pass); r2 is then not computed: the continuity pass wrote
-  // a zero entry for a listed pair it skipped (coincident double-word positions).
-  template <bool CHECK, bool CACHED = false>
+  template <bool CHECK>
   __device__ __forceinline__ bool geometry(uint32_t t, const Pre& p, df* d, df& r2, df& F, df& wv, df& mj) const {
     const float4 ah = p.ah, al = p.al;
     d[0] = df_sub_close(xi[0], df_make(ah.x, al.x));
     d[1] = df_sub_close(xi[1], df_make(ah.y, al.y));
     d[2] = DIM == 3 ? df_sub_close(xi[2], df_make(ah.z, al.z)) : df_make(0.f, 0.f);
-    r2 = df_make(0.f, 0.f);
-    if (!CACHED) {
-      r2 = df_sumsq3(d[0], d[1], d[2]);
-      if (CHECK) {
-        const df gap = df_sub(r2, df_make(w.four_h2[0], w.four_h2[1]));
-        if (fabsf(gap.hi) <= w.band) {
-          if (!exact_neighbor_call<DIM>(Xd, kself, t, four_h2)) return false;
-        } else if (!(gap.hi < 0.f)) {
-          return false;
-        }
+    r2 = df_sumsq3(d[0], d[1], d[2]);
+    if (CHECK) {
+      const df gap = df_sub(r2, df_make(w.four_h2[0], w.four_h2[1]));
+      if (fabsf(gap.hi) <= w.band) {
+        if (!exact_neighbor_call<DIM>(Xd, kself, t, four_h2)) return false;
+      } else if (!(gap.hi < 0.f)) {
+        return false;
       }
-      if (!(r2.hi > 0.f)) return false;
     }
-    if (CACHED) {
-      F = df_make(p.fw.x, p.fw.y);
-    } else {
-      const df inv_r = df_rsqrt(r2);
-      // F = c0 + c1 r + c2 / r = c0 + (c1 r^2 + c2) / r on either piece of the spline, without a
-      // branch and without forming r (F is continuous at r = h, so the piece chosen by the FP32
-      // r^2 there does not matter beyond rounding)
-      const bool near = r2.hi < w.h2;
-      const df c0 = near ? df_make(w.near0[0], w.near0[1]) : df_make(w.far0[0], w.far0[1]);
-      const df c1 = near ? df_make(w.near1[0], w.near1[1]) : df_make(w.far1[0], w.far1[1]);
-      const df c2 = near ? df_make(0.f, 0.f) : df_make(w.far2[0], w.far2[1]);
-      F = df_add_raw(c0, df_mul(df_add_raw(df_mul(c1, r2), c2), inv_r));  // consumed by products
-    }
-    if (CACHED) {
-      wv = df_make(p.fw.z, p.fw.w);
-    } else {
-      const float4 bh = p.bh, bl = p.bl;
-      // velocity differences, consumed by the dot product only
-      const df dv0 = df_sub_raw(vi[0], df_make(bh.x, bl.x));
-      const df dv1 = df_sub_raw(vi[1], df_make(bh.y, bl.y));
-      const df dv2 = DIM == 3 ? df_sub_raw(vi[2], df_make(bh.z, bl.z)) : df_make(0.f, 0.f);
-      wv = df_dot3(dv0, dv1, dv2, d[0], d[1], d[2]);
-    }
+    if (!(r2.hi > 0.f)) return false;
+    const df inv_r = df_rsqrt(r2);
+    // F = c0 + c1 r + c2 / r = c0 + (c1 r^2 + c2) / r on either piece of the spline, without a
+    // branch and without forming r (F is continuous at r = h, so the piece chosen by the FP32
+    // r^2 there does not matter beyond rounding)
+    const bool near = r2.hi < w.h2;
+    const df c0 = near ? df_make(w.near0[0], w.near0[1]) : df_make(w.far0[0], w.far0[1]);
+    const df c1 = near ? df_make(w.near1[0], w.near1[1]) : df_make(w.far1[0], w.far1[1]);
+    const df c2 = near ? df_make(0.f, 0.f) : df_make(w.far2[0], w.far2[1]);
+    F = df_add_raw(c0, df_mul(df_add_raw(df_mul(c1, r2), c2), inv_r));  // consumed by products
+    const float4 bh = p.bh, bl = p.bl;
+    // velocity differences, consumed by the dot product only
+    const df dv0 = df_sub_raw(vi[0], df_make(bh.x, bl.x));
+    const df dv1 = df_sub_raw(vi[1], df_make(bh.y, bl.y));
+    const df dv2 = DIM == 3 ? df_sub_raw(vi[2], df_make(bh.z, bl.z)) : df_make(0.f, 0.f);
+    wv = df_dot3(dv0, dv1, dv2, d[0], d[1], d[2]);
     mj = df_make(ah.w, al.w);
     return true;
   }
@@ -438,8 +443,7 @@ struct DfPairs {
     return df_div(wv, df_add_raw(r2, df_make(w.eps_h2[0], w.eps_h2[1])));  // a sum of positive terms
   }
 
-  // G = m_j F and u (computed here, or from the cache)
-  __device__ __forceinline__ void momentum(const float4& rpj, const df* d, df G, df u) {
+    __device__ __forceinline__ void momentum(const float4& rpj, const df* d, df G, df u) {
     // artificial viscosity where the pair approaches (w < 0, so u < 0), computed for every pair
     // and then selected: nearly every warp has lanes on both sides
     const df den = df_add_raw(rhoi, df_make(rpj.x, rpj.y));  // a sum of positive terms
@@ -451,30 +455,68 @@ struct DfPairs {
     if (DIM == 3) dfacc_add_prod(acc[2], ncoef, d[2]);
   }
 
-  template <bool CHECK, bool CACHED>
+  template <bool CHECK>
   __device__ __forceinline__ void terms(uint32_t t, uint32_t q, const Pre& p) {
     constexpr bool kStore = STAGE == SPH_CONT && !CHECK;  // list entries of the continuity pass
     df d[3], r2, F, wv, mj;
-    if (!geometry<CHECK, CACHED>(t, p, d, r2, F, wv, mj)) {
+    if (!geometry<CHECK>(t, p, d, r2, F, wv, mj)) {
       if (kStore && fc) fc[q * kListTile] = make_float4(0.f, 0.f, 0.f, 0.f);  // contributes nothing
       return;
     }
-    const df G = CACHED ? F : df_mul(mj, F);
-    if (kStore && fc) {
+    const df G = df_mul(mj, F);
+    if (kStore && fc) {  // (fc is set; without this branch the unrolled pairs are scheduled 10 % slower)
       const df u = visc_u(r2, wv);
       fc[q * kListTile] = make_float4(G.hi, G.lo, u.hi, u.lo);
     }
     if (kCont) dfacc_add_prod(dr, G, wv);
-    if (kMom) momentum(p.rp, d, G, CACHED ? wv : visc_u(r2, wv));
+    if (kMom) momentum(p.rp, d, G, visc_u(r2, wv));
   }
 
   // entry q of an exact neighbour list
-  __device__ __forceinline__ void pair_with(uint32_t t, uint32_t q, const Pre& p) {
-    if (STAGE == SPH_MOM && fc) terms<false, true>(t, q, p);
-    else terms<false, false>(t, q, p);
-  }
+  __device__ __forceinline__ void pair_with(uint32_t t, uint32_t q, const Pre& p) { terms<false>(t, q, p); }
   // any candidate (the walk that continues an overflowed list): everything computed here
-  __device__ __forceinline__ void pair(uint32_t t) { terms<true, false>(t, 0, fetch_entry(t, 0, false)); }
+  __device__ __forceinline__ void pair(uint32_t t) { terms<true>(t, 0, fetch_entry(t, 0, false)); }
+
+  // The continued walk of an overflowed list, summed apart (in the momentum pass from the full record: only
+  // this walk needs velocities) and added; summed into the pass's own state it slowed the loop over
+  // the list (4M particles, momentum pass 1.97 -> 2.7 ms).
+  static constexpr bool kResumeApart = kCacheF;
+  __device__ __forceinline__ void resume(const SphArgs& a, uint32_t k) {
+    DfPairs<DIM, SPH_RATES> P;
+    P.begin(a, a.sys[sys_of_slot(a, a.sorted_id[k])], k);
+    continue_walk<DIM, false>(a, k, [&](uint32_t t) { P.pair(t); });
+    if (STAGE == SPH_CONT) dr = dfacc_add(dr, P.dr);
+#pragma unroll
+    for (int cc = 0; cc < DIM; ++cc)
+      if (STAGE == SPH_MOM) acc[cc] = dfacc_add(acc[cc], P.acc[cc]);
+  }
+
+  // Two list entries of the momentum pass at once, in packed arithmetic (the operations of momentum(), half a
+  // for the first entry, half b for the second; without `both` the second contributes nothing).
+  // Packed instructions need half the issue slots, which together with the L1's accesses limit the
+  // pass: with the 32-byte records 262k particles 0.163 -> 0.131 ms, 4M 2.23 -> 1.89, 6.1M in 2D 1.15 ->
+  // 0.91.  The entries' terms are added in list order, so the sums are bit for bit those of one entry
+  // after the other (summing the halves apart would change the states' rounding, which the
+  // mixed-precision adjoint amplifies to 2e-9 of its gradients).  The continuity pass, whose FMA
+  // pipe is 67 % busy, gained nothing (262k particles 0.165 -> 0.171 to 0.188 ms).
+  __device__ __forceinline__ void pair_two(const Pre& a, const Pre& b, bool both) {
+    df2 d[3];
+    d[0] = df2_sub_close(df2_dup(xi[0]), df2_make(f2_make(a.ah.x, b.ah.x), f2_make(a.al.x, b.al.x)));
+    d[1] = df2_sub_close(df2_dup(xi[1]), df2_make(f2_make(a.ah.y, b.ah.y), f2_make(a.al.y, b.al.y)));
+    d[2] = DIM == 3 ? df2_sub_close(df2_dup(xi[2]), df2_make(f2_make(a.ah.z, b.ah.z), f2_make(a.al.z, b.al.z)))
+                    : df2_make(0ull, 0ull);
+    const df none = df_make(0.f, 0.f);
+    const df2 G = df2_pair(df_make(a.fw.x, a.fw.y), both ? df_make(b.fw.x, b.fw.y) : none);
+    const df2 u = df2_make(f2_make(a.fw.z, b.fw.z), f2_make(a.fw.w, b.fw.w));
+    const df2 den = df2_add_raw(df2_dup(rhoi), df2_make(f2_make(a.rp.x, b.rp.x), f2_make(a.rp.y, b.rp.y)));
+    const df2 av = df2_div(df2_mul(df2_make(f2_dup(w.avk[0]), f2_dup(w.avk[1])), u), den);
+    const df2 pij = df2_pair(a.fw.z < 0.f ? df2_first(av) : none, b.fw.z < 0.f ? df2_second(av) : none);
+    const df2 Pj = df2_make(f2_make(a.rp.z, b.rp.z), f2_make(a.rp.w, b.rp.w));
+    const df2 ncoef = df2_neg(df2_mul(df2_add_raw(df2_add_raw(df2_dup(Pi), Pj), pij), G));
+    dfacc_add_prod2(acc[0], ncoef, d[0]);
+    dfacc_add_prod2(acc[1], ncoef, d[1]);
+    if (DIM == 3) dfacc_add_prod2(acc[2], ncoef, d[2]);
+  }
 
   // Combine the partial sums of the LANES lanes of a slot (butterfly; every lane ends with the sum).
   template <int LANES>
@@ -621,9 +663,8 @@ void sph_sorted_layout(int arith, size_t sz[6]) {
     case ARITH_F64_EXACT:  // double4 {x,m}, double4 {v,0}, double2 {rho,P}
       sz[0] = 32; sz[1] = 32; sz[2] = 16;
       break;
-    case ARITH_F64_DF:  // DfRecord {A.hi, A.lo, V.hi, V.lo} (pair passes), float4 {rho, P} (hi, lo),
-                        // double4 exact positions
-      sz[1] = 64; sz[4] = 16; sz[5] = 32;
+    case ARITH_F64_DF:  // DfHalf {x, m}, DfRecord {x, m}, {v}, float4 {rho, P} (hi, lo), double4 exact positions
+      sz[0] = 32; sz[1] = 64; sz[4] = 16; sz[5] = 32;
       break;
     default:  // float4 {x,m}, float4 {v,0}, float2 {rho,P}
       sz[0] = 16; sz[1] = 16; sz[2] = 8;

@@ -330,6 +330,13 @@ __device__ __forceinline__ void find_in_lists(const SphArgs& a, const uint32_t (
     if (pos[i] >= L[i] || lt[i][(size_t)pos[i] * kListTile] != k) pos[i] = kNoMirror;
 }
 
+// 32 bytes from a 32-byte aligned address by one load per lane (read-only for the kernel).
+__device__ __forceinline__ void load_32b(const float4* p, float4& a, float4& b) {
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+      : "l"(p));
+}
+
 // L2 prefetch hint for one address (PTX prefetch.global.L2; a hint, it returns nothing).
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
@@ -356,6 +363,49 @@ struct PrefetchPolicy {
 template <class P>
 struct PrefetchPolicy<P, decltype((void)P::kPrefetch)> {
   static constexpr bool value = P::kPrefetch;
+};
+
+// The rest of the candidate walk of slot k after its list reached capacity, in walk order: fn(t) for every
+// candidate that passes the FP32 test.
+template <int DIM, bool EXACT_PF, class Fn>
+__device__ __forceinline__ void continue_walk(const SphArgs& a, uint32_t k, Fn&& fn) {
+  const SphK* Kp;
+  const Target T = target_of(a, k, &Kp, a.reach);
+  const SphK& K = *Kp;
+  const GridK& g = K.g;
+  const int R = a.reach, RZ = DIM == 3 ? R : 0, side = 2 * R + 1, nrows = side * (2 * RZ + 1);
+  const float4 pi = pf_at<DIM>(a.pf, k);
+  const float thr = prefilter_threshold<EXACT_PF>(K, pi);
+  const int row0 = (int)a.nresume[2 * (size_t)k];
+  const uint32_t t0 = a.nresume[2 * (size_t)k + 1];
+  for (int row = row0; row < nrows; ++row) {
+    const int z = T.cz + row / side - RZ, y = T.cy + row % side - R;
+    if (z < 0 || z >= g.nz || y < 0 || y >= g.ny) continue;
+    const uint32_t rb = g.cell_base + ((uint32_t)z * g.ny + (uint32_t)y) * g.nx;
+    const uint32_t e = a.cell_start[rb + T.x1 + 1];
+    for (uint32_t t = row == row0 ? t0 : a.cell_start[rb + T.x0]; t < e; ++t)
+      if (prefilter_hit<DIM, EXACT_PF>(pi, pf_at<DIM>(a.pf, t), thr)) fn(t);
+  }
+}
+
+// Policies that sum the continued walk apart: resume(args, slot).
+template <class P, class = void>
+struct ResumePolicy {
+  static constexpr bool value = false;
+};
+template <class P>
+struct ResumePolicy<P, decltype((void)P::kResumeApart)> {
+  static constexpr bool value = P::kResumeApart;
+};
+
+// Policies whose passes take two entries at a time: pair_two(fetched a, fetched b, both).
+template <class P, class = void>
+struct TwoPolicy {
+  static constexpr bool value = false;
+};
+template <class P>
+struct TwoPolicy<P, decltype((void)P::kTwo)> {
+  static constexpr bool value = P::kTwo;
 };
 
 // Pair pass over the lists of sph_list_kernel (any block size up to kSphMaxThreads, a
@@ -386,7 +436,32 @@ __global__ void __launch_bounds__(kSphMaxThreads) sph_list_pass_kernel(SphArgs a
     const uint32_t cnt = live ? a.nlen[k] : 0u;
     const uint32_t L = min(cnt, cap);
     const uint32_t* __restrict__ my = a.nlist + list_base(k, cap);  // entry q at my[q * kListTile]
-    if constexpr (PrefetchPolicy<Pairs>::value) {
+    if constexpr (TwoPolicy<Pairs>::value) {
+      // software pipeline over pairs of entries: list entries two pairs ahead, records one
+      constexpr uint32_t S = LANES;
+      auto at = [&](uint32_t q) { return my[(size_t)min(q, L - 1) * kListTile]; };
+      if (sub < L) {
+        uint32_t tna = at(sub + 2 * S), tnb = at(sub + 3 * S);
+        typename Pairs::Pre ca = P.fetch(at(sub), sub), cb = P.fetch(at(sub + S), min(sub + S, L - 1));
+        for (uint32_t q = sub; q < L; q += 2 * S) {
+          if (q + kL2Ahead * S < L) {
+            prefetch_l2(my + (size_t)(q + kL2Ahead * S) * kListTile);
+            prefetch_l2(my + (size_t)min(q + (kL2Ahead + 1) * S, L - 1) * kListTile);
+            if constexpr (L2EntryPolicy<Pairs>::value) {
+              P.prefetch_entry(q + kL2Ahead * S);
+              P.prefetch_entry(min(q + (kL2Ahead + 1) * S, L - 1));
+            }
+          }
+          const uint32_t ta = at(q + 4 * S), tb = at(q + 5 * S);
+          const typename Pairs::Pre na = P.fetch(tna, min(q + 2 * S, L - 1)), nb = P.fetch(tnb, min(q + 3 * S, L - 1));
+          P.pair_two(ca, cb, q + S < L);
+          ca = na;
+          cb = nb;
+          tna = ta;
+          tnb = tb;
+        }
+      }
+    } else if constexpr (PrefetchPolicy<Pairs>::value) {
       // software pipeline: list entries two ahead, the neighbour's pack records one ahead; the
       // unrolled pair bodies (branch-free) interleave
       constexpr uint32_t S = LANES;
@@ -410,25 +485,9 @@ __global__ void __launch_bounds__(kSphMaxThreads) sph_list_pass_kernel(SphArgs a
     } else {
       for (uint32_t q = sub; q < L; q += LANES) P.pair(my[q * kListTile]);
     }
-    if (cnt > cap && sub == 0) {
-      // rare: continue the candidate walk where the list stopped
-      const float* __restrict__ PF = a.pf;
-      const SphK* Kp;
-      const Target T = target_of(a, k0, &Kp, a.reach);
-      const GridK& g = K.g;
-      const int R = a.reach, RZ = DIM == 3 ? R : 0, side = 2 * R + 1, nrows = side * (2 * RZ + 1);
-      const float4 pi = pf_at<DIM>(PF, k);
-      const float thr = prefilter_threshold<EXACT_PF>(K, pi);
-      const int row0 = (int)a.nresume[2 * (size_t)k];
-      const uint32_t t0 = a.nresume[2 * (size_t)k + 1];
-      for (int row = row0; row < nrows; ++row) {
-        const int z = T.cz + row / side - RZ, y = T.cy + row % side - R;
-        if (z < 0 || z >= g.nz || y < 0 || y >= g.ny) continue;
-        const uint32_t rb = g.cell_base + ((uint32_t)z * g.ny + (uint32_t)y) * g.nx;
-        const uint32_t e = a.cell_start[rb + T.x1 + 1];
-        for (uint32_t t = row == row0 ? t0 : a.cell_start[rb + T.x0]; t < e; ++t)
-          if (prefilter_hit<DIM, EXACT_PF>(pi, pf_at<DIM>(PF, t), thr)) P.pair(t);
-      }
+    if (cnt > cap && sub == 0) {  // rare: continue the candidate walk where the list stopped
+      if constexpr (ResumePolicy<Pairs>::value) P.resume(a, k);
+      else continue_walk<DIM, EXACT_PF>(a, k, [&](uint32_t t) { P.pair(t); });
     }
     if constexpr (LANES > 1) P.template reduce_lanes<LANES>();  // whole warps: the tile loop is uniform
     if (live && sub == 0) P.finish(a, K, id, k);
