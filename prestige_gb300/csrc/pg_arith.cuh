@@ -272,15 +272,21 @@ __device__ __forceinline__ dfacc dfacc_zero() {
   return a;
 }
 
-// a += x * y
-__device__ __forceinline__ void dfacc_add_prod(dfacc& a, df x, df y) {
+// x * y as dfacc_add_term takes it
+__device__ __forceinline__ df dfacc_term(df x, df y) {
   const float p = __fmul_rn(x.hi, y.hi);
   const float e = __fmaf_rn(x.hi, y.hi, -p);
-  const float pl = fmaf(x.hi, y.lo, fmaf(x.lo, y.hi, e));
-  const df s = two_sum(a.hi, p);
-  a.hi = s.hi;
-  a.lo = a.lo + (s.lo + pl);
+  return df_make(p, fmaf(x.hi, y.lo, fmaf(x.lo, y.hi, e)));
 }
+
+__device__ __forceinline__ void dfacc_add_term(dfacc& a, df t) {
+  const df s = two_sum(a.hi, t.hi);
+  a.hi = s.hi;
+  a.lo = a.lo + (s.lo + t.lo);
+}
+
+// a += x * y
+__device__ __forceinline__ void dfacc_add_prod(dfacc& a, df x, df y) { dfacc_add_term(a, dfacc_term(x, y)); }
 
 // a + b of two accumulators (TwoSum of the high parts, the low parts added)
 __device__ __forceinline__ dfacc dfacc_add(dfacc a, dfacc b) {

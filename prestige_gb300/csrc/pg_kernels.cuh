@@ -98,7 +98,8 @@ int launch_sph_repack_rho(cudaStream_t st, const SphArgs& a, int arith);  // pac
 int launch_sph_list(cudaStream_t st, const SphArgs& a, int arith, int grid, int block);
 // lanes: threads per slot of the continuity and momentum passes (1, 2 or 4: 32, 16 or 8
 // particles per warp); only the tolerance-based modes (double-word f64, contracted f32) take
-// more than one, the others run 1 (sph_pass_lanes gives the count a pass actually uses).
+// more than one, the others run 1 (sph_pass_lanes gives the count a pass actually uses).  With 1,
+// the double-word passes of small handles run 2 or 4 threads per slot that add in list order (same bits).
 int launch_sph_list_pass(cudaStream_t st, const SphArgs& a, int arith, int stage, int grid, int block,
                          int lanes = 1);
 int sph_pass_lanes(int arith, int stage, int lanes);

@@ -456,13 +456,17 @@ struct DfPairs {
     return df_div(wv, df_add_raw(r2, df_make(w.eps_h2[0], w.eps_h2[1])));  // a sum of positive terms
   }
 
-    __device__ __forceinline__ void momentum(const float4& rpj, const df* d, df G, df u) {
+  __device__ __forceinline__ df momentum_coef(const float4& rpj, df G, df u) const {
     // artificial viscosity where the pair approaches (w < 0, so u < 0), computed for every pair
     // and then selected: nearly every warp has lanes on both sides
     const df den = df_add_raw(rhoi, df_make(rpj.x, rpj.y));  // a sum of positive terms
     const df av = df_div(df_mul(df_make(w.avk[0], w.avk[1]), u), den);
     const df pij = u.hi < 0.f ? av : df_make(0.f, 0.f);
-    const df ncoef = df_neg(df_mul(df_add_raw(df_add_raw(Pi, df_make(rpj.z, rpj.w)), pij), G));
+    return df_neg(df_mul(df_add_raw(df_add_raw(Pi, df_make(rpj.z, rpj.w)), pij), G));
+  }
+
+  __device__ __forceinline__ void momentum(const float4& rpj, const df* d, df G, df u) {
+    const df ncoef = momentum_coef(rpj, G, u);
     dfacc_add_prod(acc[0], ncoef, d[0]);
     dfacc_add_prod(acc[1], ncoef, d[1]);
     if (DIM == 3) dfacc_add_prod(acc[2], ncoef, d[2]);
@@ -487,6 +491,29 @@ struct DfPairs {
 
   // entry q of an exact neighbour list
   __device__ __forceinline__ void pair_with(uint32_t t, uint32_t q, const Pre& p) { terms<false>(t, q, p); }
+
+  // What pair_with(t, q, p) adds, without adding it (sph_ordered_pass_kernel).
+  static constexpr int kTerms = STAGE == SPH_MOM ? DIM : 1;
+  __device__ __forceinline__ void list_terms(uint32_t t, uint32_t q, const Pre& p, df (&out)[kTerms]) const {
+    if constexpr (STAGE == SPH_MOM) {
+      const df ncoef = momentum_coef(p.rp, df_make(p.fw.x, p.fw.y), df_make(p.fw.z, p.fw.w));
+      out[0] = dfacc_term(ncoef, df_sub_close(xi[0], df_make(p.ah.x, p.al.x)));
+      out[1] = dfacc_term(ncoef, df_sub_close(xi[1], df_make(p.ah.y, p.al.y)));
+      if constexpr (DIM == 3) out[2] = dfacc_term(ncoef, df_sub_close(xi[2], df_make(p.ah.z, p.al.z)));
+    } else {
+      df d[3], r2, F, wv, mj;
+      if (!geometry<false>(t, p, d, r2, F, wv, mj)) {
+        fc[q * kListTile] = make_float4(0.f, 0.f, 0.f, 0.f);
+        return;
+      }
+      const df G = df_mul(mj, F), u = visc_u(r2, wv);
+      fc[q * kListTile] = make_float4(G.hi, G.lo, u.hi, u.lo);
+      out[0] = dfacc_term(G, wv);
+    }
+  }
+  __device__ __forceinline__ void add_term(int c, df term) {
+    dfacc_add_term(STAGE == SPH_MOM ? acc[c] : dr, term);
+  }
   // any candidate (the walk that continues an overflowed list): everything computed here
   __device__ __forceinline__ void pair(uint32_t t) { terms<true>(t, 0, fetch_entry(t, 0, false)); }
 
@@ -607,6 +634,20 @@ PassKernel list_pass_for(int arith, int lanes) {
     default:
       return nullptr;
   }
+}
+
+// Threads per slot of the double-word passes of a handle of n particles with one thread per slot set:
+// more than one where one would leave schedulers idle (sph_ordered_pass_kernel).  Step in us, with 1 / 2 / 4
+// threads per slot: 2D dam break of 6,518 particles 36.7 / 31.1 / 29.2, of 13,518 39.5 / 35.1 / 33.4, of
+// 23,018 41.7 / 37.5 / 38.2, of 37,718 44.0 / 43.1 / 49.7; 3D lattice (half-size cells) of 5,000 particles
+// 89 / 72 / 61, of 10,000 90 / 73 / 69, of 20,000 91 / 84 / 86, of 30,000 101 / 99 / 109, of 45,000
+// 122 / 133 / 136.  (8 threads: 29.6 and 61.6 at the small ends, worse from there on.)
+int ordered_lanes(uint32_t n) { return n <= 16384 ? 4 : n <= 32768 ? 2 : 1; }
+
+template <int DIM, int LANES>
+PassKernel ordered_kernel(int stage) {
+  return stage == SPH_CONT ? sph_ordered_pass_kernel<DfPairs<DIM, SPH_CONT>, DIM, LANES>
+                           : sph_ordered_pass_kernel<DfPairs<DIM, SPH_MOM>, DIM, LANES>;
 }
 
 // The list kernel with the batch that suits the rows' length (see sph_list_kernel).
@@ -752,6 +793,12 @@ int launch_sph_list_exact(cudaStream_t st, const SphArgs& a, int grid, int block
 
 int launch_sph_list_pass(cudaStream_t st, const SphArgs& a, int arith, int stage, int grid, int block, int lanes) {
   lanes = sph_pass_lanes(arith, stage, lanes);
+  const int ordered = arith == ARITH_F64_DF && lanes == 1 && stage != SPH_RATES ? ordered_lanes(a.n) : 1;
+  if (ordered > 1) {
+    const PassKernel kern = ordered == 4 ? (a.dim == 2 ? ordered_kernel<2, 4>(stage) : ordered_kernel<3, 4>(stage))
+                                         : (a.dim == 2 ? ordered_kernel<2, 2>(stage) : ordered_kernel<3, 2>(stage));
+    return launch_table(st, a, kern, 0, block, ordered);  // one block per tile
+  }
   PassKernel kern = list_kernel(arith, a.dim, stage, lanes, a.reach);
   return launch_table(st, a, kern, grid, block, lanes);
 }

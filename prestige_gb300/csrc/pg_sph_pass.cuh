@@ -494,5 +494,48 @@ __global__ void __launch_bounds__(kSphMaxThreads) sph_list_pass_kernel(SphArgs a
   }
 }
 
+// The pass with LANES threads per slot for systems that leave the chip idle: a slot's pairs are
+// evaluated LANES at a time, and every lane then adds the LANES terms in list order (shuffled from the
+// lane that has them), so the sums are bit for bit those of one thread per slot.  What bounds such a
+// system is the chain of one thread's pairs, each a few hundred dependent instructions; the additions are
+// a tenth of them.  One block per tile.
+template <class Pairs, int DIM, int LANES>
+__global__ void __launch_bounds__(kSphMaxThreads) sph_ordered_pass_kernel(SphArgs a) {
+  chain_begin();
+  const uint32_t cap = a.cap, sub = threadIdx.x % LANES, spb = blockDim.x / LANES;
+  const uint32_t k0 = (a.k_begin / spb + blockIdx.x) * spb + threadIdx.x / LANES;
+  const bool live = k0 < a.k_end;
+  const uint32_t k = live ? k0 : a.n - 1;
+  const uint32_t id = a.sorted_id[k];
+  const SphK& K = a.sys[sys_of_slot(a, id)];
+  Pairs P;
+  P.begin(a, K, k);
+  const uint32_t cnt = live ? a.nlen[k] : 0u;
+  const uint32_t L = min(cnt, cap), longest = __reduce_max_sync(0xffffffffu, L);
+  const uint32_t* __restrict__ my = a.nlist + list_base(k, cap);
+  auto at = [&](uint32_t q) { return q < L ? my[(size_t)q * kListTile] : k; };
+  uint32_t t = at(sub), tn = at(sub + LANES);
+  typename Pairs::Pre cur = P.fetch(t, sub < L ? sub : 0u);
+  for (uint32_t q0 = 0; q0 < longest; q0 += LANES) {
+    const uint32_t q = q0 + sub, tnn = at(q + 2 * LANES);
+    const typename Pairs::Pre nxt = P.fetch(tn, q + LANES < L ? q + LANES : 0u);
+    df term[Pairs::kTerms];
+#pragma unroll
+    for (int c = 0; c < Pairs::kTerms; ++c) term[c] = df_make(0.f, 0.f);
+    if (q < L) P.list_terms(t, q, cur, term);
+#pragma unroll
+    for (int l = 0; l < LANES; ++l)
+#pragma unroll
+      for (int c = 0; c < Pairs::kTerms; ++c)
+        P.add_term(c, df_make(__shfl_sync(0xffffffffu, term[c].hi, l, LANES),
+                              __shfl_sync(0xffffffffu, term[c].lo, l, LANES)));
+    cur = nxt;
+    t = tn;
+    tn = tnn;
+  }
+  if (cnt > cap && sub == 0) P.resume(a, k);  // rare: continue the candidate walk where the list stopped
+  if (live && sub == 0) P.finish(a, K, id, k);
+}
+
 }  // namespace sphpass
 }  // namespace pg
