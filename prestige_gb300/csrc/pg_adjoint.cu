@@ -561,7 +561,7 @@ int pg_forward_checkpointed(pg_system* s, int nsteps, int every) {
   for (int seg = 0; seg < A->nseg; ++seg) {
     PG_TRY(pg::copy_state_out(s, A->ckpt.as<double>() + (size_t)seg * A->state_doubles));
     const int steps = std::min(every, nsteps - seg * every);
-    for (int t = 0; t < steps; ++t) PG_TRY(pg::enqueue_sph_step(s, false, 1, nullptr));
+    for (int t = 0; t < steps; ++t) PG_TRY(pg::enqueue_sph_step(s, false, 1, nullptr, t > 0));
   }
   PG_TRY(pg::copy_state_out(s, A->final_state.as<double>()));
   PG_TRY(pg::sync_and_check(s));

@@ -46,7 +46,7 @@ enum : unsigned {
 };
 
 // ---------------------------------------------------------------------------------------
-// Dependent launches inside a step.  The kernels of a step form a chain on one stream, and below about
+// Dependent launches inside a step and from one step to the next.  The kernels of a step form a chain on one stream, and below about
 // 100k particles a good part of a step is the gap between a kernel's end and the next one's first
 // instruction.  A kernel launched with launch_chained directly after another kernel (no copy, memset
 // or event in between) is set up while that one runs and starts as its last blocks end; chain_begin(),
@@ -54,6 +54,7 @@ enum : unsigned {
 // writes are visible.  Since every kernel waits for the one before, a kernel's inputs may come from
 // any earlier kernel of the stream.  us per step with plain and chained launches: dam break, 6.5k
 // particles, eager 51.8 / 38.0, as a graph 38.8 / 37.2; 100k eager 244 / 231; 262k eager 475 / 463.
+// The first kernel of a step is chained to the step before it: 3D lattice of 5,000 particles, eager, 61.5 -> 59.4.
 // Letting the next kernel's blocks in from the start of the current one (an early launch_dependents)
 // was slower (100k 273, 262k 489): they settle unevenly over the SMs.
 // ---------------------------------------------------------------------------------------
@@ -180,7 +181,8 @@ __device__ __forceinline__ uint32_t ordered_slot(const NbrOrder& o, uint32_t s, 
 // Cell of every particle (id order) with its arrival rank in the cell, counted into w.count.
 // posmin (optional, f64 positions only): per system and dimension ([3 sys + d]) the minimum
 // position, as ordered_code values, folded in with atomicMin (all ones before).
-int launch_hash(cudaStream_t st, const GridK* grid_dev, const uint32_t* sys_of_id, int f64, int dim,
+// chained: directly after another kernel of the stream.
+int launch_hash(cudaStream_t st, bool chained, const GridK* grid_dev, const uint32_t* sys_of_id, int f64, int dim,
                 const void* pos, NbrWork& w, unsigned long long* posmin = nullptr);
 
 // Order-preserving map of doubles to unsigned 64-bit integers (and back), for atomicMin.

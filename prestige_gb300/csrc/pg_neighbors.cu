@@ -379,26 +379,23 @@ inline unsigned blocks_for(size_t n, int t) { return (unsigned)((n + t - 1) / t)
 }  // namespace
 
 template <class R, int DIM>
-static void hash_dim(cudaStream_t st, const GridK* grid, const uint32_t* sys_of_id, const void* pos, NbrWork& w,
-                     unsigned long long* posmin) {
-  const unsigned b = blocks_for(w.n, 256);
-  if (sizeof(R) == 8 && posmin)
-    hash_kernel<R, DIM, true><<<b, 256, 0, st>>>(grid, sys_of_id, (const R*)pos, (uint32_t)w.n, w.key, w.rank,
-                                                 w.count, w.big, posmin);
-  else
-    hash_kernel<R, DIM, false><<<b, 256, 0, st>>>(grid, sys_of_id, (const R*)pos, (uint32_t)w.n, w.key, w.rank,
-                                                  w.count, w.big, nullptr);
+static cudaError_t hash_dim(cudaStream_t st, bool chained, const GridK* grid, const uint32_t* sys_of_id, const void* pos,
+                            NbrWork& w, unsigned long long* posmin) {
+  const bool min = sizeof(R) == 8 && posmin;
+  return launch_chained(st, chained, min ? hash_kernel<R, DIM, true> : hash_kernel<R, DIM, false>, blocks_for(w.n, 256),
+                        256, grid, sys_of_id, (const R*)pos, (uint32_t)w.n, w.key, w.rank, w.count, w.big,
+                        min ? posmin : nullptr);
 }
 
-int launch_hash(cudaStream_t st, const GridK* grid_dev, const uint32_t* sys_of_id, int f64, int dim, const void* pos,
-                NbrWork& w, unsigned long long* posmin) {
+int launch_hash(cudaStream_t st, bool chained, const GridK* grid_dev, const uint32_t* sys_of_id, int f64, int dim,
+                const void* pos, NbrWork& w, unsigned long long* posmin) {
   if (w.n == 0) return PG_OK;
   if (f64) {
-    if (dim == 2) hash_dim<double, 2>(st, grid_dev, sys_of_id, pos, w, posmin);
-    else hash_dim<double, 3>(st, grid_dev, sys_of_id, pos, w, posmin);
+    if (dim == 2) PG_CUDA_TRY((hash_dim<double, 2>(st, chained, grid_dev, sys_of_id, pos, w, posmin)));
+    else PG_CUDA_TRY((hash_dim<double, 3>(st, chained, grid_dev, sys_of_id, pos, w, posmin)));
   } else {
-    if (dim == 2) hash_dim<float, 2>(st, grid_dev, sys_of_id, pos, w, nullptr);
-    else hash_dim<float, 3>(st, grid_dev, sys_of_id, pos, w, nullptr);
+    if (dim == 2) PG_CUDA_TRY((hash_dim<float, 2>(st, chained, grid_dev, sys_of_id, pos, w, nullptr)));
+    else PG_CUDA_TRY((hash_dim<float, 3>(st, chained, grid_dev, sys_of_id, pos, w, nullptr)));
   }
   PG_CUDA_TRY(cudaGetLastError());
   return PG_OK;

@@ -87,7 +87,8 @@ struct pg_system {
   // CUDA graph of one step (DEM: one per history parity)
   bool graph_enabled = false;
   int list_arith = -1;  // arithmetic mode of the pair lists in nlist/nlen (-1: none built yet)
-  cudaGraphExec_t graph_exec[2] = {nullptr, nullptr};
+  cudaGraphExec_t graph_exec[2] = {nullptr, nullptr};   // one step (DEM: per history buffer)
+  cudaGraphExec_t graph_steps[2] = {nullptr, nullptr};  // kGraphSteps steps
 
   // step timing (pg_timing_enable): 4 events per step, consumed by pg_timing_read
   bool timing = false;
@@ -107,9 +108,9 @@ namespace pg {
 size_t pg_elem_bytes(const pg_system* s);
 int ensure_sorted_buffers(pg_system* s);
 SphArgs sph_args(pg_system* s, int integrate, bool rates);
-int enqueue_neighbors(pg_system* s);
-int enqueue_sph_step(pg_system* s, bool rates, int integrate, cudaEvent_t* ev);
-int enqueue_sph_front(pg_system* s, cudaEvent_t* ev);
+int enqueue_neighbors(pg_system* s, bool chained = false);
+int enqueue_sph_step(pg_system* s, bool rates, int integrate, cudaEvent_t* ev, bool chained = false);
+int enqueue_sph_front(pg_system* s, cudaEvent_t* ev, bool chained = false);
 int enqueue_sph_momentum(pg_system* s, bool chained, cudaEvent_t* ev);
 long long neighbor_launches(const pg_system* s);
 int sync_and_check(pg_system* s);
@@ -118,7 +119,7 @@ int retune_sph(pg_system* s, double mult, int f64_mode, int block);
 int mom_block(const pg_system* s);
 int set_momentum_block(pg_system* s, int block);
 int set_pass_lanes(pg_system* s, int lanes);
-int enqueue_step(pg_system* s);
+int enqueue_step(pg_system* s, bool chained = false);
 int apply_io_inputs(pg_system* s);
 void drop_graphs(pg_system* s);
 int capture_graphs(pg_system* s);
