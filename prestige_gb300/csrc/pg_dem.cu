@@ -183,7 +183,7 @@ __global__ void dem_gather_kernel(DemArgs a) {
   a.sF[k] = make_float4((float)x0, (float)x1, (float)x2, (float)r);
 }
 
-// The integrator's f64 divisions (a DFMA sequence each on a 1/64-rate pipe), out of line so
+// The integrator's f64 divisions (long integer sequences, soft_div), out of line so
 // that the particles that skip them (no contact force, no torque) do not run them predicated.
 struct D3 {
   double x, y, z;
@@ -502,7 +502,7 @@ __global__ void __launch_bounds__(kDemThreads) dem_pass_kernel(DemArgs a) {
     const double I = free_t ? 0.0 : dmul(dmul(dmul(0.4, me.m), me.r), me.r);
     const bool m_ok = positive_finite(me.m);
     // F / m: the divisions sit behind a branch that the particles without a contact force skip
-    // (a select would run them for every particle: the f64 division is a sequence of DFMAs)
+    // (a select would run them for every particle: the f64 division is a long integer sequence)
     double fm[3] = {F[0], F[1], F[2]};
     if (!(m_ok && is_zero(F[0]) && is_zero(F[1]) && is_zero(F[2]))) {
       const D3 q = force_per_mass(D3{F[0], F[1], F[2]}, me.m, m_ok);

@@ -17,12 +17,11 @@
 // rates from one snapshot would advance it by forward Euler, which amplifies every acoustic
 // mode.  A third variant (pg_compute_rates) evaluates C and M of one state in one pass.
 //
-// Kernel structure (one thread per target particle i, slot order; pg_sph_pass.cuh):
-//   phase 1  every candidate of the 9 (2D: 3) neighbour rows is tested in FP32 against a
-//            conservative bound on r^2; passing slots are appended to a per-thread list in
-//            shared memory.
-//   phase 2  when any lane's list is full (or all lanes are done) the warp evaluates the
-//            listed pairs: the exact neighbour test, then the pair terms.
+// Kernel structure (pg_sph_pass.cuh): the list kernel tests every candidate of the 9 (2D: 3)
+// neighbour rows in FP32 against bounds on r^2, with the exact test inside their band, and
+// writes each target's neighbours in walk order; the two passes evaluate the listed pairs, one
+// thread per target (slot order; more in small double-word systems).  The IEEE f64 step
+// evaluates each pair once instead (pg_sph_sym.cu).
 // Pairs are evaluated in the oracle's order (rows z, y ascending; slots ascending), so the
 // IEEE modes reproduce the oracle bit for bit.
 #include <cuda_runtime.h>
