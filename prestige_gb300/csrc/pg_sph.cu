@@ -268,16 +268,54 @@ struct RealPairs {
   // classified with the f64 test, f32 lists with the IEEE FP32 test), so no test is repeated.
   __device__ __forceinline__ void pair_with(uint32_t t, uint32_t, const Pre& p) { terms<false>(t, p); }
 
+  // What one pair adds: dr += m w F; acc -= coef d.
+  struct Term {
+    R m, wF, coef, d[3];
+  };
+
+  __device__ __forceinline__ void add_term(const Term& x) {
+    if (kCont) dr = Ops::add(dr, Ops::mul(x.m, x.wF));
+    if (kMom) {
+#pragma unroll
+      for (int cc = 0; cc < DIM; ++cc) acc[cc] = Ops::sub(acc[cc], Ops::mul(x.coef, x.d[cc]));
+    }
+  }
+
+  __device__ __forceinline__ void list_terms(uint32_t, uint32_t, const Pre& p, Term& x) const { evaluate<false>(p, x); }
+
+  template <int LANES>
+  static __device__ __forceinline__ Term shuffle(const Term& x, int l) {
+    Term y;
+    y.m = y.wF = y.coef = y.d[2] = R(0);
+    if (kCont) {
+      y.m = __shfl_sync(0xffffffffu, x.m, l, LANES);
+      y.wF = __shfl_sync(0xffffffffu, x.wF, l, LANES);
+    }
+    if (kMom) {
+      y.coef = __shfl_sync(0xffffffffu, x.coef, l, LANES);
+#pragma unroll
+      for (int cc = 0; cc < DIM; ++cc) y.d[cc] = __shfl_sync(0xffffffffu, x.d[cc], l, LANES);
+    }
+    return y;
+  }
+
   template <bool TEST>
-  __device__ __forceinline__ void terms(uint32_t t, const Pre& p) {
+  __device__ __forceinline__ void terms(uint32_t, const Pre& p) {
+    Term x;
+    if (evaluate<TEST>(p, x)) add_term(x);
+  }
+
+  // false: not a neighbour (TEST).
+  template <bool TEST>
+  __device__ __forceinline__ bool evaluate(const Pre& p, Term& x) const {
     const R4 Aj = p.a;
     const R d0 = Ops::sub(xi[0], Aj.x), d1 = Ops::sub(xi[1], Aj.y);
     const R d2 = DIM == 3 ? Ops::sub(xi[2], Aj.z) : R(0);
     R r2 = Ops::add(Ops::mul(d0, d0), Ops::mul(d1, d1));
     if (DIM == 3) r2 = Ops::add(r2, Ops::mul(d2, d2));
     if (TEST) {
-      if (!(r2 < c.four_h2)) return;
-      if (!(r2 > R(0))) return;
+      if (!(r2 < c.four_h2)) return false;
+      if (!(r2 > R(0))) return false;
     }
     const R4 Bj = p.b;
     const R r = Ops::sqrt(r2);
@@ -293,16 +331,20 @@ struct RealPairs {
     R w = Ops::add(Ops::mul(dv0, d0), Ops::mul(dv1, d1));
     if (DIM == 3) w = Ops::add(w, Ops::mul(dv2, d2));
     const R mj = Aj.w;
-    if (kCont) dr = Ops::add(dr, Ops::mul(mj, Ops::mul(w, F)));
+    if (kCont) {
+      x.m = mj;
+      x.wF = Ops::mul(w, F);
+    }
     if (kMom) {
       const R2 qj = p.q;
       const R av = Ops::div(Ops::mul(c.avk, w), Ops::mul(Ops::add(r2, c.eps_h2), Ops::add(rhoi, qj.x)));
       const R pij = w < R(0) ? av : R(0);
-      const R coef = Ops::mul(mj, Ops::mul(Ops::add(Ops::add(Pi, qj.y), pij), F));
-      acc[0] = Ops::sub(acc[0], Ops::mul(coef, d0));
-      acc[1] = Ops::sub(acc[1], Ops::mul(coef, d1));
-      if (DIM == 3) acc[2] = Ops::sub(acc[2], Ops::mul(coef, d2));
+      x.coef = Ops::mul(mj, Ops::mul(Ops::add(Ops::add(Pi, qj.y), pij), F));
+      x.d[0] = d0;
+      x.d[1] = d1;
+      x.d[2] = d2;
     }
+    return true;
   }
 
   // Sum the partial sums of the LANES lanes of a slot (butterfly; every lane ends with the sum).
@@ -493,7 +535,11 @@ struct DfPairs {
 
   // What pair_with(t, q, p) adds, without adding it (sph_ordered_pass_kernel).
   static constexpr int kTerms = STAGE == SPH_MOM ? DIM : 1;
-  __device__ __forceinline__ void list_terms(uint32_t t, uint32_t q, const Pre& p, df (&out)[kTerms]) const {
+  struct Term {
+    df v[kTerms];
+  };
+  __device__ __forceinline__ void list_terms(uint32_t t, uint32_t q, const Pre& p, Term& x) const {
+    df(&out)[kTerms] = x.v;
     if constexpr (STAGE == SPH_MOM) {
       const df ncoef = momentum_coef(p.rp, df_make(p.fw.x, p.fw.y), df_make(p.fw.z, p.fw.w));
       out[0] = dfacc_term(ncoef, df_sub_close(xi[0], df_make(p.ah.x, p.al.x)));
@@ -510,8 +556,17 @@ struct DfPairs {
       out[0] = dfacc_term(G, wv);
     }
   }
-  __device__ __forceinline__ void add_term(int c, df term) {
-    dfacc_add_term(STAGE == SPH_MOM ? acc[c] : dr, term);
+  __device__ __forceinline__ void add_term(const Term& x) {
+#pragma unroll
+    for (int c = 0; c < kTerms; ++c) dfacc_add_term(STAGE == SPH_MOM ? acc[c] : dr, x.v[c]);
+  }
+  template <int LANES>
+  static __device__ __forceinline__ Term shuffle(const Term& x, int l) {
+    Term y;
+#pragma unroll
+    for (int c = 0; c < kTerms; ++c)
+      y.v[c] = df_make(__shfl_sync(0xffffffffu, x.v[c].hi, l, LANES), __shfl_sync(0xffffffffu, x.v[c].lo, l, LANES));
+    return y;
   }
   // any candidate (the walk that continues an overflowed list): everything computed here
   __device__ __forceinline__ void pair(uint32_t t) { terms<true>(t, 0, fetch_entry(t, 0, false)); }
@@ -635,18 +690,34 @@ PassKernel list_pass_for(int arith, int lanes) {
   }
 }
 
-// Threads per slot of the double-word passes of a handle of n particles with one thread per slot set:
-// more than one where one would leave schedulers idle (sph_ordered_pass_kernel).  Step in us, with 1 / 2 / 4
-// threads per slot: 2D dam break of 6,518 particles 36.7 / 31.1 / 29.2, of 13,518 39.5 / 35.1 / 33.4, of
-// 23,018 41.7 / 37.5 / 38.2, of 37,718 44.0 / 43.1 / 49.7; 3D lattice (half-size cells) of 5,000 particles
+// Threads per slot of the passes of a handle of n particles with one thread per slot set: more than one
+// where one would leave schedulers idle (sph_ordered_pass_kernel).  Step in us, with 1 / 2 / 4 threads
+// per slot, double-word: 2D dam break of 6,518 particles 36.7 / 31.1 / 29.2, of 13,518 39.5 / 35.1 / 33.4,
+// of 23,018 41.7 / 37.5 / 38.2, of 37,718 44.0 / 43.1 / 49.7; 3D lattice (half-size cells) of 5,000 particles
 // 89 / 72 / 61, of 10,000 90 / 73 / 69, of 20,000 91 / 84 / 86, of 30,000 101 / 99 / 109, of 45,000
-// 122 / 133 / 136.  (8 threads: 29.6 and 61.6 at the small ends, worse from there on.)
-int ordered_lanes(uint32_t n) { return n <= 16384 ? 4 : n <= 32768 ? 2 : 1; }
+// 122 / 133 / 136.  (8 threads: 29.6 and 61.6 at the small ends, worse from there on.)  The f32 pairs
+// are shorter, so the line lies higher: 3D lattice of 5,000 80 / 63 / 55, of 20,000 86 / 69 / 65, of 27,000
+// 89 / 74 / 72, of 33,000 89 / 75 / 77, of 45,000 95 / 85 / 95, of 60,000 101 / 96 / 105, of 80,000
+// 113 / 125 / 126 (IEEE f32 within 3 % of these).
+int ordered_lanes(int arith, uint32_t n) {
+  if (arith == ARITH_F64_DF) return n <= 16384 ? 4 : n <= 32768 ? 2 : 1;
+  return n <= 28672 ? 4 : n <= 57344 ? 2 : 1;
+}
 
-template <int DIM, int LANES>
-PassKernel ordered_kernel(int stage) {
-  return stage == SPH_CONT ? sph_ordered_pass_kernel<DfPairs<DIM, SPH_CONT>, DIM, LANES>
-                           : sph_ordered_pass_kernel<DfPairs<DIM, SPH_MOM>, DIM, LANES>;
+template <int DIM, int STAGE, int LANES>
+PassKernel ordered_kernel_for(int arith) {
+  switch (arith) {
+    case ARITH_F64_DF: return sph_ordered_pass_kernel<DfPairs<DIM, STAGE>, DIM, false, LANES>;
+    case ARITH_F32_EXACT: return sph_ordered_pass_kernel<RealPairs<OpsF, DIM, false, STAGE>, DIM, true, LANES>;
+    default: return sph_ordered_pass_kernel<RealPairs<OpsFF, DIM, false, STAGE>, DIM, true, LANES>;
+  }
+}
+
+template <int LANES>
+PassKernel ordered_kernel(int arith, int dim, int stage) {
+  if (dim == 2)
+    return stage == SPH_CONT ? ordered_kernel_for<2, SPH_CONT, LANES>(arith) : ordered_kernel_for<2, SPH_MOM, LANES>(arith);
+  return stage == SPH_CONT ? ordered_kernel_for<3, SPH_CONT, LANES>(arith) : ordered_kernel_for<3, SPH_MOM, LANES>(arith);
 }
 
 // The list kernel with the batch that suits the rows' length (see sph_list_kernel).
@@ -792,12 +863,10 @@ int launch_sph_list_exact(cudaStream_t st, const SphArgs& a, int grid, int block
 
 int launch_sph_list_pass(cudaStream_t st, const SphArgs& a, int arith, int stage, int grid, int block, int lanes) {
   lanes = sph_pass_lanes(arith, stage, lanes);
-  const int ordered = arith == ARITH_F64_DF && lanes == 1 && stage != SPH_RATES ? ordered_lanes(a.n) : 1;
-  if (ordered > 1) {
-    const PassKernel kern = ordered == 4 ? (a.dim == 2 ? ordered_kernel<2, 4>(stage) : ordered_kernel<3, 4>(stage))
-                                         : (a.dim == 2 ? ordered_kernel<2, 2>(stage) : ordered_kernel<3, 2>(stage));
-    return launch_table(st, a, kern, 0, block, ordered);  // one block per tile
-  }
+  const int ordered = arith != ARITH_F64_EXACT && lanes == 1 && stage != SPH_RATES ? ordered_lanes(arith, a.n) : 1;
+  if (ordered > 1)
+    return launch_table(st, a, ordered == 4 ? ordered_kernel<4>(arith, a.dim, stage) : ordered_kernel<2>(arith, a.dim, stage),
+                        0, block, ordered);  // one block per tile
   PassKernel kern = list_kernel(arith, a.dim, stage, lanes, a.reach);
   return launch_table(st, a, kern, grid, block, lanes);
 }

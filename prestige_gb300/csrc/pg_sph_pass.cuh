@@ -499,7 +499,7 @@ __global__ void __launch_bounds__(kSphMaxThreads) sph_list_pass_kernel(SphArgs a
 // lane that has them), so the sums are bit for bit those of one thread per slot.  What bounds such a
 // system is the chain of one thread's pairs, each a few hundred dependent instructions; the additions are
 // a tenth of them.  One block per tile.
-template <class Pairs, int DIM, int LANES>
+template <class Pairs, int DIM, bool EXACT_PF, int LANES>
 __global__ void __launch_bounds__(kSphMaxThreads) sph_ordered_pass_kernel(SphArgs a) {
   chain_begin();
   const uint32_t cap = a.cap, sub = threadIdx.x % LANES, spb = blockDim.x / LANES;
@@ -519,21 +519,18 @@ __global__ void __launch_bounds__(kSphMaxThreads) sph_ordered_pass_kernel(SphArg
   for (uint32_t q0 = 0; q0 < longest; q0 += LANES) {
     const uint32_t q = q0 + sub, tnn = at(q + 2 * LANES);
     const typename Pairs::Pre nxt = P.fetch(tn, q + LANES < L ? q + LANES : 0u);
-    df term[Pairs::kTerms];
-#pragma unroll
-    for (int c = 0; c < Pairs::kTerms; ++c) term[c] = df_make(0.f, 0.f);
+    typename Pairs::Term term = {};  // adds nothing
     if (q < L) P.list_terms(t, q, cur, term);
 #pragma unroll
-    for (int l = 0; l < LANES; ++l)
-#pragma unroll
-      for (int c = 0; c < Pairs::kTerms; ++c)
-        P.add_term(c, df_make(__shfl_sync(0xffffffffu, term[c].hi, l, LANES),
-                              __shfl_sync(0xffffffffu, term[c].lo, l, LANES)));
+    for (int l = 0; l < LANES; ++l) P.add_term(Pairs::template shuffle<LANES>(term, l));
     cur = nxt;
     t = tn;
     tn = tnn;
   }
-  if (cnt > cap && sub == 0) P.resume(a, k);  // rare: continue the candidate walk where the list stopped
+  if (cnt > cap && sub == 0) {  // rare: continue the candidate walk where the list stopped
+    if constexpr (ResumePolicy<Pairs>::value) P.resume(a, k);
+    else continue_walk<DIM, EXACT_PF>(a, k, [&](uint32_t tt) { P.pair(tt); });
+  }
   if (live && sub == 0) P.finish(a, K, id, k);
 }
 

@@ -1,7 +1,8 @@
-"""The double-word passes of small handles (2 or 4 threads per particle, the terms added in list order) give
-the bits of the general pass (one thread per particle): a system stepped alone against the same
-system in a batch too large for the small-handle passes.  Sizes at the edges of warps, blocks and of
-the rule (16384, 32768 particles), both dimensions, overflowing lists, isolated particles, graph replay."""
+"""The passes of small handles (2 or 4 threads per particle, the terms added in list order) give the bits
+of the general pass (one thread per particle): a system stepped alone against the same system in a
+batch too large for the small-handle passes.  Sizes at the edges of warps, blocks and of the rule
+(16384 and 32768 particles double-word, 28672 and 57344 in f32), both dimensions, overflowing lists,
+isolated particles, graph replay."""
 import numpy as np
 import pytest
 
@@ -14,7 +15,7 @@ FIELDS = ("pos", "vel", "rho", "mass")
 
 def _lattice(n, seed, **cfg):
     w = workloads.sph_lattice_3d(n=n, seed=seed)
-    return dict(w, config=dict(w["config"], precision=1, f64_mode=1, **cfg))
+    return dict(w, config={**w["config"], "precision": 1, "f64_mode": 1, **cfg})
 
 
 def _dam(n, seed, **cfg):
@@ -27,7 +28,7 @@ def _dam(n, seed, **cfg):
     if n > 40:
         f["pos"][33] = f["pos"][7]
         f["pos"][5] = [-50.0, 80.0]
-    return {"config": dict(w["config"], precision=1, f64_mode=1, n_fluid=n, **cfg), "n": n, "fields": f}
+    return {"config": {**w["config"], "precision": 1, "f64_mode": 1, "n_fluid": n, **cfg}, "n": n, "fields": f}
 
 
 CASES = [("lattice1", lambda: _lattice(1, 1)), ("lattice31", lambda: _lattice(31, 2)), ("lattice1003", lambda: _lattice(1003, 3)),
@@ -40,12 +41,26 @@ CASES = [("lattice1", lambda: _lattice(1, 1)), ("lattice31", lambda: _lattice(31
          ("dam17001", lambda: _dam(17001, 13)), ("dam900_overflow", lambda: _dam(900, 14, list_capacity=6))]
 
 
+F32_CASES = [c for c in CASES if "32768" not in c[0] and "17001" not in c[0]] + [
+    ("lattice28673", lambda: _lattice(28673, 15)), ("lattice57344", lambda: _lattice(57344, 16)),
+    ("dam30001", lambda: _dam(30001, 17))]
+
+
 @pytest.mark.parametrize("graph", [False, True])
 @pytest.mark.parametrize("name,make", CASES)
 def test_small_handles_give_the_bits_of_the_general_pass(pg, name, make, graph):
-    w = make()
-    cfg = dict(w["config"])
-    filler = _lattice(40000, 99) if cfg["dim"] == 3 else _dam(40000, 98)
+    _compare(make(), graph, precision=1, f64_mode=1)
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("name,make", F32_CASES)
+def test_small_f32_handles_give_the_bits_of_the_general_pass(pg, name, make, mode):
+    _compare(make(), False, precision=0, f64_mode=mode)
+
+
+def _compare(w, graph, **arith):
+    cfg = dict(w["config"], **arith)
+    filler = _lattice(60000, 99, **arith) if cfg["dim"] == 3 else _dam(60000, 98, **arith)
     alone = ParticleSystem(make_config(**cfg), w["n"])
     both = ParticleSystem.batch([cfg, dict(filler["config"], list_capacity=cfg.get("list_capacity", 0),
                                            cell_multiplier=cfg.get("cell_multiplier", 1.0))], [w["n"], filler["n"]])
