@@ -571,18 +571,23 @@ struct DfPairs {
   // any candidate (the walk that continues an overflowed list): everything computed here
   __device__ __forceinline__ void pair(uint32_t t) { terms<true>(t, 0, fetch_entry(t, 0, false)); }
 
-  // The continued walk of an overflowed list, summed apart (in the momentum pass from the full record: only
-  // this walk needs velocities) and added; summed into the pass's own state it slowed the loop over
-  // the list (4M particles, momentum pass 1.97 -> 2.7 ms).
+  // The continued walk of an overflowed list, by a policy of its own that takes the sums over and hands
+  // them back, so every term is added in walk order.  Walked in the pass's own state it slowed the
+  // loop over the list (4M particles, momentum pass 1.97 -> 2.7 ms).  The momentum pass evaluates
+  // the rates' terms: only they read velocities, from the full records.  The continuity pass
+  // reads no {rho, P}, which other threads (and the other continuity launch of the overlapped
+  // schedule) are replacing.
   static constexpr bool kResumeApart = kCacheF;
   __device__ __forceinline__ void resume(const SphArgs& a, uint32_t k) {
-    DfPairs<DIM, SPH_RATES> P;
+    DfPairs<DIM, STAGE == SPH_CONT ? SPH_CONT : SPH_RATES> P;
     P.begin(a, a.sys[sys_of_slot(a, a.sorted_id[k])], k);
-    continue_walk<DIM, false>(a, k, [&](uint32_t t) { P.pair(t); });
-    if (STAGE == SPH_CONT) dr = dfacc_add(dr, P.dr);
+    P.dr = dr;
 #pragma unroll
-    for (int cc = 0; cc < DIM; ++cc)
-      if (STAGE == SPH_MOM) acc[cc] = dfacc_add(acc[cc], P.acc[cc]);
+    for (int cc = 0; cc < 3; ++cc) P.acc[cc] = acc[cc];
+    continue_walk<DIM, false>(a, k, [&](uint32_t t) { P.pair(t); });
+    dr = P.dr;
+#pragma unroll
+    for (int cc = 0; cc < 3; ++cc) acc[cc] = P.acc[cc];
   }
 
   // Two list entries of the momentum pass at once, in packed arithmetic (the operations of momentum(), half a
