@@ -86,14 +86,15 @@ struct Screen {
 // Thresholds for a decision in f64 (or by a superset): inside for certain below thr_lo, outside for
 // certain from thr on.  Every r^2 in [thr_lo, thr) has |r^2 / mid - 1| <= w, with the rounding of
 // 1 / mid and of the FMA added to w, hence r^2 |s| <= thr w = tol; and where r^2 |s| > tol, r^2 is
-// not zero and either lies beyond thr (s > 0) or has |s| > w.
+// not zero and either lies beyond thr (s > 0) or has |s| > w.  Where a square, the middle or its
+// reciprocal may leave the normal FP32 range, every candidate is left undecided.
 __device__ __forceinline__ void screen_band(Screen& s, float thr_lo, float thr) {
   const float mid = 0.5f * (thr_lo + thr);
   const float inv = 1.0f / mid;
   const float w = 0.5f * (thr - thr_lo) * inv + 4.76837158203125e-07f;  // + 8u
   s.a = f2_dup(inv);
   s.b = f2_dup(-1.0f);
-  s.tol = thr * w * 1.00001f;
+  s.tol = thr > 1e-30f && thr < 1e37f ? thr * w * 1.00001f : __int_as_float(0x7f800000);
 }
 
 // Threshold compared exactly (IEEE r^2 < thr); only r^2 = 0 (or an underflow) is left undecided.

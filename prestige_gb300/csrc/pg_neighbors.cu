@@ -285,9 +285,7 @@ __device__ __forceinline__ void for_each_hit(const NbrArgs& a, const GridK& g, u
   screen_target(S, pf);
   if (F64) {
     const float reach = g.support_f * 1.0000001f;
-    const float thr = outer_threshold(reach, pf);
-    screen_band(S, inner_threshold(reach, pf), thr);
-    if (!(thr > 1e-30f && thr < 1e37f)) S.tol = __int_as_float(0x7f800000);  // every candidate open
+    screen_band(S, inner_threshold(reach, pf), outer_threshold(reach, pf));
   } else {
     screen_exact(S, (float)s2);
   }
