@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(kDemThreads) dem_pass_kernel(DemArgs a) {
     auto row_range = [&](int z, int y, uint32_t& b, uint32_t& e) {
       b = e = 0;
       if (z >= 0 && z < g.nz && y >= 0 && y < g.ny) {
-        const uint32_t rb = g.cell_base + ((uint32_t)z * g.ny + (uint32_t)y) * g.nx;
+        const uint32_t rb = row_base(g, y, z);
         b = a.cell_start[rb + x0];
         e = a.cell_start[rb + x1 + 1];
       }

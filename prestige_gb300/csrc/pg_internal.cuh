@@ -124,6 +124,12 @@ struct GridK {
 };
 GridK grid_k(const Grid& g, uint32_t cell_base);
 
+// Index of the first cell of row (y, z).  Unsigned: a grid may have almost 2^32 cells, and the walks form the
+// bases of rows outside the grid too (such a value wraps and is not read).
+__host__ __device__ __forceinline__ uint32_t row_base(const GridK& g, int y, int z) {
+  return g.cell_base + ((uint32_t)z * (uint32_t)g.ny + (uint32_t)y) * (uint32_t)g.nx;
+}
+
 // ---------------------------------------------------------------------------------------
 // Neighbour-search workspace: stable counting sort of the particles by cell, and the cell table
 // (pg_sort.cu).

@@ -302,7 +302,7 @@ __device__ __forceinline__ void for_each_hit(const NbrArgs& a, const GridK& g, u
     for (int dy = -R1; dy <= R1; ++dy) {
       const int y = cy + dy;
       if (y < 0 || y >= g.ny) continue;
-      const uint32_t rb = g.cell_base + ((uint32_t)z * g.ny + (uint32_t)y) * g.nx;
+      const uint32_t rb = row_base(g, y, z);
       const uint32_t s = a.cell_start[rb + x0], e = a.cell_start[rb + x1 + 1];
       if (s >= e) continue;
       unsigned valid = kAll >> (s & 3u);

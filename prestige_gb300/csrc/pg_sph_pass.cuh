@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(kSphMaxThreads) sph_list_kernel(SphArgs a) {
     // uniform; a row outside the grid is empty).  tn, en: the slot range of row `row + 1`.
     uint32_t tn = 0, en = 0;
     int y = T.cy - R, z = T.cz - RZ;
-    uint32_t rb = g.cell_base + (uint32_t)((z * g.ny + y) * g.nx);  // wraps below 0 outside the grid (not read)
+    uint32_t rb = row_base(g, y, z);
     auto load_range = [&]() {
       tn = en = 0;
       if (T.live && (unsigned)y < (unsigned)g.ny && (unsigned)z < (unsigned)g.nz) {
@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(kSphMaxThreads) sph_list_kernel(SphArgs a) {
         if (++y > T.cy + R) {
           y = T.cy - R;
           ++z;
-          rb += (uint32_t)((g.ny - 2 * R) * g.nx);
+          rb += ((uint32_t)g.ny - 2u * (uint32_t)R) * (uint32_t)g.nx;
         } else {
           rb += (uint32_t)g.nx;
         }
@@ -381,7 +381,7 @@ __device__ __forceinline__ void continue_walk(const SphArgs& a, uint32_t k, Fn&&
   for (int row = row0; row < nrows; ++row) {
     const int z = T.cz + row / side - RZ, y = T.cy + row % side - R;
     if (z < 0 || z >= g.nz || y < 0 || y >= g.ny) continue;
-    const uint32_t rb = g.cell_base + ((uint32_t)z * g.ny + (uint32_t)y) * g.nx;
+    const uint32_t rb = row_base(g, y, z);
     const uint32_t e = a.cell_start[rb + T.x1 + 1];
     for (uint32_t t = row == row0 ? t0 : a.cell_start[rb + T.x0]; t < e; ++t)
       if (prefilter_hit<DIM, EXACT_PF>(pi, pf_at<DIM>(a.pf, t), thr)) fn(t);
