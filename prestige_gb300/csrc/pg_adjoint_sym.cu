@@ -218,9 +218,8 @@ struct Slot {
 
 template <int LANES>
 __device__ __forceinline__ bool slot_of(const SphArgs& a, Slot<LANES>& s) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  s.k = i / LANES;
-  s.sub = i % LANES;
+  s.k = lane_slot<LANES>(blockIdx.x, blockDim.x, threadIdx.x);
+  s.sub = threadIdx.x % LANES;
   if (s.k >= a.n) return false;
   s.id = a.sorted_id[s.k];
   const uint32_t cnt = a.nlen[s.k];

@@ -130,6 +130,13 @@ __host__ __device__ __forceinline__ uint32_t row_base(const GridK& g, int y, int
   return g.cell_base + ((uint32_t)z * (uint32_t)g.ny + (uint32_t)y) * (uint32_t)g.nx;
 }
 
+// The slot (from 0) of a thread where LANES consecutive threads share one (block: a multiple of LANES).  Not
+// the thread's number in the grid divided by LANES: that number has 34 bits at 2^32 slots.
+template <int LANES>
+__host__ __device__ __forceinline__ uint32_t lane_slot(uint32_t block_id, uint32_t block, uint32_t thread) {
+  return block_id * (block / LANES) + thread / LANES;
+}
+
 // ---------------------------------------------------------------------------------------
 // Neighbour-search workspace: stable counting sort of the particles by cell, and the cell table
 // (pg_sort.cu).

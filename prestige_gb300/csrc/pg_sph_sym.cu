@@ -163,9 +163,8 @@ struct Slot {
 
 template <int LANES = 1>
 __device__ __forceinline__ bool slot_of(const SphArgs& a, Slot& s) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  s.k = a.k_begin + i / LANES;
-  s.sub = i % LANES;
+  s.k = a.k_begin + lane_slot<LANES>(blockIdx.x, blockDim.x, threadIdx.x);
+  s.sub = threadIdx.x % LANES;
   if (s.k >= a.k_end) return false;
   s.id = a.sorted_id[s.k];
   const uint32_t cnt = a.nlen[s.k];
