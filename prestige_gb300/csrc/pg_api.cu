@@ -481,7 +481,7 @@ int enqueue_step(pg_system* s, bool chained) {
   if (s->model == PG_MODEL_DEM) {
     if (!ev && s->graph_enabled && s->graph_exec[s->hcur]) {
       PG_CUDA_TRY(cudaGraphLaunch(s->graph_exec[s->hcur], s->stream));
-      s->launches += neighbor_launches(s) + 2;
+      s->launches += s->graph_launches;
     } else {
       PG_TRY(enqueue_dem_step(s, ev, chained));
     }
@@ -490,7 +490,7 @@ int enqueue_step(pg_system* s, bool chained) {
   }
   if (!ev && s->graph_enabled && s->graph_exec[0]) {
     PG_CUDA_TRY(cudaGraphLaunch(s->graph_exec[0], s->stream));
-    s->launches += neighbor_launches(s) + 4;
+    s->launches += s->graph_launches;
     return PG_OK;
   }
   return enqueue_sph_step(s, false, 1, ev, chained);
@@ -504,7 +504,7 @@ int enqueue_steps(pg_system* s, int nsteps) {
     PG_TRY(rest_neighbors(s));
     for (; i + kGraphSteps <= nsteps; i += kGraphSteps) {
       PG_CUDA_TRY(cudaGraphLaunch(s->graph_steps[g], s->stream));
-      s->launches += kGraphSteps * (neighbor_launches(s) + (s->model == PG_MODEL_DEM ? 2 : 4));
+      s->launches += kGraphSteps * s->graph_launches;
     }
   }
   for (int first = i; i < nsteps; ++i) PG_TRY(enqueue_step(s, i > first));
@@ -558,6 +558,7 @@ int capture_steps(pg_system* s, int steps, cudaGraphExec_t* out) {
     }
   }
   s->hcur = hsave;
+  s->graph_launches = (s->launches - l0) / steps;
   s->launches = l0;
   cudaError_t ce = cudaStreamEndCapture(s->stream, &graph);
   if (st != PG_OK) {

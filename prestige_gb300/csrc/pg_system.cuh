@@ -89,6 +89,7 @@ struct pg_system {
   int list_arith = -1;  // arithmetic mode of the pair lists in nlist/nlen (-1: none built yet)
   cudaGraphExec_t graph_exec[2] = {nullptr, nullptr};   // one step (DEM: per history buffer)
   cudaGraphExec_t graph_steps[2] = {nullptr, nullptr};  // kGraphSteps steps
+  long long graph_launches = 0;                         // kernels of one captured step
 
   // step timing (pg_timing_enable): 4 events per step, consumed by pg_timing_read
   bool timing = false;
