@@ -85,7 +85,7 @@ typedef struct pg_info {
   long long n_cells;  /* all systems */
   int reach;          /* neighbour cells searched on each side */
   int pass_grid;      /* blocks of the persistent pair pass */
-  int sort_passes;    /* 8-bit digits of a cell index */
+  int sort_passes;    /* 8-bit radix passes per neighbour search (dense grids; 0: counting sort) */
   int graph;          /* 1 if steps replay a CUDA graph */
   int grid_n[3];      /* system 0 */
   double grid_lo[3];

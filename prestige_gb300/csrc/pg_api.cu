@@ -247,8 +247,7 @@ int enqueue_neighbors(pg_system* s, bool chained) {
 
 int mom_block(const pg_system* s) { return s->block_mom > 0 ? s->block_mom : s->block; }
 
-// Kernels enqueued by one neighbour search (hash, reduce, scan, scatter).
-long long neighbor_launches(const pg_system* s) { return s->nw.chunks > 1 ? 4 : 3; }
+long long neighbor_launches(const pg_system* s) { return s->nw.launches(); }
 
 // The continuity part of a step: neighbour search, sorted gather, neighbour lists and the
 // continuity pass (rho' into the canonical density and the sorted pack).  ev (optional): events
@@ -1599,7 +1598,7 @@ int pg_get_info(pg_system* s, pg_info* info) {
   info->n_cells = (long long)s->ncells;
   info->reach = s->grids[0].reach;
   info->pass_grid = s->pass_grid[SPH_MOM];
-  info->sort_passes = s->nw.passes;
+  info->sort_passes = s->nw.radix ? s->nw.passes : 0;
   for (int d = 0; d < 3; ++d) {
     info->grid_n[d] = s->grids[0].n[d];
     info->grid_lo[d] = s->grids[0].lo[d];

@@ -138,60 +138,111 @@ __host__ __device__ __forceinline__ uint32_t lane_slot(uint32_t block_id, uint32
 }
 
 // ---------------------------------------------------------------------------------------
-// Neighbour-search workspace: stable counting sort of the particles by cell, and the cell table
-// (pg_sort.cu).
+// Neighbour-search workspace: stable sort of the particles by cell, and the cell table (pg_sort.cu).
 // ---------------------------------------------------------------------------------------
 constexpr uint32_t kScanChunk = 8192;  // cells per block of the scan
-constexpr uint32_t kBigCell = 1024;    // particles of a cell that one block sorts (see pg_sort.cu)
+constexpr uint32_t kBigCell = 1024;    // larger cells are ranked by tiles of ids (see pg_sort.cu)
+constexpr uint32_t kMaxTiles = 1024;
+
+// What the hash gives the sort beside the cells.
+enum HashMode {
+  HASH_COUNT,         // counting sort: arrival ranks, an atomic per particle
+  HASH_COUNT_MERGED,  // the same, one atomic for a warp's particles of a cell
+  HASH_IDS,           // radix sort: ids
+};
 
 struct NbrWork {
   size_t n = 0;
   uint64_t ncells = 0;
+  HashMode mode = HASH_COUNT;
+  bool radix = false;  // mode == HASH_IDS
   int passes = 0;      // 8-bit digits of a cell index
-  uint32_t chunks = 0; // scan chunks: cover ncells + 1 entries
   DevBuf mem;          // all arrays below
-  uint32_t *key = nullptr, *rank = nullptr, *unsorted = nullptr;  // [n] cell and arrival rank of each id; ids by cell
-  uint32_t *sorted_cell = nullptr, *sorted_id = nullptr;          // [n] cell and id of each sorted slot
-  uint32_t* cell_start = nullptr;   // [ncells + 1], padded to whole chunks
+  uint32_t *sorted_cell = nullptr, *sorted_id = nullptr;  // [n] cell and id of each sorted slot
+  uint32_t* cell_start = nullptr;                         // [ncells + 1], padded to whole chunks
+  uint32_t *key = nullptr, *rank = nullptr;  // [n] cell and arrival rank of each id (radix: cells and ids to sort)
+  // counting sort
+  uint32_t chunks = 0;              // scan chunks: cover ncells + 1 entries
+  uint32_t* unsorted = nullptr;     // [n] ids by cell
   uint32_t* chunk_total = nullptr;  // [chunks] particles per chunk
+  uint32_t* tile_count = nullptr;   // cells of more than kBigCell: rows of tile_row words (see pg_sort.cu)
+  uint32_t tile_fine = 0, tile_row = 0;
+  int tile_shift = 0;               // log2 of the ids per tile
   uint32_t* rest = nullptr;         // the arrays that are zero between searches, rest_words in all:
   uint32_t* count = nullptr;        //   [chunks * kScanChunk] particles per cell
-  uint32_t* big = nullptr;          //   {cells listed, blocks done, cell indices ...}
+  uint32_t* big = nullptr;          //   {1 where a cell holds more than kBigCell, blocks done}
   size_t rest_words = 0;
+  // radix sort
+  uint32_t *key2 = nullptr, *id2 = nullptr;  // [n]
+  uint32_t *hist = nullptr, *digit_total = nullptr;
+  int tiles = 0;
+
   bool clean = false;  // count, big and the position minima hold their rest values
   int init(size_t n, uint64_t ncells);
   size_t bytes() const;
+  int launches() const { return radix ? 2 + 3 * passes : chunks > 1 ? 4 : 3; }  // of one search
 };
 
 // What a sorted-gather kernel needs to finish the sort: ordered_slot() gives each thread the particle
 // and the final slot of one entry of `unsorted`, and records both.
 struct NbrOrder {
   const uint32_t* unsorted;
-  const uint32_t* key;
+  const uint32_t* key;  // null: sorted already, `unsorted` being sorted_id
   const uint32_t* cell_start;
   uint32_t* sorted_cell;
   uint32_t* sorted_id;
+  const uint32_t* rank;
+  const uint32_t* tile_count;
+  uint32_t tile_fine, tile_row;
+  int tile_shift;
 };
 NbrOrder nbr_order(const NbrWork& w);
 
+// Members of a cell (slots [b, e), more than 32) with smaller ids: counted four ids a load, or in cells of more
+// than kBigCell the id's rank in its tile plus the counts of the tiles before (pg_sort.cu).  Out of
+// line, so the gathers of ordinary cells do not hold it.
+static __device__ __noinline__ uint32_t large_cell_rank(const uint32_t* unsorted, const uint32_t* rank,
+                                                        const uint32_t* tile_count, uint32_t tile_fine,
+                                                        uint32_t tile_row, int tile_shift, uint32_t id, uint32_t b,
+                                                        uint32_t e) {
+  uint32_t k = 0;
+  if (e - b <= kBigCell) {
+    uint32_t q = b;
+    for (; q & 3u; ++q) k += unsorted[q] < id ? 1u : 0u;
+    for (; q + 4 <= e; q += 4) {  // four ids a load
+      const uint4 v = *(const uint4*)(unsorted + q);
+      k += (v.x < id ? 1u : 0u) + (v.y < id ? 1u : 0u) + (v.z < id ? 1u : 0u) + (v.w < id ? 1u : 0u);
+    }
+    for (; q < e; ++q) k += unsorted[q] < id ? 1u : 0u;
+    return k;
+  }
+  k = rank[id];
+  const uint32_t* row = tile_count + (size_t)(b / kBigCell) * tile_row;
+  const uint32_t tile = id >> tile_shift;
+  for (uint32_t g = 0; g < tile / 32; ++g) k += row[tile_fine + g];
+  for (uint32_t t = tile & ~31u; t < tile; ++t) k += row[t];
+  return k;
+}
+
 // Within a cell the scatter left the ids in arrival order: an id's slot is the cell's first plus the
-// number of smaller ids in the cell, so equal cells end up in id order (the stable order).  Cells of
-// more than kBigCell particles are in id order already.
+// number of smaller ids in the cell, so equal cells end up in id order (the stable order).
 __device__ __forceinline__ uint32_t ordered_slot(const NbrOrder& o, uint32_t s, uint32_t& id) {
   id = o.unsorted[s];
+  if (!o.key) return s;
   const uint32_t c = o.key[id];
   const uint32_t b = o.cell_start[c], e = o.cell_start[c + 1];
-  uint32_t k = s;
-  if (e - b <= kBigCell) {
-    k = b;
+  uint32_t k = b;
+  if (e - b <= 32)
     for (uint32_t q = b; q < e; ++q) k += o.unsorted[q] < id ? 1u : 0u;
-  }
+  else
+    k += large_cell_rank(o.unsorted, o.rank, o.tile_count, o.tile_fine, o.tile_row, o.tile_shift, id, b, e);
   o.sorted_id[k] = id;
   o.sorted_cell[k] = c;
   return k;
 }
 
-// Cell of every particle (id order) with its arrival rank in the cell, counted into w.count.
+// Cell of every particle (id order) with its arrival rank in the cell, counted into w.count (radix sort:
+// with its id).
 // posmin (optional, f64 positions only): per system and dimension ([3 sys + d]) the minimum
 // position, as ordered_code values, folded in with atomicMin (all ones before).
 // chained: directly after another kernel of the stream.
@@ -206,7 +257,7 @@ __device__ __forceinline__ unsigned long long ordered_code(double x) {
 __device__ __forceinline__ double ordered_value(unsigned long long u) {
   return __longlong_as_double((long long)((u >> 63) ? (u & 0x7fffffffffffffffull) : ~u));
 }
-// Cell table and the ids grouped by cell, from launch_hash's counts; the sorted gather that follows
+// Cell table and the ids grouped by cell, from launch_hash's arrays; the sorted gather that follows
 // orders the ids within each cell (ordered_slot).  nmin position minima move from minacc to minout
 // (both optional), minacc going back to all ones.
 int launch_sort(cudaStream_t st, NbrWork& w, unsigned long long* minacc, unsigned long long* minout, uint32_t nmin);

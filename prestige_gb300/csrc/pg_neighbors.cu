@@ -164,11 +164,11 @@ __device__ __forceinline__ void fold_min(unsigned long long* p, unsigned long lo
   if (v < *(volatile unsigned long long*)p) atomicMin(p, v);
 }
 
-// Cell and arrival rank of every particle (pg_sort.cu).  MIN: also the minimum position per system
-// and dimension (posmin[3 sys + d]): a block reduction and one fold per block and dimension
-// (blockDim.x == 256), or one per particle where a block spans systems of a batch (ids are
-// contiguous per system).
-template <class R, int DIM, bool MIN>
+// Cell of every particle, and by MODE (HashMode, pg_internal.cuh) its arrival rank in the cell or its id.
+// MIN: also the minimum position per system and dimension (posmin[3 sys + d]): a block reduction
+// and one fold per block and dimension (blockDim.x == 256), or one per particle where a block
+// spans systems of a batch (ids are contiguous per system).
+template <class R, int DIM, bool MIN, int MODE>
 __global__ void hash_kernel(const GridK* __restrict__ grid, const uint32_t* __restrict__ sys_of_id,
                             const R* __restrict__ pos, uint32_t n, uint32_t* __restrict__ keys,
                             uint32_t* __restrict__ rank, uint32_t* __restrict__ count,
@@ -177,6 +177,7 @@ __global__ void hash_kernel(const GridK* __restrict__ grid, const uint32_t* __re
   chain_begin();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   unsigned long long m[3] = {~0ull, ~0ull, ~0ull};
+  uint32_t key = 0xffffffffu;  // (no cell: a grid has fewer)
   if (i < n) {
     const GridK& g = grid[sys_of_id ? sys_of_id[i] : 0u];
     int c[3] = {0, 0, 0};
@@ -188,12 +189,20 @@ __global__ void hash_kernel(const GridK* __restrict__ grid, const uint32_t* __re
       else c[d] = cell_coord_f((float)x, g.lof[d], g.invf, nn[d]);
       if (MIN) m[d] = ordered_code((double)x);
     }
-    const uint32_t key =
-        g.cell_base + ((uint32_t)c[2] * (uint32_t)g.ny + (uint32_t)c[1]) * (uint32_t)g.nx + (uint32_t)c[0];
+    key = row_base(g, c[1], c[2]) + (uint32_t)c[0];
     keys[i] = key;
-    const uint32_t r = atomicAdd(count + key, 1u);
+  }
+  uint32_t r = i;
+  if (MODE == HASH_COUNT_MERGED) {
+    const unsigned peers = __match_any_sync(0xffffffffu, key), lane = threadIdx.x & 31, leader = __ffs(peers) - 1;
+    if (i < n && lane == leader) r = atomicAdd(count + key, (uint32_t)__popc(peers));
+    r = __shfl_sync(0xffffffffu, r, leader) + __popc(peers & ((1u << lane) - 1u));
+  } else if (MODE == HASH_COUNT && i < n) {
+    r = atomicAdd(count + key, 1u);
+  }
+  if (i < n) {
     rank[i] = r;
-    if (r == kBigCell) big[2 + atomicAdd(big, 1u)] = key;  // one thread per cell that large
+    if (MODE != HASH_IDS && r == kBigCell) *big = 1u;
   }
   if (MIN) {
     // the block's particles belong to one system unless its id range spans a boundary
@@ -376,13 +385,23 @@ inline unsigned blocks_for(size_t n, int t) { return (unsigned)((n + t - 1) / t)
 
 }  // namespace
 
+template <class R, int DIM, int MODE>
+static cudaError_t hash_mode(cudaStream_t st, bool chained, const GridK* grid, const uint32_t* sys_of_id,
+                             const void* pos, NbrWork& w, unsigned long long* posmin) {
+  const bool min = sizeof(R) == 8 && posmin;
+  return launch_chained(st, chained, min ? hash_kernel<R, DIM, sizeof(R) == 8, MODE> : hash_kernel<R, DIM, false, MODE>,
+                        blocks_for(w.n, 256), 256, grid, sys_of_id, (const R*)pos, (uint32_t)w.n, w.key, w.rank,
+                        w.count, w.big, min ? posmin : nullptr);
+}
+
 template <class R, int DIM>
 static cudaError_t hash_dim(cudaStream_t st, bool chained, const GridK* grid, const uint32_t* sys_of_id, const void* pos,
                             NbrWork& w, unsigned long long* posmin) {
-  const bool min = sizeof(R) == 8 && posmin;
-  return launch_chained(st, chained, min ? hash_kernel<R, DIM, true> : hash_kernel<R, DIM, false>, blocks_for(w.n, 256),
-                        256, grid, sys_of_id, (const R*)pos, (uint32_t)w.n, w.key, w.rank, w.count, w.big,
-                        min ? posmin : nullptr);
+  switch (w.mode) {
+    case HASH_COUNT: return hash_mode<R, DIM, HASH_COUNT>(st, chained, grid, sys_of_id, pos, w, posmin);
+    case HASH_COUNT_MERGED: return hash_mode<R, DIM, HASH_COUNT_MERGED>(st, chained, grid, sys_of_id, pos, w, posmin);
+    default: return hash_mode<R, DIM, HASH_IDS>(st, chained, grid, sys_of_id, pos, w, posmin);
+  }
 }
 
 int launch_hash(cudaStream_t st, bool chained, const GridK* grid_dev, const uint32_t* sys_of_id, int f64, int dim,

@@ -15,15 +15,20 @@
 //   cell_scan    cell_start = exclusive scan of the counts: a block per chunk, its base the sum of
 //                the totals of the chunks before it; the counts go back to zero for the next search
 //   cell_scatter id -> slot cell_start[cell] + rank, so ids are grouped by cell in arrival order
-//   the gather   ranks each id among the few ids of its cell (ordered_slot): the stable order
+//   the gather   ranks each id among the ids of its cell (ordered_slot): the stable order
 // It is bound by the latency of these few launches below about 1M particles and by the scattered
-// 4-byte writes and atomics above.  It replaced an LSD radix sort by 8-bit digits with a binary search
-// per cell for the table (3 launches per digit, 8 to 11 in all).  Search plus gather, ms, before and
-// after: 6.5k particles 0.049 / 0.025, 200k spheres 0.085 / 0.045, 262k 0.082 / 0.041, 700k f32
+// 4-byte writes and atomics above.  Search plus gather, ms, by the radix sort below and by this one:
+// 6.5k particles 0.049 / 0.025, 200k spheres 0.085 / 0.045, 262k 0.082 / 0.041, 700k f32
 // 0.073 / 0.050, 4M 0.409 / 0.254, 6.1M in 512 systems 0.589 / 0.401.
+//
+// Ranking an id among the m ids of its cell takes the gather m reads.  Cells of more than kBigCell
+// particles take counts per tile of consecutive ids instead: rank = rank within the tile + the counts of
+// the tiles before (rank_big_cells, large_cell_rank).  Search of 1M particles in 100 of 10,000 cells 0.35 ms; one
+// block that sorts such cells one after the other takes 8.5, the radix sort about 0.1.  Dense grids take an LSD radix sort (sort_mode).
 #include <cuda_runtime.h>
 
 #include <mutex>
+#include <utility>
 
 #include "pg_internal.cuh"
 
@@ -224,6 +229,26 @@ __global__ void __launch_bounds__(kSortThreads) digit_scatter_kernel(
   }
 }
 
+// cell_start[c] = first sorted slot whose cell is >= c, for c = 0 .. ncells (so cell_start[ncells]
+// = n), by a binary search over the sorted cells.  The position minima move as in cell_scan_kernel.
+__global__ void cell_start_kernel(const uint32_t* __restrict__ cell, uint32_t n, uint32_t ncells,
+                                  uint32_t* __restrict__ start, unsigned long long* minacc,
+                                  unsigned long long* minout, uint32_t nmin) {
+  const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+  for (uint32_t i = c; i < nmin; i += gridDim.x * blockDim.x) {
+    minout[i] = minacc[i];
+    minacc[i] = ~0ull;
+  }
+  if (c > ncells) return;
+  uint32_t lo = 0, hi = n;
+  while (lo < hi) {
+    const uint32_t mid = lo + (hi - lo) / 2;
+    if (__ldg(cell + mid) < c) lo = mid + 1;
+    else hi = mid;
+  }
+  start[c] = lo;
+}
+
 // ---------------------------------------------------------------------------------------
 // Counting sort.
 // ---------------------------------------------------------------------------------------
@@ -244,7 +269,8 @@ __global__ void __launch_bounds__(kCellScanThreads) cell_reduce_kernel(const uin
 __global__ void __launch_bounds__(kCellScanThreads) cell_scan_kernel(uint32_t* __restrict__ count,
                                                                      const uint32_t* __restrict__ chunk_total,
                                                                      uint32_t* __restrict__ start,
-                                                                     unsigned long long* minacc,
+                                                                     uint32_t* __restrict__ tile_count,
+                                                                     uint32_t tile_row, unsigned long long* minacc,
                                                                      unsigned long long* minout, uint32_t nmin) {
   __shared__ uint32_t base;
   chain_begin();
@@ -272,6 +298,15 @@ __global__ void __launch_bounds__(kCellScanThreads) cell_scan_kernel(uint32_t* _
   uint4* sp = (uint4*)(start + (size_t)blockIdx.x * kScanChunk) + 2 * tid;
   sp[0] = o;
   sp[1] = p;
+  if ((a.x | a.y | a.z | a.w | b.x | b.y | b.z | b.w) > kBigCell) {  // (at least their maximum)
+    const uint32_t m[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w}, first[8] = {o.x, o.y, o.z, o.w, p.x, p.y, p.z, p.w};
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (m[i] > kBigCell) {
+        uint4* row = (uint4*)(tile_count + (size_t)(first[i] / kBigCell) * tile_row);
+        for (uint32_t w = 0; w < tile_row / 4; ++w) row[w] = make_uint4(0, 0, 0, 0);
+      }
+  }
   if (blockIdx.x == 0)
     for (uint32_t i = tid; i < nmin; i += kCellScanThreads) {
       minout[i] = minacc[i];
@@ -279,82 +314,71 @@ __global__ void __launch_bounds__(kCellScanThreads) cell_scan_kernel(uint32_t* _
     }
 }
 
-// Sort the m distinct ids of one cell ascending, by one block of kSortThreads threads: LSD radix by
-// 8-bit digits, tile after tile, between ids and tmp (m values each).
-__device__ __noinline__ void sort_segment(uint32_t* ids, uint32_t* tmp, uint32_t m, int bits) {
-  __shared__ uint32_t wcnt[kSortWarps][kRadix];
-  __shared__ uint32_t next[kRadix];  // next free position of each digit
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  uint32_t *src = ids, *dst = tmp;
-  for (int shift = 0; shift < bits; shift += 8) {
-    next[tid] = 0;
-    __syncthreads();
-    for (uint32_t i = tid; i < m; i += kSortThreads) atomicAdd(&next[(src[i] >> shift) & 0xffu], 1u);
-    __syncthreads();
-    uint32_t total;
-    const uint32_t first = block_excl_scan(next[tid], &total);
-    next[tid] = first;
-    __syncthreads();
-    for (uint32_t t0 = 0; t0 < m; t0 += kSortThreads) {
-#pragma unroll
-      for (int w = 0; w < kSortWarps; ++w) wcnt[w][tid] = 0;
-      __syncthreads();
-      const uint32_t i = t0 + tid;
-      const bool valid = i < m;
-      const uint32_t v = valid ? src[i] : 0u;
-      const uint32_t d = valid ? ((v >> shift) & 0xffu) : 0x100u;
-      const uint32_t peers = __match_any_sync(0xffffffffu, d);
-      const uint32_t below = __popc(peers & ((1u << lane) - 1u));
-      if (valid && below == 0) wcnt[warp][d] = __popc(peers);
-      __syncthreads();
-      uint32_t run = next[tid];  // per digit: positions of the warps' runs
-#pragma unroll
-      for (int w = 0; w < kSortWarps; ++w) {
-        const uint32_t c = wcnt[w][tid];
-        wcnt[w][tid] = run;
-        run += c;
-      }
-      next[tid] = run;
-      __syncthreads();
-      if (valid) dst[wcnt[warp][d] + below] = v;
-      __syncthreads();
+// The ids of cells of more than kBigCell particles, one warp per tile of consecutive ids: to their cell's
+// slots in arrival order like the others; the rank of each within its cell and tile replaces its arrival rank,
+// and the row of its cell gets the tile's count and the count of the tile's group of 32.  (A cell that
+// large has its first slot in a block of kBigCell slots of its own, which numbers the rows.)
+__device__ __noinline__ void rank_big_cells(const uint32_t* __restrict__ key, uint32_t* rank,
+                                            const uint32_t* __restrict__ start, uint32_t n, uint32_t* unsorted,
+                                            uint32_t* tile_count, uint32_t tile_fine, uint32_t tile_row,
+                                            int tile_shift) {
+  const uint32_t tile = blockIdx.x * kSortWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (tile > (n - 1) >> tile_shift) return;
+  const uint32_t i0 = tile << tile_shift, len = min(1u << tile_shift, n - i0);
+  uint32_t b = 0, m = 0, r = 0;  // of this round's id: the cell's first slot and size, the arrival rank
+  auto load = [&](uint32_t j) {
+    m = 0;
+    if (j < len) {
+      const uint32_t c = key[i0 + j];
+      b = start[c];
+      m = start[c + 1] - b;
+      r = rank[i0 + j];
     }
-    uint32_t* t = src;
-    src = dst;
-    dst = t;
-  }
-  if (src != ids) {
-    for (uint32_t i = tid; i < m; i += kSortThreads) ids[i] = src[i];
-    __syncthreads();
+  };
+  load(lane);
+  for (uint32_t j0 = 0; j0 < len; j0 += 32) {
+    const uint32_t b0 = b, r0 = r, i = i0 + j0 + lane;
+    const bool big = m > kBigCell;
+    load(j0 + 32 + lane);  // the next round's, while this one's count is read
+    const unsigned peers = __match_any_sync(0xffffffffu, big ? b0 / kBigCell : 0xffffffffu);
+    if (big) {
+      uint32_t* row = tile_count + (size_t)(b0 / kBigCell) * tile_row;
+      const int leader = __ffs(peers) - 1;
+      uint32_t before = 0;
+      if (lane == (uint32_t)leader) {
+        before = row[tile];  // (only this warp writes the tile's counts)
+        row[tile] = before + __popc(peers);
+        atomicAdd(row + tile_fine + tile / 32, (uint32_t)__popc(peers));
+      }
+      rank[i] = __shfl_sync(peers, before, leader) + __popc(peers & ((1u << lane) - 1u));
+      unsorted[b0 + r0] = i;
+    }
+    __syncwarp();  // the counts, for the next round's leaders
   }
 }
 
-// ids to their cell's slots in arrival order.  Ranking an id among the ids of its cell costs the gather
-// as many reads as the cell holds, so the cells of more than kBigCell particles (a degenerate
-// distribution: the hash listed them) are sorted here, by the block that finishes last; it waits
-// for nothing, and a search without such cells has no last block.
+// ids to their cell's slots in arrival order.
 __global__ void __launch_bounds__(kSortThreads) cell_scatter_kernel(const uint32_t* __restrict__ key,
                                                                     uint32_t* rank,
                                                                     const uint32_t* __restrict__ start, uint32_t n,
-                                                                    uint32_t* unsorted, uint32_t* big, int id_bits) {
+                                                                    uint32_t* unsorted, uint32_t* tile_count,
+                                                                    uint32_t tile_fine, uint32_t tile_row,
+                                                                    int tile_shift, uint32_t* big) {
   chain_begin();
   const uint32_t i = blockIdx.x * kSortThreads + threadIdx.x;
-  if (i < n) unsorted[start[key[i]] + rank[i]] = i;
-  const uint32_t nbig = ((volatile uint32_t*)big)[0];
-  if (nbig == 0) return;
-  __shared__ bool last;
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(&big[1], 1u) == gridDim.x - 1;
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  for (uint32_t b = 0; b < nbig; ++b) {
-    const uint32_t c = big[2 + b];
-    const uint32_t s0 = start[c];
-    sort_segment(unsorted + s0, rank + s0, start[c + 1] - s0, id_bits);  // the ranks are done with
+  uint32_t c = 0, b = 0, r = 0;
+  if (i < n) {
+    r = *(volatile uint32_t*)(rank + i);  // (before the flag is known, not after)
+    c = key[i];
+    b = start[c];
   }
-  if (threadIdx.x == 0) big[0] = big[1] = 0;
+  const bool big_cells = *(volatile uint32_t*)big != 0;
+  if (i < n && (!big_cells || start[c + 1] - b <= kBigCell)) unsorted[b + r] = i;
+  if (!big_cells) return;
+  rank_big_cells(key, rank, start, n, unsorted, tile_count, tile_fine, tile_row, tile_shift);
+  // the block that finishes last clears the flag for the next search
+  __syncthreads();
+  if (threadIdx.x == 0 && atomicAdd(&big[1], 1u) == gridDim.x - 1) big[0] = big[1] = 0;
 }
 
 int bits_needed(uint64_t v) {
@@ -383,18 +407,76 @@ int launch_exclusive_scan(cudaStream_t st, const uint32_t* in, uint32_t* out, si
   return PG_OK;
 }
 
+namespace {
+
+constexpr int kDenseItems = 4;  // keys per thread of the radix kernels
+
+// The sort for n particles in ncells cells, by their mean number per cell.  The more there are, the longer a
+// gather thread's rank loop and the more atomics fall on one address; the radix sort's time only falls, with
+// the digits.  Search and gather in us, one atomic per particle / merged per warp / radix sort, ids in
+// random order and (from 256k) in cell order:
+//   n    mean   random order        cell order
+//   16k  593    33 / 32 / 35
+//   64k  296    33 / 33 / 35
+//   64k  512    40 / 38 / 36
+//   256k 32     34 / 34 / 59        31 / 26 / 56
+//   256k 256    55 / 56 / 58        64 / 37 / 55
+//   256k 500    82 / 81 / 58       102 / 48 / 56
+//   1M   16     65 / 69 / 104       54 / 52 / 80
+//   1M   64     71 / 72 / 103       78 / 57 / 80
+//   1M   125    83 / 83 / 100      101 / 64 / 80
+//   1M   244   107 / 107 / 99      150 / 81 / 81
+//   1M   579   174 / 174 / 95      265 / 131 / 81
+//   4M   64    225 / 238 / 304     254 / 172 / 192
+//   4M   134   245 / 255 / 302     359 / 207 / 190
+//   4M   256   315 / 318 / 294     559 / 276 / 190
+HashMode sort_mode(size_t n, uint64_t ncells) {
+  const uint64_t mean = n / (ncells ? ncells : 1);
+  if (mean >= (n >= 1000000 ? 192u : n >= 50000 ? 448u : 1024u)) return HASH_IDS;
+  return mean >= 32 ? HASH_COUNT_MERGED : HASH_COUNT;
+}
+
+}  // namespace
+
 int NbrWork::init(size_t n_, uint64_t ncells_) {
   n = n_;
   ncells = ncells_;
+  mode = sort_mode(n, ncells);
+  radix = mode == HASH_IDS;
   passes = (bits_needed(ncells ? ncells - 1 : 0) + 7) / 8;
+  const size_t nn = n ? n : 1;
   chunks = (uint32_t)(ncells / kScanChunk + 1);
-  const size_t nn = n ? n : 1, cells = (size_t)chunks * kScanChunk;
-  rest_words = cells + 2 + nn / kBigCell;
+  const size_t cells = (size_t)chunks * kScanChunk;
+  size_t counts = 0, tile_words = 0, nradix = 0;
+  if (radix) {
+    nradix = nn;
+    tiles = (int)((nn + kSortThreads * kDenseItems - 1) / (kSortThreads * kDenseItems));
+  } else {
+    counts = cells;
+    // large cells: a row of counts per tile of ids and per group of 32 tiles
+    tile_shift = 10;
+    while ((nn - 1) >> tile_shift >= kMaxTiles) ++tile_shift;
+    tile_fine = (uint32_t)(((nn - 1) >> tile_shift) / 32 + 1) * 32;
+    tile_row = tile_fine + (tile_fine / 32 + 3) / 4 * 4;
+    if (nn > kBigCell) tile_words = (nn / kBigCell + 1) * tile_row;
+  }
+  rest_words = counts + 2;
   struct {
     uint32_t** p;
     size_t words;
-  } parts[] = {{&key, nn},           {&rank, nn},          {&unsorted, nn},       {&sorted_cell, nn},
-               {&sorted_id, nn},     {&cell_start, cells}, {&chunk_total, chunks}, {&rest, rest_words}};
+  } parts[] = {{&key, nn},
+               {&rank, nn},
+               {&cell_start, cells},
+               {&rest, rest_words},
+               {&unsorted, nn - nradix},
+               {&sorted_cell, nn - nradix},
+               {&sorted_id, nn - nradix},
+               {&chunk_total, radix ? 0 : chunks},
+               {&tile_count, tile_words},
+               {&key2, nradix},
+               {&id2, nradix},
+               {&hist, radix ? (size_t)kRadix * tiles : 0},
+               {&digit_total, radix ? kRadix : 0}};
   size_t words = 0;
   for (auto& part : parts) words += (part.words + 63) / 64 * 64;  // each from a 256-byte boundary
   PG_TRY(mem.ensure(words * 4));
@@ -403,8 +485,12 @@ int NbrWork::init(size_t n_, uint64_t ncells_) {
     *part.p = at;
     at += (part.words + 63) / 64 * 64;
   }
+  if (radix) {  // the buffers that the last pass writes
+    sorted_cell = passes & 1 ? key2 : key;
+    sorted_id = passes & 1 ? id2 : rank;
+  }
   count = rest;
-  big = rest + cells;
+  big = rest + counts;
   clean = false;
   return PG_OK;
 }
@@ -413,23 +499,44 @@ size_t NbrWork::bytes() const { return mem.bytes; }
 
 NbrOrder nbr_order(const NbrWork& w) {
   NbrOrder o;
-  o.unsorted = w.unsorted;
-  o.key = w.key;
+  o.unsorted = w.radix ? w.sorted_id : w.unsorted;
+  o.key = w.radix ? nullptr : w.key;
   o.cell_start = w.cell_start;
   o.sorted_cell = w.sorted_cell;
   o.sorted_id = w.sorted_id;
+  o.rank = w.rank;
+  o.tile_count = w.tile_count;
+  o.tile_fine = w.tile_fine;
+  o.tile_row = w.tile_row;
+  o.tile_shift = w.tile_shift;
   return o;
 }
 
 int launch_sort(cudaStream_t st, NbrWork& w, unsigned long long* minacc, unsigned long long* minout, uint32_t nmin) {
+  if (w.radix) {
+    uint32_t *k0 = w.key, *v0 = w.rank, *k1 = w.key2, *v1 = w.id2;
+    for (int p = 0; p < w.passes; ++p) {
+      digit_hist_kernel<kDenseItems><<<w.tiles, kSortThreads, 0, st>>>(k0, w.n, 8 * p, w.tiles, w.hist);
+      digit_scan_kernel<<<kRadix, kSortThreads, 0, st>>>(w.hist, w.tiles, w.digit_total);
+      digit_scatter_kernel<kDenseItems><<<w.tiles, kSortThreads, 0, st>>>(k0, v0, k1, v1, w.n, 8 * p, w.tiles, w.hist,
+                                                                         w.digit_total);
+      std::swap(k0, k1);
+      std::swap(v0, v1);
+    }
+    cell_start_kernel<<<(unsigned)(w.ncells / 256 + 1), 256, 0, st>>>(w.sorted_cell, (uint32_t)w.n, (uint32_t)w.ncells,
+                                                                     w.cell_start, minacc, minout, minacc ? nmin : 0u);
+    PG_CUDA_TRY(cudaGetLastError());
+    return PG_OK;
+  }
   if (w.chunks > 1)
     PG_CUDA_TRY(launch_chained(st, w.n > 0, cell_reduce_kernel, w.chunks, kCellScanThreads, w.count, w.chunk_total));
   PG_CUDA_TRY(launch_chained(st, w.n > 0 || w.chunks > 1, cell_scan_kernel, w.chunks, kCellScanThreads, w.count,
-                             w.chunk_total, w.cell_start, minacc, minout, minacc ? nmin : 0u));
+                             w.chunk_total, w.cell_start, w.tile_count, w.tile_row, minacc, minout,
+                             minacc ? nmin : 0u));
   if (w.n)
     PG_CUDA_TRY(launch_chained(st, true, cell_scatter_kernel, (unsigned)((w.n + kSortThreads - 1) / kSortThreads),
-                               kSortThreads, w.key, w.rank, w.cell_start, (uint32_t)w.n, w.unsorted, w.big,
-                               bits_needed(w.n - 1)));
+                               kSortThreads, w.key, w.rank, w.cell_start, (uint32_t)w.n, w.unsorted, w.tile_count,
+                               w.tile_fine, w.tile_row, w.tile_shift, w.big));
   PG_CUDA_TRY(cudaGetLastError());
   return PG_OK;
 }
