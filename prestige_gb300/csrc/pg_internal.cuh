@@ -140,7 +140,7 @@ __host__ __device__ __forceinline__ uint32_t lane_slot(uint32_t block_id, uint32
 // ---------------------------------------------------------------------------------------
 // Neighbour-search workspace: stable sort of the particles by cell, and the cell table (pg_sort.cu).
 // ---------------------------------------------------------------------------------------
-constexpr uint32_t kScanChunk = 8192;  // cells per block of the scan
+constexpr uint32_t kScanChunk = 8192;  // cells a block of the scan takes at a time
 constexpr uint32_t kBigCell = 1024;    // larger cells are ranked by tiles of ids (see pg_sort.cu)
 constexpr uint32_t kMaxTiles = 1024;
 
@@ -164,7 +164,7 @@ struct NbrWork {
   // counting sort
   uint32_t chunks = 0;              // scan chunks: cover ncells + 1 entries
   uint32_t* unsorted = nullptr;     // [n] ids by cell
-  uint32_t* chunk_total = nullptr;  // [chunks] particles per chunk
+  uint32_t* chunk_total = nullptr;  // [chunks] particles per block of the scan
   uint32_t* tile_count = nullptr;   // cells of more than kBigCell: rows of tile_row words (see pg_sort.cu)
   uint32_t tile_fine = 0, tile_row = 0;
   int tile_shift = 0;               // log2 of the ids per tile

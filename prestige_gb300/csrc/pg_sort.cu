@@ -10,10 +10,10 @@
 // The sort of a handle takes three or four launches and a share of the sorted gather that follows:
 //   hash (pg_neighbors.cu)  cell of each id; an atomic on the cell's count gives the id its arrival
 //                rank there
-//   cell_reduce  totals per chunk of kScanChunk cells (grids of more than one chunk; adding them up by
+//   cell_reduce  totals per block of the scan (grids of more than one chunk of kScanChunk cells; adding them up by
 //                atomics in the hash took 5 ns per warp of particles: one address at a time)
-//   cell_scan    cell_start = exclusive scan of the counts: a block per chunk, its base the sum of
-//                the totals of the chunks before it; the counts go back to zero for the next search
+//   cell_scan    cell_start = exclusive scan of the counts: a block per chunk (in the largest grids for
+//                several), its base the sum of the totals of the blocks before it; the counts go back to zero for the next search
 //   cell_scatter id -> slot cell_start[cell] + rank, so ids are grouped by cell in arrival order
 //   the gather   ranks each id among the ids of its cell (ordered_slot): the stable order
 // It is bound by the latency of these few launches below about 1M particles and by the scattered
@@ -254,19 +254,47 @@ __global__ void cell_start_kernel(const uint32_t* __restrict__ cell, uint32_t n,
 // ---------------------------------------------------------------------------------------
 constexpr int kCellScanThreads = 1024;
 constexpr int kCellScanItems = kScanChunk / kCellScanThreads;
+constexpr uint32_t kScanBlocks = 16384;
 static_assert(kCellScanItems == 8, "two 16-byte loads per thread");
 
+// MANY: blocks of `per_block` chunks each (all but the last), of `chunks` in all; otherwise one chunk a block.
+// Every block adds up the totals of the blocks before it, so their number is kept to kScanBlocks: with one chunk a
+// block a search over 4.2e9 cells takes 27.0 ms, most of it for these sums, and 8.2 with 16384 blocks (the radix
+// sort 16.5); 1e9 cells 3.2 and 2.0.
+template <bool MANY>
 __global__ void __launch_bounds__(kCellScanThreads) cell_reduce_kernel(const uint32_t* __restrict__ count,
+                                                                       uint32_t chunks, uint32_t per_block,
                                                                        uint32_t* __restrict__ chunk_total) {
   chain_begin();
-  const uint4* cp = (const uint4*)(count + (size_t)blockIdx.x * kScanChunk) + 2 * threadIdx.x;
-  const uint4 a = cp[0], b = cp[1];
+  const uint32_t c0 = MANY ? blockIdx.x * per_block : blockIdx.x, c1 = MANY ? min(c0 + per_block, chunks) : c0 + 1;
+  uint32_t sum = 0;
+  for (uint32_t c = c0; c < c1; ++c) {
+    const uint4* cp = (const uint4*)(count + (size_t)c * kScanChunk) + 2 * threadIdx.x;
+    const uint4 a = cp[0], b = cp[1];
+    sum += a.x + a.y + a.z + a.w + b.x + b.y + b.z + b.w;
+  }
   uint32_t total;
-  block_excl_scan(a.x + a.y + a.z + a.w + b.x + b.y + b.z + b.w, &total);
+  block_excl_scan(sum, &total);
   if (threadIdx.x == 0) chunk_total[blockIdx.x] = total;
 }
 
-__global__ void __launch_bounds__(kCellScanThreads) cell_scan_kernel(uint32_t* __restrict__ count,
+// Zero rows for those of 8 consecutive cells that hold more than kBigCell (first: their first slots, just
+// written; end: the slot after the last).
+__device__ __noinline__ void clear_rows(uint32_t* tile_count, uint32_t tile_row, const uint32_t* first, uint32_t end) {
+  for (int i = 7; i >= 0; --i) {
+    const uint32_t b = first[i];
+    if (end - b > kBigCell) {
+      uint4* row = (uint4*)(tile_count + (size_t)(b / kBigCell) * tile_row);
+      for (uint32_t w = 0; w < tile_row / 4; ++w) row[w] = make_uint4(0, 0, 0, 0);
+    }
+    end = b;
+  }
+}
+
+// (two blocks per SM: with more than 32 registers a thread there is one, and 1e8 cells take 0.35 ms in place of 0.27)
+template <bool MANY>
+__global__ void __launch_bounds__(kCellScanThreads, 2) cell_scan_kernel(uint32_t* __restrict__ count, uint32_t chunks,
+                                                                     uint32_t per_block,
                                                                      const uint32_t* __restrict__ chunk_total,
                                                                      uint32_t* __restrict__ start,
                                                                      uint32_t* __restrict__ tile_count,
@@ -275,37 +303,37 @@ __global__ void __launch_bounds__(kCellScanThreads) cell_scan_kernel(uint32_t* _
   __shared__ uint32_t base;
   chain_begin();
   const uint32_t tid = threadIdx.x;
-  // cells of the chunks before this one
+  // cells of the blocks before this one
   uint32_t before = 0;
   for (uint32_t c = tid; c < blockIdx.x; c += kCellScanThreads) before += chunk_total[c];
   uint32_t total;
   block_excl_scan(before, &total);
   if (tid == 0) base = total;
-  uint4* cp = (uint4*)(count + (size_t)blockIdx.x * kScanChunk) + 2 * tid;
-  const uint4 a = cp[0], b = cp[1];
-  if (a.x | a.y | a.z | a.w) cp[0] = make_uint4(0, 0, 0, 0);
-  if (b.x | b.y | b.z | b.w) cp[1] = make_uint4(0, 0, 0, 0);
-  uint32_t ex = block_excl_scan(a.x + a.y + a.z + a.w + b.x + b.y + b.z + b.w, &total) + base;
-  uint4 o, p;
-  o.x = ex;
-  o.y = o.x + a.x;
-  o.z = o.y + a.y;
-  o.w = o.z + a.z;
-  p.x = o.w + a.w;
-  p.y = p.x + b.x;
-  p.z = p.y + b.y;
-  p.w = p.z + b.z;
-  uint4* sp = (uint4*)(start + (size_t)blockIdx.x * kScanChunk) + 2 * tid;
-  sp[0] = o;
-  sp[1] = p;
-  if ((a.x | a.y | a.z | a.w | b.x | b.y | b.z | b.w) > kBigCell) {  // (at least their maximum)
-    const uint32_t m[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w}, first[8] = {o.x, o.y, o.z, o.w, p.x, p.y, p.z, p.w};
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-      if (m[i] > kBigCell) {
-        uint4* row = (uint4*)(tile_count + (size_t)(first[i] / kBigCell) * tile_row);
-        for (uint32_t w = 0; w < tile_row / 4; ++w) row[w] = make_uint4(0, 0, 0, 0);
-      }
+  const uint32_t c0 = MANY ? blockIdx.x * per_block : blockIdx.x, c1 = MANY ? min(c0 + per_block, chunks) : c0 + 1;
+  for (uint32_t c = c0; c < c1; ++c) {
+    uint4* cp = (uint4*)(count + (size_t)c * kScanChunk) + 2 * tid;
+    const uint4 a = cp[0], b = cp[1];
+    if (a.x | a.y | a.z | a.w) cp[0] = make_uint4(0, 0, 0, 0);
+    if (b.x | b.y | b.z | b.w) cp[1] = make_uint4(0, 0, 0, 0);
+    const uint32_t ex = block_excl_scan(a.x + a.y + a.z + a.w + b.x + b.y + b.z + b.w, &total) + base;
+    if (MANY) {
+      __syncthreads();  // (base has been read)
+      if (tid == 0) base += total;
+    }
+    uint4 o, p;
+    o.x = ex;
+    o.y = o.x + a.x;
+    o.z = o.y + a.y;
+    o.w = o.z + a.z;
+    p.x = o.w + a.w;
+    p.y = p.x + b.x;
+    p.z = p.y + b.y;
+    p.w = p.z + b.z;
+    uint4* sp = (uint4*)(start + (size_t)c * kScanChunk) + 2 * tid;
+    sp[0] = o;
+    sp[1] = p;
+    if ((a.x | a.y | a.z | a.w | b.x | b.y | b.z | b.w) > kBigCell)  // (at least their maximum)
+      clear_rows(tile_count, tile_row, start + (size_t)c * kScanChunk + 8 * tid, p.w + b.w);
   }
   if (blockIdx.x == 0)
     for (uint32_t i = tid; i < nmin; i += kCellScanThreads) {
@@ -528,11 +556,14 @@ int launch_sort(cudaStream_t st, NbrWork& w, unsigned long long* minacc, unsigne
     PG_CUDA_TRY(cudaGetLastError());
     return PG_OK;
   }
-  if (w.chunks > 1)
-    PG_CUDA_TRY(launch_chained(st, w.n > 0, cell_reduce_kernel, w.chunks, kCellScanThreads, w.count, w.chunk_total));
-  PG_CUDA_TRY(launch_chained(st, w.n > 0 || w.chunks > 1, cell_scan_kernel, w.chunks, kCellScanThreads, w.count,
-                             w.chunk_total, w.cell_start, w.tile_count, w.tile_row, minacc, minout,
-                             minacc ? nmin : 0u));
+  const uint32_t per_block = (w.chunks + kScanBlocks - 1) / kScanBlocks;
+  const uint32_t blocks = (w.chunks + per_block - 1) / per_block;
+  if (blocks > 1)
+    PG_CUDA_TRY(launch_chained(st, w.n > 0, per_block > 1 ? cell_reduce_kernel<true> : cell_reduce_kernel<false>, blocks,
+                               kCellScanThreads, w.count, w.chunks, per_block, w.chunk_total));
+  PG_CUDA_TRY(launch_chained(st, w.n > 0 || blocks > 1, per_block > 1 ? cell_scan_kernel<true> : cell_scan_kernel<false>,
+                             blocks, kCellScanThreads, w.count, w.chunks, per_block, w.chunk_total, w.cell_start,
+                             w.tile_count, w.tile_row, minacc, minout, minacc ? nmin : 0u));
   if (w.n)
     PG_CUDA_TRY(launch_chained(st, true, cell_scatter_kernel, (unsigned)((w.n + kSortThreads - 1) / kSortThreads),
                                kSortThreads, w.key, w.rank, w.cell_start, (uint32_t)w.n, w.unsorted, w.tile_count,
