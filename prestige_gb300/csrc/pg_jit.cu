@@ -517,6 +517,8 @@ int pg_run_equations(pg_system* s, const char* const* bodies, int n_bodies) {
     pg::set_error("pg_run_equations runs on single-system handles");
     return PG_EINVAL;
   }
+  // staged inputs first: they may trade a field's buffer, whose address is taken below
+  PG_TRY(pg::apply_io_inputs(s));
   pg::Translation tr;
   std::string err;
   if (!pg::translate(v, tr, err)) {
