@@ -137,6 +137,9 @@ int pg_get_field(pg_system* sys, const char* name, void* host, size_t count, int
  *                       first moves it into the field (the buffers trade places; a handle with
  *                       a captured graph copies it in).  So inputs for step k+1 upload while
  *                       step k runs.
+ *                       pg_backward, which goes back over a recorded run and ends in its final
+ *                       state, leaves them to the call after it, as do the calls that only
+ *                       change settings (tuning).
  *   pg_get_field_async  snapshots the field at this point of the handle's work (a device copy)
  *                       and copies the snapshot to `host` on an output copy stream; later steps
  *                       do not disturb it.  So results of step k download while step k+1 runs.

@@ -548,6 +548,7 @@ int pg_forward_checkpointed(pg_system* s, int nsteps, int every) {
     pg::set_error("need nsteps >= 0 and every >= 1");
     return PG_EINVAL;
   }
+  PG_TRY(pg::apply_io_inputs(s));
   if (!s->adj) s->adj = new pg_adjoint();
   pg_adjoint* A = s->adj;
   A->have_forward = false;

@@ -246,6 +246,7 @@ int pg_autotune(pg_system* s, int trial_steps, int* best_block, double* best_mul
     pg::set_error("trial_steps must be >= 1");
     return PG_EINVAL;
   }
+  PG_TRY(pg::apply_io_inputs(s));
   PG_CUDA_TRY(cudaStreamSynchronize(s->stream));
   const bool graph = s->graph_enabled;
   const bool timing = s->timing;

@@ -56,3 +56,45 @@ def test_run_equations(pg, bodies, last, graph):
     del keep
     for k in out[0]:
         assert np.array_equal(out[0][k], out[1][k]), k
+
+
+@pytest.mark.parametrize("last", ["pos", "vel", "rho", "mass"])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_forward_checkpointed(pg, mode, last):
+    w = workloads.differentiable_3d(n=2000)
+    rng = np.random.default_rng(3)
+    new = {k: v * (1.0 + 1e-3 * rng.uniform(-1.0, 1.0, size=v.shape)) for k, v in w["fields"].items()}
+    later = {k: v * (1.0 + 1e-3 * rng.uniform(-1.0, 1.0, size=v.shape)) for k, v in w["fields"].items()}
+    out = []
+    for staged in (False, True):
+        s = _system(w, mode, False)
+        if staged:
+            keep = _stage(s, new, last)
+        else:
+            for k, v in new.items():
+                s.set(k, v)
+        s.forward_checkpointed(5, 2)
+        out.append([s.get(k) for k in ("pos", "vel", "rho", "mass")])
+        if staged:  # staged before the backward pass: taken by the call after it
+            t = _pinned(later[last])
+            s.set_ptr_async(last, t.data_ptr(), t.numel())
+        out[-1] += [np.asarray(g) for g in s.backward(out[-1][0] - w["target"])]
+        if staged:
+            assert np.array_equal(s.get(last), later[last])
+        s.wait_io()
+        s.close()
+    del keep
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
+
+
+def test_autotune_keeps_them(pg):
+    w = workloads.sph_lattice_3d(n=1000, seed=4)
+    s = _system(w, 1, False)
+    vel = w["fields"]["vel"] + 0.5
+    keep = _stage(s, {"vel": vel}, "vel")
+    s.autotune(trial_steps=1)
+    assert np.array_equal(s.get("vel"), vel)
+    s.wait_io()
+    s.close()
+    del keep
