@@ -212,7 +212,8 @@ __global__ void adjoint_prep_f_kernel(SphArgs a) {
   const double P = tait_pterm<OpsD>(K.d, K.gamma, rho);
   const double Pd = soft_div(K.d.B * ((double)(K.gamma - 2) * pw + 2.0) * inv_r2, rho);
   const double PB = (pw - 1.0) * inv_r2;
-  float4 *X = (float4*)a.s[0] + 2 * (size_t)k, *V = (float4*)a.s[1] + 2 * (size_t)k, *Q = (float4*)a.s[2] + 2 * (size_t)k;
+  float4 *X = (float4*)a.s[0] + 2 * (size_t)k, *V = (float4*)a.s[1] + 2 * (size_t)k;
+  float4* Q = (float4*)a.s[2] + 2 * (size_t)k;
   X[0] = make_float4(hx[0], hx[1], hx[2], (float)m);
   X[1] = make_float4(lxs[0], lxs[1], lxs[2], 0.f);
   V[0] = make_float4(hv[0], hv[1], hv[2], (float)rho);

@@ -256,7 +256,8 @@ long long neighbor_launches(const pg_system* s) { return s->nw.launches(); }
 // The IEEE f64 step evaluates each pair once (pg_sph_sym.cu: four kernels) at every size.  The two-sided
 // passes (two launches) were the faster ones below 16,384 particles while a slot's pairs ran on one
 // thread; with four threads per slot the 2D dam break of 6,518 particles takes 72 us a step
-// pair-once against 92 two-sided, 4,000 particles in 3D 162 against 266.  Both give the oracle's bits.
+// pair-once (70 from a graph) against 92 two-sided, 4,000 particles in 3D 162 against 266.  Both
+// give the oracle's bits.
 bool pair_once(const pg_system* s) { return s->arith == ARITH_F64_EXACT; }
 
 bool overlapped(const pg_system* s) { return s->ov_split > 0 && s->ov_split < s->n; }
@@ -595,28 +596,6 @@ int capture_graphs(pg_system* s) {
   return st;
 }
 
-// Overlap of the continuity pass (FMA-bound) with the list kernel (ALU-bound) for double-word
-// SPH handles of at least 1M particles: the lists of the first 70 % of the slots are built
-// first, then the continuity pass over them runs beside the lists of the rest, and the
-// continuity pass over the rest follows those lists on their stream.  The list kernel's
-// persistent grid leaves room on every SM for two thirds of the pass's blocks (registers per
-// block from the kernels' attributes) and runs on a stream of the highest priority, so its
-// blocks are placed first; the continuity passes run one block per tile and fill the SMs as the
-// list blocks finish.  Measured at 4M particles (ms per step):
-//   no overlap, persistent grids                                          9.46
-//   overlap with both kernels on persistent grids                        9.27
-//   the same build later: persistent grids 8.10, backfilling pass 8.11,
-//   backfilling pass and list-stream priority 7.76
-//   continuity over the rest on the list stream                           7.65 (7.70 without)
-//   splits 0.5 / 0.6 / 0.8 of the slots                                   7.92 / 7.72 / 7.69
-//   the same after the per-entry cache held u (7.02 at 0.7): 0.6 / 0.8    7.02 / 7.05
-// A finer pipeline (the slots in 4, 8 or 16 even chunks, each chunk's continuity pass starting
-// when its lists are done) gave 7.80 / 7.84 / 8.02 ms against 7.76 for two chunks on the same
-// box: lists and continuity add up to about 4.4 ms however they are interleaved, so once the SMs
-// are backfilled the two kernels share a saturated machine.
-// At 1M particles it is even (1.965 ms either way), at 256k slower (0.690 against 0.670 ms),
-// hence the threshold.  The 512-system batch of 2D dam breaks (6.1M particles, one handle)
-// gains too: 3.36 against 3.45 ms (with persistent grids it had lost, 3.91 against 3.81).
 // The auxiliary stream of the overlapped schedules (greatest priority: the list kernel's blocks
 // are placed first, the pair pass beside it fills the rest) and its two events.
 int ensure_aux_stream(pg_system* s) {
@@ -630,6 +609,23 @@ int ensure_aux_stream(pg_system* s) {
   return PG_OK;
 }
 
+// Overlap of the continuity pass (FMA-bound) with the list kernel (ALU-bound) for double-word
+// SPH handles of at least 1M particles: the lists of the first 70 % of the slots are built
+// first, then the continuity pass over them runs beside the lists of the rest, and the
+// continuity pass over the rest follows those lists on their stream.  The list kernel's
+// persistent grid leaves room on every SM for two thirds of the pass's blocks (registers per
+// block from the kernels' attributes) and runs on a stream of the highest priority, so its
+// blocks are placed first; the continuity passes run one block per tile and fill the SMs as the
+// list blocks finish.  Step in ms, replayed, without overlap and with 50 / 60 / 70 / 80 % first:
+//   3D lattice, half-size cells,  262k    0.424   0.440 / 0.435 / 0.443 / 0.440
+//                                 500k    0.796   0.776 / 0.788 / 0.787 / 0.785
+//                                 1M      1.588   1.518 / 1.523 / 1.528 / 1.530
+//                                 2M      3.175   3.010 / 3.018 / 3.026 / 3.035
+//                                 4M      6.69    6.09  / 6.11  / 6.10  / 6.12
+//   512 2D dam breaks, 6.1M               2.708       -   / 2.528 / 2.532 / 2.539
+// The split hardly matters, and the line could lie at 500k (1.5 %).  The IEEE step's overlap, without and with
+// 12.5 / 25 / 50 % first: 1M 4.716, 4.740 / 4.747 / 4.806, 2M 9.513, 9.521 / 9.523 / 9.622: with sym_c1 at its
+// present length it gains nothing (it did when that kernel took twice as long).
 int choose_overlap(pg_system* s, int sms) {
   s->ov_split = 0;
   if (s->model == PG_MODEL_SPH && s->arith == ARITH_F64_EXACT && s->n >= 1000000) {
@@ -644,7 +640,8 @@ int choose_overlap(pg_system* s, int sms) {
     return PG_OK;
   }
   if (s->model != PG_MODEL_SPH || s->arith != ARITH_F64_DF || s->n < 1000000) return PG_OK;
-  const int rp = sph_list_regs(s->arith, s->dim, s->grids[0].reach, SPH_CONT, s->lanes), rl = sph_list_regs(s->arith, s->dim, s->grids[0].reach, -1);
+  const int rp = sph_list_regs(s->arith, s->dim, s->grids[0].reach, SPH_CONT, s->lanes);
+  const int rl = sph_list_regs(s->arith, s->dim, s->grids[0].reach, -1);
   if (rp <= 0 || rl <= 0) return PG_OK;
   const int per_block_p = ((rp + 7) / 8) * 8 * s->block, per_block_l = ((rl + 7) / 8) * 8 * s->block;
   const int regs = 65536, threads = 2048;

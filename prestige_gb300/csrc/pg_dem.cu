@@ -210,7 +210,7 @@ __device__ __noinline__ D3 spin_update(D3 w, D3 T, double I, double dt) {
 // contacts of the whole warp together: the warp's contacts are numbered in (lane, order found)
 // order and each lane evaluates one contact of a chunk of 32, whichever particle owns it; the
 // terms of an owner's contacts are then added in the order it found them, so the sums and the
-// history are the oracle's, bit for bit.  (What bounds it: the FP64 pipe in a dense packing, 78 % busy;
+// history are the oracle's, bit for bit.  (What bounds it: the FP64 pipe in a dense packing, 76 % busy;
 // the walk's loads in a loose one.)  Evaluated in the walk, each lane's contact ran alone
 // while the others waited (a few contacts per particle among about 200 candidates, at different
 // iterations per lane); evaluated per lane after the walk, a warp ran as many rounds as its
@@ -544,7 +544,8 @@ int launch_dem_gather(cudaStream_t st, const DemArgs& a) {
 
 int launch_dem_pass(cudaStream_t st, const DemArgs& a) {
   if (a.n == 0) return PG_OK;
-  PG_CUDA_TRY(launch_chained(st, a.chained != 0, dem_pass_kernel, (a.n + kDemThreads - 1) / kDemThreads, kDemThreads, a));
+  const unsigned blocks = (a.n + kDemThreads - 1) / kDemThreads;
+  PG_CUDA_TRY(launch_chained(st, a.chained != 0, dem_pass_kernel, blocks, kDemThreads, a));
   PG_CUDA_TRY(cudaGetLastError());
   return PG_OK;
 }

@@ -46,12 +46,12 @@ enum : unsigned {
 };
 
 // ---------------------------------------------------------------------------------------
-// Dependent launches inside a step and from one step to the next.  The kernels of a step form a chain on one stream, and below about
-// 100k particles a good part of a step is the gap between a kernel's end and the next one's first
-// instruction.  A kernel launched with launch_chained directly after another kernel (no copy, memset
-// or event in between) is set up while that one runs and starts as its last blocks end; chain_begin(),
-// first in every kernel that is launched so, waits until the earlier kernel is complete and its
-// writes are visible.  Since every kernel waits for the one before, a kernel's inputs may come from
+// Dependent launches inside a step and from one step to the next.  The kernels of a step form a chain on
+// one stream, and below about 100k particles a good part of a step is the gap between a kernel's end
+// and the next one's first instruction.  A kernel launched with launch_chained directly after another
+// kernel (no copy, memset or event in between) is set up while that one runs and starts as its last
+// blocks end; chain_begin(), first in every kernel that is launched so, waits until the earlier kernel
+// is complete and its writes are visible.  Since every kernel waits for the one before, a kernel's inputs may come from
 // any earlier kernel of the stream.  us per step with plain and chained launches: dam break, 6.5k
 // particles, eager 51.8 / 38.0, as a graph 38.8 / 37.2; 100k eager 244 / 231; 262k eager 475 / 463.
 // The first kernel of a step is chained to the step before it: 3D lattice of 5,000 particles, eager, 61.5 -> 59.4.
@@ -63,7 +63,8 @@ __device__ __forceinline__ void chain_begin() {
 }
 
 template <class... P, class... A>
-cudaError_t launch_chained(cudaStream_t st, bool chained, void (*kernel)(P...), unsigned grid, unsigned block, A... args) {
+cudaError_t launch_chained(cudaStream_t st, bool chained, void (*kernel)(P...), unsigned grid, unsigned block,
+                           A... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(block);

@@ -99,12 +99,14 @@ int launch_sph_list(cudaStream_t st, const SphArgs& a, int arith, int grid, int 
 // lanes: threads per slot of the continuity and momentum passes (1, 2 or 4: 32, 16 or 8
 // particles per warp); only the tolerance-based modes (double-word f64, contracted f32) take
 // more than one, the others run 1 (sph_pass_lanes gives the count a pass actually uses).  With 1,
-// the double-word passes of small handles run 2 or 4 threads per slot that add in list order (same bits).
+// the double-word and f32 passes of small handles run 2 or 4 threads per slot that add in list order
+// (the same bits).
 int launch_sph_list_pass(cudaStream_t st, const SphArgs& a, int arith, int stage, int grid, int block,
                          int lanes = 1);
 int sph_pass_lanes(int arith, int stage, int lanes);
-int sph_list_regs(int arith, int dim, int reach, int stage, int lanes = 1);  // registers per thread of a list kernel (stage < 0) or pass
-int sph_list_occupancy(int arith, int dim, int reach, int stage, int block, int lanes = 1);  // stage < 0: the list kernel
+// Registers per thread and resident blocks per SM of a pass (stage < 0: the list kernel).
+int sph_list_regs(int arith, int dim, int reach, int stage, int lanes = 1);
+int sph_list_occupancy(int arith, int dim, int reach, int stage, int block, int lanes = 1);
 // The list kernel with the conservative FP32 test on the positions a.pf.
 int launch_sph_list_pf(cudaStream_t st, const SphArgs& a, int grid, int block);
 // The IEEE f64 step with each neighbour pair evaluated once (pg_sph_sym.cu), over complete lists:

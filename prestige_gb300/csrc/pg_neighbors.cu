@@ -395,8 +395,8 @@ static cudaError_t hash_mode(cudaStream_t st, bool chained, const GridK* grid, c
 }
 
 template <class R, int DIM>
-static cudaError_t hash_dim(cudaStream_t st, bool chained, const GridK* grid, const uint32_t* sys_of_id, const void* pos,
-                            NbrWork& w, unsigned long long* posmin) {
+static cudaError_t hash_dim(cudaStream_t st, bool chained, const GridK* grid, const uint32_t* sys_of_id,
+                            const void* pos, NbrWork& w, unsigned long long* posmin) {
   switch (w.mode) {
     case HASH_COUNT: return hash_mode<R, DIM, HASH_COUNT>(st, chained, grid, sys_of_id, pos, w, posmin);
     case HASH_COUNT_MERGED: return hash_mode<R, DIM, HASH_COUNT_MERGED>(st, chained, grid, sys_of_id, pos, w, posmin);
@@ -421,12 +421,17 @@ int launch_hash(cudaStream_t st, bool chained, const GridK* grid_dev, const uint
 int launch_sorted_positions(cudaStream_t st, const NbrArgs& a, const void* pos, void* spos) {
   if (a.n == 0) return PG_OK;
   const unsigned b = blocks_for(a.n, 256);
+  auto launch = [&](auto kernel, auto* p, auto* sp) { return launch_chained(st, true, kernel, b, 256, a, p, sp); };
   if (a.f64) {
-    if (a.dim == 2) PG_CUDA_TRY(launch_chained(st, true, sorted_positions_kernel<double, 2>, b, 256, a, (const double*)pos, (double4_32a*)spos));
-    else PG_CUDA_TRY(launch_chained(st, true, sorted_positions_kernel<double, 3>, b, 256, a, (const double*)pos, (double4_32a*)spos));
+    const double* p = (const double*)pos;
+    double4_32a* sp = (double4_32a*)spos;
+    if (a.dim == 2) PG_CUDA_TRY(launch(sorted_positions_kernel<double, 2>, p, sp));
+    else PG_CUDA_TRY(launch(sorted_positions_kernel<double, 3>, p, sp));
   } else {
-    if (a.dim == 2) PG_CUDA_TRY(launch_chained(st, true, sorted_positions_kernel<float, 2>, b, 256, a, (const float*)pos, (float4*)spos));
-    else PG_CUDA_TRY(launch_chained(st, true, sorted_positions_kernel<float, 3>, b, 256, a, (const float*)pos, (float4*)spos));
+    const float* p = (const float*)pos;
+    float4* sp = (float4*)spos;
+    if (a.dim == 2) PG_CUDA_TRY(launch(sorted_positions_kernel<float, 2>, p, sp));
+    else PG_CUDA_TRY(launch(sorted_positions_kernel<float, 3>, p, sp));
   }
   PG_CUDA_TRY(cudaGetLastError());
   return PG_OK;

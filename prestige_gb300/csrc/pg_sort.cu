@@ -13,7 +13,8 @@
 //   cell_reduce  totals per block of the scan (grids of more than one chunk of kScanChunk cells; adding them up by
 //                atomics in the hash took 5 ns per warp of particles: one address at a time)
 //   cell_scan    cell_start = exclusive scan of the counts: a block per chunk (in the largest grids for
-//                several), its base the sum of the totals of the blocks before it; the counts go back to zero for the next search
+//                several), its base the sum of the totals of the blocks before it; the counts go
+//                back to zero for the next search
 //   cell_scatter id -> slot cell_start[cell] + rank, so ids are grouped by cell in arrival order
 //   the gather   ranks each id among the ids of its cell (ordered_slot): the stable order
 // It is bound by the latency of these few launches below about 1M particles and by the scattered
@@ -24,7 +25,8 @@
 // Ranking an id among the m ids of its cell takes the gather m reads.  Cells of more than kBigCell
 // particles take counts per tile of consecutive ids instead: rank = rank within the tile + the counts of
 // the tiles before (rank_big_cells, large_cell_rank).  Search of 1M particles in 100 of 10,000 cells 0.35 ms; one
-// block that sorts such cells one after the other takes 8.5, the radix sort about 0.1.  Dense grids take an LSD radix sort (sort_mode).
+// block that sorts such cells one after the other takes 8.5, the radix sort about 0.1.  Dense grids take
+// an LSD radix sort (sort_mode).
 #include <cuda_runtime.h>
 
 #include <mutex>
@@ -559,11 +561,12 @@ int launch_sort(cudaStream_t st, NbrWork& w, unsigned long long* minacc, unsigne
   const uint32_t per_block = (w.chunks + kScanBlocks - 1) / kScanBlocks;
   const uint32_t blocks = (w.chunks + per_block - 1) / per_block;
   if (blocks > 1)
-    PG_CUDA_TRY(launch_chained(st, w.n > 0, per_block > 1 ? cell_reduce_kernel<true> : cell_reduce_kernel<false>, blocks,
-                               kCellScanThreads, w.count, w.chunks, per_block, w.chunk_total));
-  PG_CUDA_TRY(launch_chained(st, w.n > 0 || blocks > 1, per_block > 1 ? cell_scan_kernel<true> : cell_scan_kernel<false>,
-                             blocks, kCellScanThreads, w.count, w.chunks, per_block, w.chunk_total, w.cell_start,
-                             w.tile_count, w.tile_row, minacc, minout, minacc ? nmin : 0u));
+    PG_CUDA_TRY(launch_chained(st, w.n > 0, per_block > 1 ? cell_reduce_kernel<true> : cell_reduce_kernel<false>,
+                               blocks, kCellScanThreads, w.count, w.chunks, per_block, w.chunk_total));
+  PG_CUDA_TRY(launch_chained(st, w.n > 0 || blocks > 1,
+                             per_block > 1 ? cell_scan_kernel<true> : cell_scan_kernel<false>, blocks, kCellScanThreads,
+                             w.count, w.chunks, per_block, w.chunk_total, w.cell_start, w.tile_count, w.tile_row,
+                             minacc, minout, minacc ? nmin : 0u));
   if (w.n)
     PG_CUDA_TRY(launch_chained(st, true, cell_scatter_kernel, (unsigned)((w.n + kSortThreads - 1) / kSortThreads),
                                kSortThreads, w.key, w.rank, w.cell_start, (uint32_t)w.n, w.unsorted, w.tile_count,
@@ -577,8 +580,8 @@ int launch_sort(cudaStream_t st, NbrWork& w, unsigned long long* minacc, unsigne
 //
 // The radix sort (digit_hist, digit_scan, digit_scatter above) needs scratch beyond its inputs and
 // outputs: a second key/value buffer for the ping-pong passes, the per-tile digit histograms and
-// the digit totals.  It comes from one file-scope device array, so a call allocates nothing.  Its size fixes the largest
-// system it accepts (kNoAllocMaxParticles).
+// the digit totals.  It comes from one file-scope device array, so a call allocates nothing.  Its size
+// fixes the largest system it accepts (kNoAllocMaxParticles).
 //
 // The array is shared by every call on a device and keeps the previous call's contents.
 // Nothing in it needs to start at zero: the hash writes every key, each histogram launch

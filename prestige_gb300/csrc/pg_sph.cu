@@ -20,7 +20,7 @@
 // Kernel structure (pg_sph_pass.cuh): the list kernel tests every candidate of the 9 (2D: 3)
 // neighbour rows in FP32 against bounds on r^2, with the exact test inside their band, and
 // writes each target's neighbours in walk order; the two passes evaluate the listed pairs, one
-// thread per target (slot order; more in small double-word systems).  The IEEE f64 step
+// thread per target (slot order; more in small double-word and f32 systems).  The IEEE f64 step
 // evaluates each pair once instead (pg_sph_sym.cu).
 // Pairs are evaluated in the oracle's order (rows z, y ascending; slots ascending), so the
 // IEEE modes reproduce the oracle bit for bit.
@@ -720,9 +720,10 @@ PassKernel ordered_kernel_for(int arith) {
 
 template <int LANES>
 PassKernel ordered_kernel(int arith, int dim, int stage) {
+  const bool cont = stage == SPH_CONT;
   if (dim == 2)
-    return stage == SPH_CONT ? ordered_kernel_for<2, SPH_CONT, LANES>(arith) : ordered_kernel_for<2, SPH_MOM, LANES>(arith);
-  return stage == SPH_CONT ? ordered_kernel_for<3, SPH_CONT, LANES>(arith) : ordered_kernel_for<3, SPH_MOM, LANES>(arith);
+    return cont ? ordered_kernel_for<2, SPH_CONT, LANES>(arith) : ordered_kernel_for<2, SPH_MOM, LANES>(arith);
+  return cont ? ordered_kernel_for<3, SPH_CONT, LANES>(arith) : ordered_kernel_for<3, SPH_MOM, LANES>(arith);
 }
 
 // The list kernel with the batch that suits the rows' length (see sph_list_kernel).
@@ -869,9 +870,9 @@ int launch_sph_list_exact(cudaStream_t st, const SphArgs& a, int grid, int block
 int launch_sph_list_pass(cudaStream_t st, const SphArgs& a, int arith, int stage, int grid, int block, int lanes) {
   lanes = sph_pass_lanes(arith, stage, lanes);
   const int ordered = arith != ARITH_F64_EXACT && lanes == 1 && stage != SPH_RATES ? ordered_lanes(arith, a.n) : 1;
-  if (ordered > 1)
-    return launch_table(st, a, ordered == 4 ? ordered_kernel<4>(arith, a.dim, stage) : ordered_kernel<2>(arith, a.dim, stage),
-                        0, block, ordered);  // one block per tile
+  // (one block per tile)
+  if (ordered == 4) return launch_table(st, a, ordered_kernel<4>(arith, a.dim, stage), 0, block, 4);
+  if (ordered == 2) return launch_table(st, a, ordered_kernel<2>(arith, a.dim, stage), 0, block, 2);
   PassKernel kern = list_kernel(arith, a.dim, stage, lanes, a.reach);
   return launch_table(st, a, kern, grid, block, lanes);
 }

@@ -39,7 +39,9 @@
 // four threads per slot in c1 and m1 another 0.25 less together.
 // Where a warp or two share a scheduler and latency decides, the FP64 multiplication is the faster
 // one (two-sided passes at 6.5k particles: 0.118 ms a step against 0.153 with soft_mul; the dense DEM
-// pass 0.296 against 0.368), so only these kernels use the integer one.
+// pass 0.296 against 0.368), so only these kernels use the integer one.  (Step of 1M moving
+// particles 4.80 ms, with FP64 products 5.64; at rest on a regular lattice, where a zero factor in any lane
+// takes the warp through both, 7.70 and 7.69; the 2D dam break of 6,518 70 us and 60.)
 #include <cuda_runtime.h>
 #include <stdint.h>
 
