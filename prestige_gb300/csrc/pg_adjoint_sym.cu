@@ -36,10 +36,10 @@ namespace {
 
 using namespace sphpass;
 
-constexpr int kPlanes = 15;  // doubles per list entry (plus the mirror index and the partner)
+constexpr int kPlanes = 15;  // doubles per list entry (plus the word with mirror index and partner)
 // the partner's momentum share (Vx, Vv, F x.E, Pi / rho_ij); for the continuity pass, the pair's
 // vectors U1 = G w x + F v and U2 = F x and the partner's mass (own entries above the slot).  The first
-// group is indexed like the list; the second and {mirror index, partner}, which only the slot
+// group is indexed like the list; the second and the mirror words (mirror_word), which only the slot
 // itself reads, by the number of the entry among those above the slot, so lanes that each start at
 // their own first entry above the slot read and write whole rows of them.
 enum { kMx = 0, kMv = 3, kFxE = 6, kPIrb = 7, kU1 = 8, kU2 = 11, kMt = 14 };
@@ -51,7 +51,7 @@ struct Planes {
   double* base;
   size_t plane;  // entries per plane
   __device__ __forceinline__ double& at(int j, size_t e) const { return base[j * plane + e]; }
-  __device__ __forceinline__ uint2& mirror(size_t e) const { return ((uint2*)(base + kPlanes * plane))[e]; }
+  __device__ __forceinline__ uint32_t& mirror(size_t e) const { return ((uint32_t*)(base + kPlanes * plane))[e]; }
 };
 
 __device__ __forceinline__ Planes planes_of(const SphArgs& a) {
@@ -290,7 +290,7 @@ __global__ void __launch_bounds__(kSphMaxThreads) adj_mirror_kernel(SphArgs a) {
     find_in_lists(a, t, s.k, m);
 #pragma unroll
     for (int i = 0; i < kSearch; ++i)
-      if (j + i < U) E.mirror(entry(s.k, j + i, a.cap)) = make_uint2(m[i], t[i]);
+      if (j + i < U) E.mirror(entry(s.k, j + i, a.cap)) = mirror_word(m[i], t[i], s.k);
   }
 }
 
@@ -308,19 +308,20 @@ __global__ void __launch_bounds__(kSphMaxThreads) adj_a1_kernel(SphArgs a) {
   Sums sum = {{0, 0, 0}, {0, 0, 0}, 0, 0, 0};
   // each lane from its own first entry above the slot, so the lanes of a warp evaluate their
   // pairs in the same iterations
-  const uint32_t U = s.L - lower_bound(my, s.L, s.k);
+  const uint32_t q0 = lower_bound(my, s.L, s.k), U = s.L - q0;
+  my += (size_t)q0 * kListTile;
   for (uint32_t j = s.sub; j < U; j += LANES) {
     const size_t e = entry(s.k, j, a.cap);
-    const uint2 mt = E.mirror(e);
-    const MomTerms<DIM> m = mom_terms<DIM>(K, P, s.k, mt.y, xk, vk);
+    const Mirror mt = mirror_of(E.mirror(e), s.k, my, j);
+    const MomTerms<DIM> m = mom_terms<DIM>(K, P, s.k, mt.slot, xk, vk);
 #pragma unroll
     for (int cc = 0; cc < DIM; ++cc) {
       E.at(kU1 + cc, e) = m.U1[cc];
       E.at(kU2 + cc, e) = m.U2[cc];
     }
     E.at(kMt, e) = m.mt;
-    if (mt.x != kNoMirror) {
-      const size_t f = entry(mt.y, mt.x, a.cap);
+    if (mt.pos != kNoPos) {
+      const size_t f = entry(mt.slot, mt.pos, a.cap);
 #pragma unroll
       for (int cc = 0; cc < DIM; ++cc) {
         E.at(kMx + cc, f) = m.Vx[cc];
@@ -329,7 +330,7 @@ __global__ void __launch_bounds__(kSphMaxThreads) adj_a1_kernel(SphArgs a) {
       E.at(kFxE, f) = m.FxE;
       E.at(kPIrb, f) = m.PIrb;
     }
-    add_own<DIM>(sum, m, Pdk, mt.x != kNoMirror ? 1.0 : 0.5);
+    add_own<DIM>(sum, m, Pdk, mt.pos != kNoPos ? 1.0 : 0.5);
   }
   lane_sums<LANES>(sum, kSlotSums);
   if (s.sub == 0) store_sums(a, P, s.k, sum, kSlotSums);
@@ -416,7 +417,8 @@ __global__ void __launch_bounds__(kSphMaxThreads) adj_c1_kernel(SphArgs a) {
   const uint32_t* __restrict__ my = a.nlist + list_base(s.k, a.cap);
   Sums sum = {{0, 0, 0}, {0, 0, 0}, 0, 0, 0};
   // this pass waits on its loads: the partner two entries ahead, everything else one ahead
-  const uint32_t U = s.L - lower_bound(my, s.L, s.k);
+  const uint32_t q0 = lower_bound(my, s.L, s.k), U = s.L - q0;
+  my += (size_t)q0 * kListTile;
   if (s.sub < U) {
     auto row = [&](uint32_t j) { return entry(s.k, min(j, U - 1), a.cap); };
     struct Vals {
@@ -431,12 +433,14 @@ __global__ void __launch_bounds__(kSphMaxThreads) adj_c1_kernel(SphArgs a) {
       v.mt = E.at(kMt, e);
       v.db = P.DB[t];
     };
-    uint2 m = E.mirror(row(s.sub)), mn = E.mirror(row(s.sub + LANES));
+    Mirror m = mirror_of(E.mirror(row(s.sub)), s.k, my, s.sub);
+    uint32_t next = E.mirror(row(s.sub + LANES));
     Vals v, vn;
-    load(row(s.sub), m.y, v);
+    load(row(s.sub), m.slot, v);
     for (uint32_t j = s.sub; j < U; j += LANES) {
-      const uint2 mnn = E.mirror(row(j + 2 * LANES));
-      load(row(j + LANES), mn.y, vn);
+      const uint32_t next2 = E.mirror(row(j + 2 * LANES));
+      const Mirror mn = mirror_of(next, s.k, my, min(j + LANES, U - 1));
+      load(row(j + LANES), mn.slot, vn);
       const double D = dbk * v.mt + v.db * mk;
       double Vx[DIM], Vv[DIM];
 #pragma unroll
@@ -446,8 +450,8 @@ __global__ void __launch_bounds__(kSphMaxThreads) adj_c1_kernel(SphArgs a) {
         sum.gx[cc] += Vx[cc];
         sum.gv[cc] += Vv[cc];
       }
-      if (m.x != kNoMirror) {
-        const size_t f = entry(m.y, m.x, a.cap);
+      if (m.pos != kNoPos) {
+        const size_t f = entry(m.slot, m.pos, a.cap);
 #pragma unroll
         for (int cc = 0; cc < DIM; ++cc) {
           E.at(kMx + cc, f) = Vx[cc];
@@ -455,7 +459,7 @@ __global__ void __launch_bounds__(kSphMaxThreads) adj_c1_kernel(SphArgs a) {
         }
       }
       m = mn;
-      mn = mnn;
+      next = next2;
       v = vn;
     }
   }
@@ -519,7 +523,7 @@ AdjSymKernel adj_sym_kernel(int part) {
 
 }  // namespace
 
-size_t adjoint_sym_entry_bytes() { return kPlanes * sizeof(double) + 2 * sizeof(uint32_t); }
+size_t adjoint_sym_entry_bytes() { return kPlanes * sizeof(double) + sizeof(uint32_t); }
 size_t adjoint_sym_slot_bytes() { return kSlotSums * sizeof(double); }
 
 int launch_adjoint_sym(cudaStream_t st, const SphArgs& a, int part) {

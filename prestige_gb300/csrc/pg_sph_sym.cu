@@ -58,10 +58,10 @@ using namespace sphpass;
 typedef OpsDI D;  // multiplications, divisions and roots on the integer pipe
 
 // Entry planes of the per-entry store (a.fcache): doubles F, w, r^2 + eps h^2, S (w F after
-// sym_c1, X after sym_m1), then the u32 pairs {mirror index, partner}, each plane in the tiled list
-// layout.  S is indexed like the list; the others, which only the slot itself reads, by the number
-// of the entry among those above the slot, so a warp whose lanes each start at their own first
-// entry above the slot still reads and writes whole rows of them.
+// sym_c1, X after sym_m1), then a word with the mirror index and the partner (mirror_word), each plane
+// in the tiled list layout.  S is indexed like the list; the others, which only the slot itself reads,
+// by the number of the entry among those above the slot, so a warp whose lanes each start at their own
+// first entry above the slot still reads and writes whole rows of them.
 struct Planes {
   double* base;
   size_t plane;  // entries per plane
@@ -69,7 +69,7 @@ struct Planes {
   __device__ __forceinline__ double* W(size_t e) const { return base + plane + e; }
   __device__ __forceinline__ double* R(size_t e) const { return base + 2 * plane + e; }
   __device__ __forceinline__ double* S(size_t e) const { return base + 3 * plane + e; }
-  __device__ __forceinline__ uint2* M(size_t e) const { return (uint2*)(base + 4 * plane) + e; }
+  __device__ __forceinline__ uint32_t* M(size_t e) const { return (uint32_t*)(base + 4 * plane) + e; }
 };
 
 __device__ __forceinline__ Planes planes_of(const SphArgs& a) {
@@ -207,18 +207,20 @@ __global__ void __launch_bounds__(kSphMaxThreads) sym_c1_kernel(SphArgs a, uint3
     find_in_lists(a, t, s.k, m);
 #pragma unroll
     for (int i = 0; i < kSearch; ++i)
-      if (j + i * kPairLanes < U) *P.M(entry(s.k, j + i * kPairLanes, a.cap)) = make_uint2(m[i], t[i]);
+      if (j + i * kPairLanes < U) *P.M(entry(s.k, j + i * kPairLanes, a.cap)) = mirror_word(m[i], t[i], s.k);
   }
   if (s.sub >= U) return;
   // software pipeline: entries two ahead, the partner's records one ahead (each thread reads back the
   // entries it wrote above)
   constexpr uint32_t N = kPairLanes;
   const uint32_t last = s.sub + (U - 1 - s.sub) / N * N;  // the thread's last entry
-  uint2 m = *P.M(entry(s.k, s.sub, a.cap)), mn = *P.M(entry(s.k, min(s.sub + N, last), a.cap));
-  double4_32a Aj = A[m.y], Bj = B[m.y];
+  Mirror m = mirror_of(*P.M(entry(s.k, s.sub, a.cap)), s.k, my, s.sub);
+  uint32_t next = *P.M(entry(s.k, min(s.sub + N, last), a.cap));
+  double4_32a Aj = A[m.slot], Bj = B[m.slot];
   for (uint32_t j = s.sub; j < U; j += N) {
-    const uint2 mnn = *P.M(entry(s.k, min(j + 2 * N, last), a.cap));
-    const double4_32a An = A[mn.y], Bn = B[mn.y];
+    const uint32_t next2 = *P.M(entry(s.k, min(j + 2 * N, last), a.cap));
+    const Mirror mn = mirror_of(next, s.k, my, min(j + N, last));
+    const double4_32a An = A[mn.slot], Bn = B[mn.slot];
     double d[3], r2, F, w;
     pair_geometry<DIM>(K.d, Ai, Bi, Aj, Bj, d, r2, F, w);
     const double wF = D::mul(w, F);
@@ -227,9 +229,9 @@ __global__ void __launch_bounds__(kSphMaxThreads) sym_c1_kernel(SphArgs a, uint3
     *P.W(e) = w;
     *P.R(e) = D::add(r2, K.d.eps_h2);
     *P.S(entry(s.k, q0 + j, a.cap)) = wF;
-    if (m.x != kNoMirror) *P.S(entry(m.y, m.x, a.cap)) = wF;
+    if (m.pos != kNoPos) *P.S(entry(m.slot, m.pos, a.cap)) = wF;
     m = mn;
-    mn = mnn;
+    next = next2;
     Aj = An;
     Bj = Bn;
   }
@@ -298,21 +300,24 @@ __global__ void __launch_bounds__(kSphMaxThreads) sym_m1_kernel(SphArgs a) {
   // the partner's index is loaded two entries ahead and everything else one ahead
   const uint32_t q0 = lower_bound(my, s.L, s.k), U = s.L - q0;
   if (s.sub >= U) return;
+  my += (size_t)q0 * kListTile;
   constexpr uint32_t N = kPairLanes;
-  uint2 m = *P.M(entry(s.k, s.sub, a.cap)), mn = *P.M(entry(s.k, min(s.sub + N, U - 1), a.cap));
+  Mirror m = mirror_of(*P.M(entry(s.k, s.sub, a.cap)), s.k, my, s.sub);
+  uint32_t next = *P.M(entry(s.k, min(s.sub + N, U - 1), a.cap));
   size_t e = entry(s.k, s.sub, a.cap);
   double F = *P.F(e), w = *P.W(e), r2e = *P.R(e);
-  double2 qt = Q[m.y];
+  double2 qt = Q[m.slot];
   for (uint32_t j = s.sub; j < U; j += N) {
-    const uint2 mnn = *P.M(entry(s.k, min(j + 2 * N, U - 1), a.cap));
+    const uint32_t next2 = *P.M(entry(s.k, min(j + 2 * N, U - 1), a.cap));
+    const Mirror mn = mirror_of(next, s.k, my, min(j + N, U - 1));
     e = entry(s.k, min(j + N, U - 1), a.cap);
     const double Fn = *P.F(e), wn = *P.W(e), rn = *P.R(e);
-    const double2 qn = Q[mn.y];
+    const double2 qn = Q[mn.slot];
     const double X = momentum_factor(K.d, F, w, r2e, qk, qt);
     *P.S(entry(s.k, q0 + j, a.cap)) = X;
-    if (m.x != kNoMirror) *P.S(entry(m.y, m.x, a.cap)) = X;
+    if (m.pos != kNoPos) *P.S(entry(m.slot, m.pos, a.cap)) = X;
     m = mn;
-    mn = mnn;
+    next = next2;
     F = Fn;
     w = wn;
     r2e = rn;
@@ -391,7 +396,7 @@ SymKernel sym_kernel(int part) {
 
 }  // namespace
 
-size_t sph_sym_entry_bytes() { return 4 * sizeof(double) + 2 * sizeof(uint32_t); }
+size_t sph_sym_entry_bytes() { return 4 * sizeof(double) + sizeof(uint32_t); }
 
 int launch_sph_sym(cudaStream_t st, const SphArgs& a, int part, int block, uint32_t split, int second) {
   SymKernel kern = a.dim == 2 ? sym_kernel<2>(part) : sym_kernel<3>(part);
