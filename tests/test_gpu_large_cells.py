@@ -77,16 +77,18 @@ def test_order(pg, oracle, kind, empty, order):
     s.close()
 
 
+@pytest.mark.parametrize("scale", [1, 10])  # counted tiles, radix sort
 @pytest.mark.parametrize("mode", [0, 1])
-def test_batch(pg, oracle, mode):
+def test_batch(pg, oracle, mode, scale):
     """Systems with and without large cells in one handle: each as in a handle of its own."""
     rng = np.random.default_rng(5)
-    counts = [np.array([1500, 3, 2000]), np.array([20, 20, 20]), np.array([0, 5000, 1025, 1])]
+    counts = [scale * np.array(c) for c in ([1500, 3, 2000], [20, 20, 20], [0, 5000, 1025, 1])]
     cfgs = [_cfg(len(c), f64_mode=mode) for c in counts]
     pos = [_positions(c, rng, "shuffled") for c in counts]
     s = ParticleSystem.batch(cfgs, [p.shape[0] for p in pos])
     s.set("pos", np.concatenate(pos))
     cell, ids, start = s.neighbors()
+    assert (s.info()["sort_passes"] > 0) == (scale == 10)
     first = base = 0
     for p, cfg in zip(pos, cfgs):
         ocell, oid, ostart = oracle.cell_list(p, cfg["domain_lo"], cfg["domain_hi"], 2.0 * cfg["h"], 1.0, True)
@@ -100,10 +102,11 @@ def test_batch(pg, oracle, mode):
 
 
 @pytest.mark.parametrize("graph", [False, True])
-@pytest.mark.parametrize("n,mult", [(20000, 5.0), (60000, 4.0)])
+@pytest.mark.parametrize("n,mult", [(20000, 5.0), (60000, 4.0), (1048577, 3.0)])
 @pytest.mark.parametrize("mode", [0, 1])
 def test_steps(pg, mode, n, mult, graph):
-    """A lattice in large cells (counted tiles, radix sort) against the same one in ordinary cells."""
+    """A lattice in large cells (counted tiles, radix sort; beyond 1M particles on the overlapped schedule) against
+    the same one in ordinary cells."""
     w = workloads.sph_lattice_3d(n=n, seed=11, f64_mode=mode)
     out = []
     for m in (mult, 1.0):
@@ -111,14 +114,41 @@ def test_steps(pg, mode, n, mult, graph):
         workloads.load_into(s, w)
         if m > 1.0:
             _, _, start = s.neighbors()
-            assert np.diff(start.astype(np.int64)).max() > 1024
-            assert (s.info()["sort_passes"] > 0) == (n == 60000)
+            assert np.diff(start.astype(np.int64)).max() > (1024 if n < 1000000 else 400)
+            assert (s.info()["sort_passes"] > 0) == (n > 20000)
         s.enable_graph(graph)
         s.step(5)
         out.append([s.get(k) for k in ("pos", "vel", "rho")])
         s.close()
     for a, b in zip(*out):
         assert np.abs(a - b).max() <= 1e-10 * np.abs(b).max()
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+def test_batch_steps(pg, mode):
+    """Three lattices in one handle (radix sort, a position minimum per system) and each alone (counted tiles):
+    the same bits."""
+    ws = [workloads.sph_lattice_3d(n=n, seed=n, f64_mode=mode, cell_multiplier=5.0) for n in (19000, 20000, 21000)]
+    for i, w in enumerate(ws):  # apart from one another, so that the minima differ
+        w["fields"]["pos"] += 10.0 * i
+        for k in ("domain_lo", "domain_hi"):
+            w["config"][k] = [x + 10.0 * i for x in w["config"][k]]
+    both = ParticleSystem.batch([w["config"] for w in ws], [w["n"] for w in ws])
+    assert both.info()["sort_passes"] > 0
+    for k in ("pos", "vel", "rho", "mass"):
+        both.set(k, np.concatenate([w["fields"][k] for w in ws]))
+    both.step(3)
+    first = 0
+    for w in ws:
+        s = ParticleSystem(make_config(**w["config"]), w["n"])
+        assert s.info()["sort_passes"] == 0
+        workloads.load_into(s, w)
+        s.step(3)
+        for k in ("pos", "vel", "rho"):
+            assert np.array_equal(both.get(k)[first:first + w["n"]], s.get(k)), k
+        first += w["n"]
+        s.close()
+    both.close()
 
 
 def test_cost(pg):
