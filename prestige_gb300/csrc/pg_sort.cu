@@ -355,7 +355,7 @@ __device__ __noinline__ void rank_big_cells(const uint32_t* __restrict__ key, ui
   const uint32_t tile = blockIdx.x * kSortWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (tile > (n - 1) >> tile_shift) return;
   const uint32_t i0 = tile << tile_shift, len = min(1u << tile_shift, n - i0);
-  uint32_t b = 0, m = 0, r = 0;  // of this round's id: the cell's first slot and size, the arrival rank
+  uint32_t b = 0, m = 0, r = 0;  // of the id at hand: the cell's first slot and size, the arrival rank
   auto load = [&](uint32_t j) {
     m = 0;
     if (j < len) {
@@ -369,7 +369,7 @@ __device__ __noinline__ void rank_big_cells(const uint32_t* __restrict__ key, ui
   for (uint32_t j0 = 0; j0 < len; j0 += 32) {
     const uint32_t b0 = b, r0 = r, i = i0 + j0 + lane;
     const bool big = m > kBigCell;
-    load(j0 + 32 + lane);  // the next round's, while this one's count is read
+    load(j0 + 32 + lane);  // the next ids', while these ids' counts are read
     const unsigned peers = __match_any_sync(0xffffffffu, big ? b0 / kBigCell : 0xffffffffu);
     if (big) {
       uint32_t* row = tile_count + (size_t)(b0 / kBigCell) * tile_row;
@@ -383,7 +383,7 @@ __device__ __noinline__ void rank_big_cells(const uint32_t* __restrict__ key, ui
       rank[i] = __shfl_sync(peers, before, leader) + __popc(peers & ((1u << lane) - 1u));
       unsorted[b0 + r0] = i;
     }
-    __syncwarp();  // the counts, for the next round's leaders
+    __syncwarp();  // the counts, for the next leaders
   }
 }
 
